@@ -43,17 +43,21 @@ struct GridImpl {
     double2 *xieta = nullptr;
     int32_t *perm = nullptr;
     double4 *pool = nullptr;      // n points + nsrc*P proxies
-    Group *leaf_groups = nullptr;
-    Item *leaf_items = nullptr;
+    EvalUnit *eval_units = nullptr;
+    EvalStage *eval_stages = nullptr;
+    EvalItem *eval_items = nullptr;
     uint32_t *masks = nullptr;
-    Group *proxy_groups = nullptr;
-    Item *proxy_items = nullptr;
-    int32_t *proxy_unit_beg = nullptr;
+    LeafFin *leaf_fin = nullptr;
+    int32_t *down_slots = nullptr;
+    double2 *leaf_part = nullptr;
+    int32_t *eval_proxy_unit_beg = nullptr;
+    int32_t *proxy_unit_beg = nullptr;   // 32-field blocks
     double4 *tgt_proxy = nullptr;
     double *records = nullptr;
     double4 *proxy_partial = nullptr;
-    UpUnit *up_units = nullptr;
-    int32_t *up_unit_beg = nullptr;
+    UpUnit *up64_units = nullptr;
+    int32_t *up64_unit_beg = nullptr;
+    int32_t *up_unit_beg = nullptr;      // 32-field blocks
     double *src_nodes = nullptr;
     double *up_partial = nullptr;
     int *err = nullptr;
@@ -276,7 +280,7 @@ extern "C" int sal_grid_create(const sal_tree *t_, const sal_grid_desc *d, sal_g
     g.max_fields = d->max_fields;
     if (d->mode == SAL_MODE_DTT) g.tree = t;
     std::string err;
-    if (!plan_build(t, d->interp_degree, d->mode, d->list, d->list_count, d->pc_list, d->pc_count, d->pp_list,
+    if (!plan_build(t, d->xs, d->ys, d->zs, d->interp_degree, d->mode, d->list, d->list_count, d->pc_list, d->pc_count, d->pp_list,
                     d->pp_count, &g.plan, &err)) {
         delete G;
         return set_error(SAL_EINVAL, err);
@@ -333,18 +337,22 @@ extern "C" int sal_grid_create(const sal_tree *t_, const sal_grid_desc *d, sal_g
             for (int i = 0; i < 2 * nd; ++i) rec[(size_t)s * g.rec_stride + 4 * P + i] = pl.tgt_nodes[(size_t)s * 2 * nd + i];
         TRY(dupload(g, &g.records, rec.data(), rec.size()));
     }
-    TRY(dupload(g, &g.leaf_groups, pl.leaf_groups.data(), pl.leaf_groups.size()));
-    TRY(dupload(g, &g.leaf_items, pl.leaf_items.data(), pl.leaf_items.size()));
+    TRY(dupload(g, &g.eval_units, pl.eval_units.data(), pl.eval_units.size()));
+    TRY(dupload(g, &g.eval_stages, pl.eval_stages.data(), pl.eval_stages.size()));
+    TRY(dupload(g, &g.eval_items, pl.eval_items.data(), pl.eval_items.size()));
     TRY(dupload(g, &g.masks, pl.masks.data(), pl.masks.size()));
-    TRY(dupload(g, &g.proxy_groups, pl.proxy_groups.data(), pl.proxy_groups.size()));
-    TRY(dupload(g, &g.proxy_items, pl.proxy_items.data(), pl.proxy_items.size()));
+    TRY(dupload(g, &g.leaf_fin, pl.leaf_fin.data(), pl.leaf_fin.size()));
+    TRY(dupload(g, &g.down_slots, pl.down_slots.data(), pl.down_slots.size()));
+    TRY(dalloc(g, &g.leaf_part, (size_t)pl.leaf_part_rows));
+    TRY(dupload(g, &g.eval_proxy_unit_beg, pl.eval_proxy_unit_beg.data(), pl.eval_proxy_unit_beg.size()));
     TRY(dupload(g, &g.proxy_unit_beg, pl.proxy_unit_beg.data(), pl.proxy_unit_beg.size()));
-    TRY(dalloc(g, &g.proxy_partial, (size_t)g.nproxy_units * P));
-    TRY(dupload(g, &g.up_units, pl.up_units.data(), pl.up_units.size()));
+    TRY(dalloc(g, &g.proxy_partial, (size_t)pl.n_proxy_eval * P));
+    TRY(dupload(g, &g.up64_units, pl.up64_units.data(), pl.up64_units.size()));
+    TRY(dupload(g, &g.up64_unit_beg, pl.up64_unit_beg.data(), pl.up64_unit_beg.size()));
     TRY(dupload(g, &g.up_unit_beg, pl.up_unit_beg.data(), pl.up_unit_beg.size()));
     TRY(dupload(g, &g.src_nodes, pl.src_nodes.data(), pl.src_nodes.size()));
     TRY(dupload(g, &g.tgt_nodes, pl.tgt_nodes.data(), pl.tgt_nodes.size()));
-    TRY(dalloc(g, &g.up_partial, (size_t)g.nup * P));
+    TRY(dalloc(g, &g.up_partial, pl.up64_units.size() * (size_t)P));
     TRY(dalloc(g, &g.err, 1));
     CK(cudaMemset(g.err, 0, sizeof(int)));
     if (cudaMallocHost((void **)&g.h_flag, sizeof(int)) != cudaSuccess) {
@@ -443,62 +451,67 @@ extern "C" int sal_grid_stats_get(const sal_grid *G, sal_grid_stats *s) {
     return SAL_OK;
 }
 
-// One FP64 solve of one field: ssh (caller order, device) -> outputs (caller order, device).
-static void solve_fp64(GridImpl &g, const double *ssh, double *ox, double *oy, int form, int kinds, bool do_up,
-                       cudaStream_t st) {
+// The FP64 upward pass: proxy weights of every source slot into the pool.
+static void upward_fp64(GridImpl &g, cudaStream_t st) {
     const Plan &pl = g.plan;
-    const int n = pl.n, P = pl.P;
-    if (g.timing) cudaEventRecord(g.ev[0], st);
-    dev::launch_prep(g.xyz, g.area, ssh, g.perm, n, g.pool, st);
-    if (do_up && g.nup > 0) {
-        dev::UpArgs u{g.pool, g.xieta, g.up_units, g.src_nodes, pl.d, P, g.up_partial};
-        dev::launch_upward(u, g.nup, st);
-        dev::launch_upward_finalize(g.up_unit_beg, g.up_partial, g.nsrc, pl.d, pl.mode == SAL_MODE_STT_REF_COMPAT ? 1 : 0,
-                                    g.pool + n, st);
-    }
-    if (g.timing) cudaEventRecord(g.ev[1], st);
-    if (g.nproxy_units > 0) {
-        dev::EvalArgs a{};
-        a.pool = g.pool;
-        a.groups = g.proxy_groups;
-        a.items = g.proxy_items;
-        a.masks = g.masks;
-        a.tgt = g.tgt_proxy;
-        a.xieta = g.xieta;
-        a.records = g.records;
-        a.rec_stride = g.rec_stride;
-        a.d = pl.d;
-        a.P = P;
-        a.kinds = 3;
-        a.perm = g.perm;
-        a.partial = g.proxy_partial;
-        a.err = g.err;
-        dev::launch_eval(1, form, a, g.nproxy_units, st);
-        dev::launch_proxy_finalize(g.proxy_unit_beg, g.proxy_partial, g.ntgt, P, g.rec_stride, g.records, st);
-    }
-    if (g.timing) cudaEventRecord(g.ev[2], st);
+    dev::launch_upward(dev::UpArgs{g.pool, g.xieta, g.up64_units, g.src_nodes, g.up_partial}, pl.d,
+                       (int)pl.up64_units.size(), st);
+    dev::launch_upward_finalize(g.up64_unit_beg, g.up_partial, g.nsrc, pl.d, pl.mode == SAL_MODE_STT_REF_COMPAT ? 1 : 0,
+                                g.pool + pl.n, st);
+}
+
+// The FP64 pair evaluation and the leaves' ends: proxy potentials, point
+// sources (kinds bit 0) and proxy sources (bit 1) of every leaf -> outputs
+// (caller order, device).  inject: a pending sal_grid_inject_timeout applies.
+static void eval_fp64(GridImpl &g, double *ox, double *oy, int form, int kinds, bool inject, cudaStream_t st) {
+    const Plan &pl = g.plan;
+    const int P = pl.P, np = pl.n_proxy_eval, nu = (int)pl.eval_units.size();
     dev::EvalArgs a{};
     a.pool = g.pool;
-    a.groups = g.leaf_groups;
-    a.items = g.leaf_items;
+    a.units = g.eval_units;
+    a.stages = g.eval_stages;
+    a.items = g.eval_items;
     a.masks = g.masks;
-    a.tgt = g.pool;
-    a.xieta = g.xieta;
-    a.records = g.records;
-    a.rec_stride = g.rec_stride;
-    a.d = pl.d;
+    a.tgt_proxy = g.tgt_proxy;
     a.P = P;
     a.kinds = kinds;
     a.perm = g.perm;
     a.out_x = ox;
     a.out_y = oy;
+    a.leaf_part = g.leaf_part;
+    a.proxy_part = g.proxy_partial;
     a.err = g.err;
-    if (g.inject_polls) {
+    if (inject && g.inject_polls) {
         a.polls = g.inject_polls;
         a.skip_last = 1;
         g.inject_polls = 0;
     }
-    dev::launch_eval(0, form, a, (int)pl.leaf_groups.size(), st);
+    // proxy and leaf units do not depend on one another: one launch, so that
+    // small grids' few units of either kind fill the GPU together (two when
+    // the passes are timed apart)
+    if (g.timing) {
+        dev::launch_eval(form, a, np, st);
+        cudaEventRecord(g.ev[2], st);
+        a.units += np;
+        dev::launch_eval(form, a, nu - np, st);
+    } else {
+        dev::launch_eval(form, a, nu, st);
+    }
+    if (np > 0)
+        dev::launch_proxy_finalize(g.eval_proxy_unit_beg, g.proxy_partial, g.ntgt, P, g.rec_stride, g.records, st);
+    dev::launch_leaf_fin(form, pl.d,
+                         dev::FinArgs{g.leaf_fin, g.down_slots, g.pool, g.xieta, g.records, g.rec_stride, g.leaf_part,
+                                      g.perm, ox, oy},
+                         (int)pl.leaf_fin.size(), st);
+}
+
+// One FP64 solve of one field: ssh (caller order, device) -> outputs (caller order, device).
+static void solve_fp64(GridImpl &g, const double *ssh, double *ox, double *oy, int form, cudaStream_t st) {
+    if (g.timing) cudaEventRecord(g.ev[0], st);
+    dev::launch_prep(g.xyz, g.area, ssh, g.perm, g.plan.n, g.pool, st);
+    upward_fp64(g, st);
+    if (g.timing) cudaEventRecord(g.ev[1], st);
+    eval_fp64(g, ox, oy, form, 3, true, st);
     if (g.timing) {
         cudaEventRecord(g.ev[3], st);
         cudaEventSynchronize(g.ev[3]);
@@ -950,7 +963,7 @@ extern "C" int sal_solve(sal_grid *G, const double *ssh, int32_t nf, int64_t ld_
     }
     for (int f = 0; f < nf; ++f)
         solve_fp64(g, ssh + (size_t)f * ld_ssh, ox + (size_t)f * ld_out, oy + (size_t)f * ld_out,
-                   g.plan.mode == SAL_MODE_DTT ? form : SAL_FORM_REF, 7, true, st);
+                   g.plan.mode == SAL_MODE_DTT ? form : SAL_FORM_REF, st);
     CK(cudaGetLastError());
     return SAL_OK;
 }
@@ -1363,7 +1376,7 @@ extern "C" int sal_fast_sum_host(sal_grid *G, const double *ssh, double *lon, do
     int rc = ensure_host_staging(g);
     if (rc) return rc;
     CK(cudaMemcpyAsync(g.h_ssh, ssh, (size_t)g.plan.n * 8, cudaMemcpyHostToDevice, g.stream));
-    solve_fp64(g, g.h_ssh, g.h_ox, g.h_oy, form, 7, true, g.stream);
+    solve_fp64(g, g.h_ssh, g.h_ox, g.h_oy, form, g.stream);
     CK(cudaGetLastError());
     return add_back(g, lon, lat);
 }
@@ -1380,10 +1393,7 @@ extern "C" int sal_proxy_source_compute_host(sal_grid *G, const double *sshs, do
     const int n = pl.n, P = pl.P;
     CK(cudaMemcpyAsync(g.h_ssh, sshs, (size_t)n * 8, cudaMemcpyHostToDevice, g.stream));
     dev::launch_prep(g.xyz, g.area, g.h_ssh, g.perm, n, g.pool, g.stream);
-    dev::UpArgs u{g.pool, g.xieta, g.up_units, g.src_nodes, pl.d, P, g.up_partial};
-    dev::launch_upward(u, g.nup, g.stream);
-    dev::launch_upward_finalize(g.up_unit_beg, g.up_partial, g.nsrc, pl.d, pl.mode == SAL_MODE_STT_REF_COMPAT ? 1 : 0,
-                                g.pool + n, g.stream);
+    upward_fp64(g, g.stream);
     const size_t cnt = (size_t)P * g.nsrc;
     dev::launch_extract_w(g.pool + n, (int)cnt, g.h_w, g.stream);
     std::vector<double> w(cnt);
@@ -1406,11 +1416,7 @@ extern "C" int sal_pc_compute_host(sal_grid *G, const double *weights, double *s
     CK(cudaMemcpyAsync(g.h_w, weights, cnt * 8, cudaMemcpyHostToDevice, g.stream));
     dev::launch_insert_w(g.h_w, (int)cnt, g.pool + g.plan.n, g.stream);
     // PC items only: point weights are not read, so no prep is needed
-    dev::EvalArgs a{};
-    a.pool = g.pool; a.groups = g.leaf_groups; a.items = g.leaf_items; a.masks = g.masks; a.tgt = g.pool;
-    a.xieta = g.xieta; a.records = g.records; a.rec_stride = g.rec_stride; a.d = g.plan.d; a.P = g.plan.P;
-    a.kinds = 2; a.perm = g.perm; a.out_x = g.h_ox; a.out_y = g.h_oy; a.err = g.err;
-    dev::launch_eval(0, SAL_FORM_REF, a, (int)g.plan.leaf_groups.size(), g.stream);
+    eval_fp64(g, g.h_ox, g.h_oy, SAL_FORM_REF, 2, false, g.stream);
     CK(cudaGetLastError());
     return add_back(g, sx, sy);
 }
@@ -1425,11 +1431,7 @@ extern "C" int sal_pp_compute_host(sal_grid *G, const double *sshs, double *sx, 
     if (rc) return rc;
     CK(cudaMemcpyAsync(g.h_ssh, sshs, (size_t)g.plan.n * 8, cudaMemcpyHostToDevice, g.stream));
     dev::launch_prep(g.xyz, g.area, g.h_ssh, g.perm, g.plan.n, g.pool, g.stream);
-    dev::EvalArgs a{};
-    a.pool = g.pool; a.groups = g.leaf_groups; a.items = g.leaf_items; a.masks = g.masks; a.tgt = g.pool;
-    a.xieta = g.xieta; a.records = g.records; a.rec_stride = g.rec_stride; a.d = g.plan.d; a.P = g.plan.P;
-    a.kinds = 1; a.perm = g.perm; a.out_x = g.h_ox; a.out_y = g.h_oy; a.err = g.err;
-    dev::launch_eval(0, SAL_FORM_REF, a, (int)g.plan.leaf_groups.size(), g.stream);
+    eval_fp64(g, g.h_ox, g.h_oy, SAL_FORM_REF, 1, false, g.stream);
     CK(cudaGetLastError());
     return add_back(g, sx, sy);
 }

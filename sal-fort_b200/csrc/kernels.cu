@@ -30,52 +30,102 @@ void launch_prep(const double4 *xyz, const double *area, const double *ssh, cons
 }
 
 // ------------------------------------------------------------------ upward pass
-// Proxy weights of one (source slot, chunk) unit: W[j + k n] = sum over the
+// Proxy weights of one (source slot, chunk) unit: W[j + k N] = sum over the
 // chunk's points of xi_basis_j * eta_basis_k * w (fast_sum_module.f90:99-111).
-// Threads 0..127 form the xi bases of 128 points, threads 128..255 the eta
-// bases times w; then P accumulators (3 thread groups for d = 8) reduce the
-// tile.
-__global__ void __launch_bounds__(kThreads) upward_kernel(UpArgs a) {
-    __shared__ double fx[128][kMaxDegree + 1];
-    __shared__ double fe[128][kMaxDegree + 1];
-    __shared__ double nod[2 * (kMaxDegree + 1)];
-    __shared__ double red[kThreads];
+// The threads form the xi bases and the eta bases times w of a tile of points
+// in shared memory; then thread (kb, g) adds three eta rows 3 kb.. of points
+// g, g + 64, ...: N + 3 shared loads feed 3 N multiply-adds, and a warp's 32
+// points are summed with shuffles once per unit.  Bound by the FP64 pipe and
+// the shared loads together; the bases use fast_rcp (18 IEEE divisions a point
+// at d = 8 were most of the pass).
+constexpr int kUpTile = 128;
+template <int N>
+__global__ void __launch_bounds__(64 * ((N + 2) / 3)) upward_kernel(UpArgs a) {
+    constexpr int KB = (N + 2) / 3, T = 64 * KB, P = N * N, NS = N | 1;   // odd row strides: no bank conflicts
+    __shared__ double fx[kUpTile][NS];
+    __shared__ double fe[kUpTile][NS];
+    __shared__ double nod[2 * N];
+    __shared__ double red[KB][2][3 * N];
     const UpUnit u = a.units[blockIdx.x];
-    const int tid = threadIdx.x, n = a.d + 1, P = a.P;
-    if (tid < 2 * n) nod[tid] = a.nodes[(size_t)u.slot * 2 * n + tid];
-    __syncthreads();
-    const int nsub = kThreads / P;
-    const int grp = tid / P, pidx = tid % P, j = pidx % n, k = pidx / n;
-    double W = 0.0;
-    double f[kMaxDegree + 1];
-    for (int b = u.beg; b < u.end; b += 128) {
-        const int m = min(128, u.end - b);
-        if (tid < m) {
-            bli_basis(a.xieta[b + tid].x, nod, n, f);
-            for (int i = 0; i < n; ++i) fx[tid][i] = f[i];
-        } else if (tid >= 128 && tid - 128 < m) {
-            const int s = tid - 128;
-            bli_basis(a.xieta[b + s].y, nod + n, n, f);
-            const double w = a.pool[b + s].w;
-            for (int i = 0; i < n; ++i) fe[s][i] = f[i] * w;
+    const int tid = threadIdx.x, kb = tid >> 6, g = tid & 63;
+    if (tid < 2 * N) nod[tid] = a.nodes[(size_t)u.slot * 2 * N + tid];
+    double acc[3][N];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int j = 0; j < N; ++j) acc[r][j] = 0.0;
+    for (int b = u.beg; b < u.end; b += kUpTile) {
+        const int m = min(kUpTile, u.end - b);
+        __syncthreads();
+        for (int e = tid; e < 2 * m; e += T) {
+            const int s = e < m ? e : e - m;
+            const double2 xe = a.xieta[b + s];
+            const double w = e < m ? 1.0 : a.pool[b + s].w;
+            double f[N];
+            bli_basis_n<N>(e < m ? xe.x : xe.y, e < m ? nod : nod + N, f);
+            double *o = e < m ? fx[s] : fe[s];
+#pragma unroll
+            for (int i = 0; i < N; ++i) o[i] = f[i] * w;
         }
         __syncthreads();
-        if (grp < nsub)
-            for (int s = grp; s < m; s += nsub) W += fx[s][j] * fe[s][k];
-        __syncthreads();
+        for (int s = g; s < m; s += 64) {
+            double h[3];
+#pragma unroll
+            for (int r = 0; r < 3; ++r) h[r] = 3 * kb + r < N ? fe[s][3 * kb + r] : 0.0;
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const double v = fx[s][j];
+#pragma unroll
+                for (int r = 0; r < 3; ++r) acc[r][j] = fma(v, h[r], acc[r][j]);
+            }
+        }
     }
-    red[tid] = W;
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            double v = acc[r][j];
+#pragma unroll
+            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if ((tid & 31) == 0) red[kb][(tid >> 5) & 1][r * N + j] = v;
+        }
     __syncthreads();
-    if (grp == 0) {
-        double acc = 0.0;
-        for (int g = 0; g < nsub; ++g) acc += red[g * P + pidx];
-        a.partial[(size_t)blockIdx.x * P + pidx] = acc;
+    for (int p = tid; p < P; p += T) {
+        const int k = p / N, j = p % N;
+        const double *q = red[k / 3][0] + (k % 3) * N + j;
+        a.partial[(size_t)blockIdx.x * P + p] = q[0] + q[3 * N];
     }
 }
 
-void launch_upward(const UpArgs &a, int nunits, cudaStream_t st) {
+// One instantiation per N = d + 1 from 2 to kMaxDegree + 1.
+#define SAL_DEGREE_DISPATCH(fn, d, ...)                  \
+    switch ((d) + 1) {                                   \
+        case 2: fn<2>(__VA_ARGS__); break;               \
+        case 3: fn<3>(__VA_ARGS__); break;               \
+        case 4: fn<4>(__VA_ARGS__); break;               \
+        case 5: fn<5>(__VA_ARGS__); break;               \
+        case 6: fn<6>(__VA_ARGS__); break;               \
+        case 7: fn<7>(__VA_ARGS__); break;               \
+        case 8: fn<8>(__VA_ARGS__); break;               \
+        case 9: fn<9>(__VA_ARGS__); break;               \
+        case 10: fn<10>(__VA_ARGS__); break;             \
+        case 11: fn<11>(__VA_ARGS__); break;             \
+        case 12: fn<12>(__VA_ARGS__); break;             \
+        case 13: fn<13>(__VA_ARGS__); break;             \
+        case 14: fn<14>(__VA_ARGS__); break;             \
+        case 15: fn<15>(__VA_ARGS__); break;             \
+        default: break;                                  \
+    }
+static_assert(kMaxDegree + 1 == 15, "the dispatch covers every degree");
+
+template <int N>
+static void launch_upward_n(const UpArgs &a, int nunits, cudaStream_t st) {
+    upward_kernel<N><<<nunits, 64 * ((N + 2) / 3), 0, st>>>(a);
+}
+
+void launch_upward(const UpArgs &a, int d, int nunits, cudaStream_t st) {
     if (nunits <= 0) return;
-    upward_kernel<<<nunits, kThreads, 0, st>>>(a);
+    SAL_DEGREE_DISPATCH(launch_upward_n, d, a, nunits, st)
 }
 
 // Sums each slot's unit partials in unit order into the w of its pool
@@ -103,172 +153,267 @@ void launch_upward_finalize(const int32_t *unit_beg, const double *partial, int 
 }
 
 // ------------------------------------------------------------------ targets x staged sources
-// One CTA per group (a leaf, or a unit of a target slot's proxies).  Its item
-// list is walked in order; each item's sources (a pool range, or a DOWN record)
-// are brought into shared memory by one bulk copy, double-buffered, and every
-// target of the group consumes them.  Targets are spread over the 256 threads
-// as ti = tid % ntp with nsplit = 256 / ntp source splits that are summed in
-// a fixed order at the end, so results are deterministic.
-//   TGT 0: leaf targets (pool points), items PP / PC / DOWN, writes outputs.
-//   TGT 1: proxy targets, items CP (points) / CC (proxies), writes partials.
-//   FORM 0: reference kernel everywhere (2 components in each target's frame).
-//   FORM 1: proxy targets accumulate the Cartesian sum val*(s-x)*w with the
-//           antipode-stable val; DOWN interpolates it and projects on the
-//           leaf target's frame.
-template <int TGT, int FORM>
-__global__ void __launch_bounds__(kThreads) eval_kernel(EvalArgs a) {
-    __shared__ __align__(128) double4 buf[2][kMaxStage];
-    __shared__ __align__(8) uint64_t bar[2];
-    __shared__ double red[3][kThreads];
-    __shared__ int tout;
-    const Group G = a.groups[blockIdx.x];
-    const int tid = threadIdx.x;
-    const int nt = G.nt;
-    const int ntp = (nt + 31) & ~31;
-    const int nsplit = max(1, kThreads / ntp);
-    const int ti = tid % ntp, sp = tid / ntp;
-    const bool active = (ti < nt) && (sp < nsplit);
+// One CTA per unit: the targets of a leaf, or a target slot's proxies, against
+// the unit's stages.  A stage is up to 256 sources gathered from up to 32 pool
+// ranges; lane i of warp 0 copies range i (one bulk copy each, completing on
+// the stage's mbarrier) into a ring of kRing buffers, two stages ahead, so a
+// warp that is through with a stage goes on without a CTA-wide barrier.
+// Targets and source splits fill the threads without gaps: thread tid has
+// target tid % nt and sources tid / nt, tid / nt + nsplit, ...; the splits are
+// summed in a fixed order at the end, so results are deterministic.  Stages
+// are near (gref_near: the reference's operation order where its rounding
+// noise counts) or far (gref_far).
+//   Leaf units and FORM 0 proxies: the reference kernel.  FORM 1 proxies: the
+//   Cartesian sum val (s - x) w with the antipode-stable val.
+// Bound by the FP64 pipe (two cycles an instruction and warp on each of the
+// four schedulers).
+constexpr int kEvalThreads = 256, kEvalCtas = 3, kIlp = 2, kNearIlp = 2, kRing = 4, kAhead = 2;
+
+template <int FORM>
+__global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs a) {
+    __shared__ __align__(128) double4 buf[kRing][kMaxStage];
+    __shared__ __align__(8) uint64_t full[kRing], empty[kRing];
+    __shared__ int abort_;
+    volatile int *abort = &abort_;
+    const EvalUnit U = a.units[blockIdx.x];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nt = U.nt, nsplit = kEvalThreads / nt;
+    const int ti = tid % nt, sp = tid / nt;
+    const bool active = sp < nsplit;
+    const bool cart = FORM == 1 && U.proxy;
+    const int sb = (U.proxy || (a.kinds & 1)) ? U.sb : U.sm, se = (U.proxy || (a.kinds & 2)) ? U.se : U.sm;
+    const int ns = se - sb;
+    const uint32_t polls = a.polls ? a.polls : kDefaultPolls;
+    const int nissue = (a.skip_last && !U.proxy) ? ns - 1 : ns;
     Tgt T;
-    double txi = 0.0, teta = 0.0;
+    double mt[3] = {0.0, 0.0, 0.0};
     if (active) {
-        const double4 c = (TGT == 0) ? a.tgt[G.tgt + ti] : a.tgt[(size_t)G.tgt * a.P + ti];
+        const double4 c = U.proxy ? a.tgt_proxy[(size_t)U.tgt * a.P + ti] : a.pool[U.tgt + ti];
         tgt_init(T, c.x, c.y, c.z);
-        if (TGT == 0) {
-            const double2 e = a.xieta[G.tgt + ti];
-            txi = e.x;
-            teta = e.y;
-        }
     } else {
         tgt_init(T, 0.0, 0.0, 0.5);
         T.live = false;
     }
-    double ax = 0.0, ay = 0.0, az = 0.0;  // PP/PC sums, before the target factor (proxy targets in FORM 1: Cartesian)
-    double ux = 0.0, uy = 0.0, uz = 0.0;  // DOWN sums (FORM 0: east/north; FORM 1: Cartesian)
+    mt[0] = -2.0 * T.x;
+    mt[1] = -2.0 * T.y;
+    mt[2] = -2.0 * T.z;
+    const bool work = active && (T.live || cart);
     if (tid == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
+        for (int i = 0; i < kRing; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], kEvalThreads / 32);
+        }
         fence_mbar_init();
-        tout = 0;
+        abort_ = 0;
     }
     __syncthreads();
-    const int ni = G.ie - G.ib;
-    const uint32_t polls = a.polls ? a.polls : kDefaultPolls;
+    // warp 0: stage k's copies, once every warp is through with the stage that
+    // last used its buffer.  Nothing is issued after a wait gave up.
+    int issued = 0;
     auto issue = [&](int k) {
-        // fault injection (tests of the time-out path): the group's last copy
+        const int b = k % kRing;
+        if (k >= kRing && !*abort &&
+            !mbar_wait_bounded(&empty[b], (uint32_t)((k / kRing - 1) & 1), a.err, kDefaultPolls))
+            *abort = 1;
+        // fault injection (tests of the time-out path): the unit's last stage
         // is never issued, so its wait runs out with no copy in flight
-        if (a.skip_last && k == ni - 1) return;
-        const Item it = a.items[G.ib + k];
-        const void *src;
-        uint32_t bytes;
-        if (it.kind == 2) {
-            src = a.records + (size_t)it.off * a.rec_stride;
-            bytes = (uint32_t)a.rec_stride * 8u;
-        } else {
-            src = a.pool + it.off;
-            bytes = (uint32_t)it.cnt * 32u;
-        }
-        uint64_t *b = &bar[k & 1];
+        if (__any_sync(0xffffffffu, k >= nissue || *abort)) return;
+        issued = k + 1;
         fence_proxy_async();
-        mbar_expect_tx(b, bytes);
-        bulk_g2s(buf[k & 1], src, bytes, b);
+        const EvalStage S = a.stages[sb + k];
+        if (lane == 0) mbar_expect_tx(&full[b], (uint32_t)S.cnt * 32u);
+        __syncwarp();
+        if (lane < S.ie - S.ib) {
+            const EvalItem it = a.items[S.ib + lane];
+            bulk_g2s(&buf[b][it.dst], a.pool + it.off, (uint32_t)it.cnt * 32u, &full[b]);
+        }
+        __syncwarp();
     };
-    if (tid == 0 && ni > 0) issue(0);
-    const int n = a.d + 1;
-    for (int k = 0; k < ni; ++k) {
-        if (tid == 0 && k + 1 < ni) issue(k + 1);
-        const Item it = a.items[G.ib + k];
-        if (!mbar_wait_bounded(&bar[k & 1], (uint32_t)((k >> 1) & 1), a.err, polls)) tout = 1;
-        const double4 *S = buf[k & 1];
-        if (it.kind == 2) {
-            if (TGT == 0 && active && sp == 0 && ((a.kinds >> 2) & 1)) {
-                // interp_vals_bli + the loops of fast_sum_module.f90:186-199
-                const double *R = reinterpret_cast<const double *>(S);
-                const double *nodes = R + 4 * a.P;
-                double fx[kMaxDegree + 1], fe[kMaxDegree + 1];
-                bli_basis(txi, nodes, n, fx);
-                bli_basis(teta, nodes + n, n, fe);
-                for (int kk = 0; kk < n; ++kk)
-                    for (int jj = 0; jj < n; ++jj) {
-                        const double bv = fx[jj] * fe[kk];
-                        const double4 ph = S[jj + kk * n];
-                        if (FORM == 0) {
-                            ux += bv * ph.x;
-                            uy += bv * ph.y;
-                        } else {
-                            ux += bv * ph.x;
-                            uy += bv * ph.y;
-                            uz += bv * ph.z;
-                        }
-                    }
-            }
-        } else if ((a.kinds >> it.kind) & 1) {
-            bool on = active && (T.live || (TGT == 1 && FORM == 1));
-            if (on && it.mask >= 0) on = (a.masks[it.mask + (ti >> 5)] >> (ti & 31)) & 1u;
-            if (on) {
-                if (TGT == 1 && FORM == 1) {
-                    for (int s = sp; s < it.cnt; s += nsplit) {
-                        const double4 q = S[s];
-                        const double dx = q.x - T.x, dy = q.y - T.y, dz = q.z - T.z;
-                        const double v = vstable(dx * dx + dy * dy + dz * dz) * q.w;
-                        ax += v * dx;
-                        ay += v * dy;
-                        az += v * dz;
-                    }
-                } else {
-                    for (int s = sp; s < it.cnt; s += nsplit) {
-                        const double4 q = S[s];
-                        gref_fast(T, q.x, q.y, q.z, q.w, ax, ay);
-                    }
+    if (warp == 0)
+        for (int k = 0; k < kAhead && k < ns; ++k) issue(k);
+    double A[3] = {0.0, 0.0, 0.0};   // far pairs: Sum val w s; Cartesian proxies: Sum val w (s - x)
+    double ax = 0.0, ay = 0.0;       // near pairs
+    for (int k = 0; k < ns; ++k) {
+        if (warp == 0 && k + kAhead < ns) issue(k + kAhead);
+        const int b = k % kRing;
+        const EvalStage S = a.stages[sb + k];
+        if (!*abort && !mbar_wait_bounded(&full[b], (uint32_t)((k / kRing) & 1), a.err, polls)) *abort = 1;
+        const double4 *src = buf[b];
+        // several pairs at a time: independent chains
+        auto range = [&](int beg, int end) {
+            int s = beg + sp;
+            if (cart) {
+                for (; s < end; s += nsplit) {
+                    const double4 q = src[s];
+                    const double dx = q.x - T.x, dy = q.y - T.y, dz = q.z - T.z;
+                    const double v = vstable(fma(dx, dx, fma(dy, dy, dz * dz))) * q.w;
+                    A[0] = fma(v, dx, A[0]);
+                    A[1] = fma(v, dy, A[1]);
+                    A[2] = fma(v, dz, A[2]);
                 }
+            } else if (S.flags & kEvalNear) {
+                for (; s + (kNearIlp - 1) * nsplit < end; s += kNearIlp * nsplit) gref_near<kNearIlp>(T, src + s, nsplit, ax, ay);
+                for (; s < end; s += nsplit) gref_near<1>(T, src + s, nsplit, ax, ay);
+            } else {
+                for (; s + (kIlp - 1) * nsplit < end; s += kIlp * nsplit) {
+#pragma unroll
+                    for (int u = 0; u < kIlp; ++u) gref_far(mt, src[s + u * nsplit], A);
+                }
+                for (; s < end; s += nsplit) gref_far(mt, src[s], A);
+            }
+        };
+        if (!(S.flags & kEvalMasked)) {
+            if (work) range(0, S.cnt);
+        } else {
+            for (int i = S.ib; i < S.ie; ++i) {
+                const EvalItem it = a.items[i];
+                if (work && ((a.masks[it.mask + (ti >> 5)] >> (ti & 31)) & 1u)) range(it.dst, it.dst + it.cnt);
             }
         }
-        __syncthreads();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[b]);
     }
-    if (!(TGT == 1 && FORM == 1)) {
-        // the target factor 1/sqrt(1 - tz^2) of every pair sum (zero outside the pole guard)
-        ax *= T.live ? T.inv_mp2 : 0.0;
-        ay *= T.live ? T.inv_mp2 : 0.0;
+    // the kernel's constant; leaves and reference proxies: the projection of
+    // the far pairs' vector and the target factor 1/sqrt(1 - tz^2) (zero
+    // inside the pole guard)
+    if (cart) {
+        ax = kCons * A[0];
+        ay = kCons * A[1];
+        A[2] *= kCons;
+    } else {
+        const double tf = T.live ? kCons * T.inv_mp2 : 0.0;
+        ax = tf * (ax + (T.x * A[1] - T.y * A[0]));
+        ay = tf * (ay + (T.omx32 * A[2] - T.z * (T.x * A[0] + T.y * A[1])));
+        A[2] = 0.0;
     }
-    if (TGT == 0 && FORM == 0) {
-        ax += ux;
-        ay += uy;
+    __syncthreads();   // every stage is consumed: the ring holds the reduction
+    double *red = reinterpret_cast<double *>(buf);
+    if (active) {
+        red[3 * tid] = ax;
+        red[3 * tid + 1] = ay;
+        red[3 * tid + 2] = A[2];
     }
-    if (TGT == 0 && FORM == 1 && active && sp == 0 && T.live) {
-        // project the interpolated Cartesian sum on the target's east/north frame
-        ax += (T.x * uy - T.y * ux) * T.inv_mp2;
-        ay += (uz * T.omx32 - T.z * (T.x * ux + T.y * uy)) * T.inv_mp2;
+    if (*abort && tid == 0) {
+        // a wait gave up: copies still in flight get a last bounded wait
+        // before their buffers go (their values are lost anyway)
+        for (int k = max(0, issued - kRing); k < issued; ++k)
+            mbar_wait_bounded(&full[k % kRing], (uint32_t)((k / kRing) & 1), a.err, kDefaultPolls);
     }
-    red[0][tid] = ax;
-    red[1][tid] = ay;
-    red[2][tid] = az;
     __syncthreads();
     if (active && sp == 0) {
         double rx = 0.0, ry = 0.0, rz = 0.0;
         for (int s = 0; s < nsplit; ++s) {
-            rx += red[0][s * ntp + ti];
-            ry += red[1][s * ntp + ti];
-            rz += red[2][s * ntp + ti];
+            rx += red[3 * (s * nt + ti)];
+            ry += red[3 * (s * nt + ti) + 1];
+            rz += red[3 * (s * nt + ti) + 2];
         }
-        if (TGT == 0) {
-            const int idx = a.perm[G.tgt + ti];
+        if (U.proxy) {
+            a.proxy_part[(size_t)U.out * a.P + ti] = make_double4(rx, ry, rz, 0.0);
+        } else if (U.out >= 0) {
+            a.leaf_part[(size_t)U.out + ti] = make_double2(rx, ry);
+        } else {
+            const int idx = a.perm[U.tgt + ti];
             a.out_x[idx] = rx;
             a.out_y[idx] = ry;
-        } else {
-            a.partial[(size_t)G.out * a.P + ti] = make_double4(rx, ry, rz, 0.0);
         }
     }
-    if (tout && tid == 0) {
-        // a copy timed out: give any copy still in flight a last bounded wait
-        for (int k = max(0, ni - 2); k < ni; ++k) mbar_wait_bounded(&bar[k & 1], (uint32_t)((k >> 1) & 1), a.err, polls);
-    }
+}
+static_assert(sizeof(double) * 3 * kEvalThreads <= sizeof(double4) * kRing * kMaxStage, "the reduction fits the ring");
+
+void launch_eval(int form, const EvalArgs &a, int nunits, cudaStream_t st) {
+    if (nunits <= 0) return;
+    if (form == 0) eval_kernel<0><<<nunits, kEvalThreads, 0, st>>>(a);
+    else eval_kernel<1><<<nunits, kEvalThreads, 0, st>>>(a);
 }
 
-void launch_eval(int tgt_kind, int form, const EvalArgs &a, int ngroups, cudaStream_t st) {
-    if (ngroups <= 0) return;
-    if (tgt_kind == 0 && form == 0) eval_kernel<0, 0><<<ngroups, kThreads, 0, st>>>(a);
-    else if (tgt_kind == 0) eval_kernel<0, 1><<<ngroups, kThreads, 0, st>>>(a);
-    else if (form == 0) eval_kernel<1, 0><<<ngroups, kThreads, 0, st>>>(a);
-    else eval_kernel<1, 1><<<ngroups, kThreads, 0, st>>>(a);
+// ------------------------------------------------------------------ leaf ends
+// One CTA per leaf: its units' partial sums in unit order, plus the
+// interpolation of its target slots' proxy potentials (interp_vals_bli and
+// the loops of fast_sum_module.f90:186-199).  FORM 0 interpolates east/north
+// components, FORM 1 the Cartesian vector, projected on the target's frame.
+// Thread tid has target tid % nt and the eta rows tid / nt, + nsplit, ... of
+// every slot, whose record (potentials, nodes) the CTA copies to shared
+// memory.
+constexpr int kFinThreads = 256;
+template <int N, int FORM>
+__global__ void __launch_bounds__(kFinThreads) leaf_fin_kernel(FinArgs a) {
+    constexpr int P = N * N;
+    __shared__ double4 rec[P + (2 * N + 3) / 4];
+    __shared__ double red[3][kFinThreads];
+    const LeafFin L = a.fin[blockIdx.x];
+    const int tid = threadIdx.x, nt = L.nt, nsplit = kFinThreads / nt, ti = tid % nt, sp = tid / nt;
+    const bool active = sp < nsplit;
+    const double2 xe = active ? a.xieta[L.tgt + ti] : make_double2(0.0, 0.0);
+    double ux = 0.0, uy = 0.0, uz = 0.0;
+    for (int e = L.db; e < L.de; ++e) {
+        const double4 *src = reinterpret_cast<const double4 *>(a.records + (size_t)a.down_slots[e] * a.rec_stride);
+        __syncthreads();
+        for (int i = tid; i < a.rec_stride / 4; i += kFinThreads) rec[i] = src[i];
+        __syncthreads();
+        if (active) {
+            const double *nodes = reinterpret_cast<const double *>(rec + P);
+            double fx[N], fe[N];
+            bli_basis_n<N>(xe.x, nodes, fx);
+            bli_basis_n<N>(xe.y, nodes + N, fe);
+            int turn = sp;   // eta row k is this thread's when turn is 0
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                if (turn == 0) {
+                    double rx = 0.0, ry = 0.0, rz = 0.0;
+#pragma unroll
+                    for (int j = 0; j < N; ++j) {
+                        const double4 ph = rec[j + k * N];
+                        rx = fma(fx[j], ph.x, rx);
+                        ry = fma(fx[j], ph.y, ry);
+                        if (FORM == 1) rz = fma(fx[j], ph.z, rz);
+                    }
+                    ux = fma(fe[k], rx, ux);
+                    uy = fma(fe[k], ry, uy);
+                    if (FORM == 1) uz = fma(fe[k], rz, uz);
+                    turn = nsplit;
+                }
+                --turn;
+            }
+        }
+    }
+    red[0][tid] = ux;
+    red[1][tid] = uy;
+    if (FORM == 1) red[2][tid] = uz;
+    __syncthreads();
+    if (!active || sp != 0) return;
+    for (int s = 1; s < nsplit; ++s) {
+        ux += red[0][s * nt + ti];
+        uy += red[1][s * nt + ti];
+        if (FORM == 1) uz += red[2][s * nt + ti];
+    }
+    if (FORM == 1) {
+        const double4 c = a.pool[L.tgt + ti];
+        Tgt T;
+        tgt_init(T, c.x, c.y, c.z);
+        const double tf = T.live ? T.inv_mp2 : 0.0;
+        const double ex = (T.x * uy - T.y * ux) * tf;
+        uy = (uz * T.omx32 - T.z * (T.x * ux + T.y * uy)) * tf;
+        ux = ex;
+    }
+    for (int k = 0; k < L.parts; ++k) {
+        const double2 v = a.leaf_part[(size_t)L.part + (size_t)k * nt + ti];
+        ux += v.x;
+        uy += v.y;
+    }
+    const int idx = a.perm[L.tgt + ti];
+    a.out_x[idx] = ux;
+    a.out_y[idx] = uy;
+}
+
+template <int N>
+static void launch_leaf_fin_n(int form, const FinArgs &a, int nfin, cudaStream_t st) {
+    if (form == 0) leaf_fin_kernel<N, 0><<<nfin, kFinThreads, 0, st>>>(a);
+    else leaf_fin_kernel<N, 1><<<nfin, kFinThreads, 0, st>>>(a);
+}
+
+void launch_leaf_fin(int form, int d, const FinArgs &a, int nfin, cudaStream_t st) {
+    if (nfin <= 0) return;
+    SAL_DEGREE_DISPATCH(launch_leaf_fin_n, d, form, a, nfin, st)
 }
 
 // Sums each target slot's unit partials in unit order into its record.

@@ -33,6 +33,9 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                  : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 // Bulk (non-tensor) TMA copy global -> this CTA's shared memory, completing
 // on an mbarrier.  No multicast.  Both addresses 16-byte aligned, bytes a
 // multiple of 16.
@@ -119,67 +122,134 @@ __device__ __forceinline__ void gref_exact(const Tgt &t, double sx, double sy, d
     gx = __dmul_rn(__dmul_rn(nx, t.inv_mp2), val);
 }
 
-// Reciprocal and square root for the treecode's inner loops: an FP32
-// hardware approximation refined by Newton-Raphson iterations in FP64
-// (reciprocal: r <- r + r(1 - x r), twice; square root: one step of the
-// inverse-square-root iteration y <- y(3 - x y^2)/2, then one Heron step
-// s <- s + y(x - s^2)/2), accurate to about one ulp.  Valid for
-// 1e-37 < |x| < 1e37 (fast_rcp) and x == 0 or 1e-37 < x < 1e37 (fast_sqrt),
-// the ranges their callers produce.
+// Reciprocal and inverse square root for the treecode's inner loops: the
+// hardware's FP64 approximation (about 20 good bits, no conversion to FP32 and
+// back, which costs four conversions a pair on the SFU's pipe), refined by one
+// step of Householder's third-order iteration, whose error is the cube of the
+// seed's: for 1/x, r (1 + e + e^2) with e = 1 - x r; for 1/sqrt(x),
+// y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2.  Accurate to about one ulp for
+// normal x whose reciprocal (square root) is normal; 0, infinities and NaN do
+// not give IEEE results, and callers keep them away.
 __device__ __forceinline__ double fast_rcp(double x) {
-    float xf = __double2float_rn(x), rf;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(xf));
-    double r = (double)rf;
-    double e = fma(-x, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-x, r, 1.0);
-    return fma(r, e, r);
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
 }
-__device__ __forceinline__ double fast_sqrt(double x) {
-    float xf = __double2float_rn(x), yf;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(xf));
-    double y = (double)yf;
-    double h = 0.5 * x;
-    y = y * fma(-h * y, y, 1.5);
-    double s = x * y;
-    s = fma(fma(-s, s, x), 0.5 * y, s);
-    return x > 0.0 ? s : 0.0;
+__device__ __forceinline__ double fast_rsqrt(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(fma(e, 0.375, 0.5), y * e, y);
 }
 
-// The reference kernel as the treecode evaluates it: g, mp = 2 - 2g, the two
-// denominators and the two numerators in the reference's exact operation
-// order (these carry the cancellations that make the self pair pure rounding
-// noise), p1 + p2 over one common denominator, and the target factor
-// 1/sqrt(1 - tz^2) left to the caller (applied once per target).  Adds the
-// un-normalised (nx, ny) * val * w into (ax, ay).
-__device__ __forceinline__ void gref_fast(const Tgt &t, double sx, double sy, double sz, double w, double &ax,
-                                          double &ay) {
-    double gxy = __dadd_rn(__dmul_rn(t.x, sx), __dmul_rn(t.y, sy));
-    double g = __dadd_rn(gxy, __dmul_rn(t.z, sz));
+// The kernel's scalar val / kCons as a function of mp = 2 - 2g alone.  With
+// q = sqrt(mp): 2g + q = (2 - q)(1 + q) and 2(g^2 - 1) = -mp (2 - q)(2 + q)/2,
+// so p1 + p2 = [kC1 - 2 kC2 q (1 + q)/(2 + q)] / q^3 and
+// q (1 + q)/(2 + q) = q - 1 + 2/(2 + q): one inverse square root and one
+// reciprocal, and no cancellation.  kReg: p1's + 1e-16 to first order
+// (1/(q^3 + c) = 1/q^3 - c/q^6); p2's is below 2e-13 of the value for
+// q > 1e-3.  22 FP64 instructions against 31 of the two denominators' form.
+template <bool kReg>
+__device__ __forceinline__ double val_chord(double mp) {
+    const double y = fast_rsqrt(mp);
+    const double q = mp * y;
+    const double r = fast_rcp(q + 2.0);
+    double f = fma(-2.0 * kC2, q, kC1 + 2.0 * kC2);
+    f = fma(-4.0 * kC2, r, f);
+    const double y3 = y * y * y;
+    if (kReg) f = fma(-1e-16 * kC1, y3, f);
+    return f * y3;
+}
+
+// Where val_chord<true> stands for the reference's expressions: q >= 1e-3
+// (the second-order term of the + 1e-16 is below 1e-14 of the value) and off
+// the antipode, where the reference's (2g + q) and (g^2 - 1) cancel to
+// rounding noise that has to be reproduced.  False for NaN.
+__device__ __forceinline__ bool chord_plain(double mp) { return mp >= 1e-6 && mp <= 3.99; }
+
+// sal_grad_gfunc's val / kCons in the reference's operation order: g clamped,
+// mp = 2 - 2g, the two denominators and the two numerators (these carry the
+// cancellations that make the self pair pure rounding noise), p1 + p2 over one
+// common denominator.
+__device__ __forceinline__ double val_ref(double g) {
     g = fmax(fmin(g, 1.0), -1.0);
-    double g2 = __dmul_rn(2.0, g);
-    double mp = __dsub_rn(2.0, g2);
-    double sqp = fast_sqrt(mp);
-    double d1 = __dadd_rn(__dmul_rn(sqp, mp), 1e-16);
-    double n2 = __dmul_rn(kC2, __dadd_rn(g2, sqp));
-    double d2 = __dadd_rn(__dmul_rn(2.0, __dsub_rn(__dmul_rn(g, g), 1.0)), 1e-16);
-    double val = fma(kC1, d2, n2 * d1) * fast_rcp(d1 * d2) * (kCons * w);
-    double ny = __dsub_rn(__dmul_rn(sz, t.omx32), __dmul_rn(t.z, gxy));
-    double nx = __dsub_rn(__dmul_rn(t.x, sy), __dmul_rn(t.y, sx));
-    ax = fma(nx, val, ax);
-    ay = fma(ny, val, ay);
+    const double g2 = __dmul_rn(2.0, g);
+    const double mp = __dsub_rn(2.0, g2);
+    const double sqp = __dsqrt_rn(mp);
+    const double d1 = __dadd_rn(__dmul_rn(sqp, mp), 1e-16);
+    const double n2 = __dmul_rn(kC2, __dadd_rn(g2, sqp));
+    const double d2 = __dadd_rn(__dmul_rn(2.0, __dsub_rn(__dmul_rn(g, g), 1.0)), 1e-16);
+    return __ddiv_rn(fma(kC1, d2, n2 * d1), d1 * d2);
 }
 
-// The scalar val of the kernel with its removable antipodal singularity
-// cancelled analytically (q = |t - s|):  2g + q = (2 - q)(1 + q) and
-// 2(g^2 - 1) = -q^2 (2 - q)(2 + q)/2, so p2 = -2 * 8.7 * (1 + q) / (q^2 (2 + q)).
-// mp = q^2 comes from coordinate differences, not from 2 - 2 t.s.
+// K pairs of the reference kernel (sources s[0], s[stride], ...) as the
+// treecode evaluates them: g and 2 - 2g in the reference's operation order,
+// then val_chord, K independent chains side by side; or, if any of the K is
+// one of the rare pairs (the self pair, near duplicates, antipodes) whose
+// value is the reference's rounding noise, one after another with val_ref for
+// those.  Adds (nx, ny) val w / kCons into (ax, ay); the constant and the
+// target factor 1/sqrt(1 - tz^2) are applied once per target.
+template <int K>
+__device__ __forceinline__ void gref_near(const Tgt &t, const double4 *s, int stride, double &ax, double &ay) {
+    double gxy[K], g[K], mp[K];
+    bool plain = true;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const double4 q = s[k * stride];
+        gxy[k] = __dadd_rn(__dmul_rn(t.x, q.x), __dmul_rn(t.y, q.y));
+        g[k] = __dadd_rn(gxy[k], __dmul_rn(t.z, q.z));
+        mp[k] = fma(-2.0, g[k], 2.0);   // 2 g is exact: rounds as 2 - 2g
+        plain = plain && chord_plain(mp[k]);
+    }
+    if (plain) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const double4 q = s[k * stride];
+            const double val = val_chord<true>(mp[k]) * q.w;
+            ax = fma(fma(-t.y, q.x, t.x * q.y), val, ax);
+            ay = fma(fma(-t.z, gxy[k], q.z * t.omx32), val, ay);
+        }
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < K; ++k) {
+            const double4 q = s[k * stride];
+            const double gk = __dadd_rn(__dadd_rn(__dmul_rn(t.x, q.x), __dmul_rn(t.y, q.y)), __dmul_rn(t.z, q.z));
+            const double m = fma(-2.0, gk, 2.0);
+            const double val = (chord_plain(m) ? val_chord<true>(m) : val_ref(gk)) * q.w;
+            const double nx = __dsub_rn(__dmul_rn(t.x, q.y), __dmul_rn(t.y, q.x));
+            const double ny = __dsub_rn(__dmul_rn(q.z, t.omx32),
+                                        __dmul_rn(t.z, __dadd_rn(__dmul_rn(t.x, q.x), __dmul_rn(t.y, q.y))));
+            ax = fma(nx, val, ax);
+            ay = fma(ny, val, ay);
+        }
+    }
+}
+
+// A pair that EvalBounds has shown to be plain: the dot product fused, and
+// Sum val w s as a vector, from which the two components follow once per
+// target (nx = tx Ay - ty Ax, ny = (1 - tz^2) Az - tz (tx Ax + ty Ay)).  The
+// vector cancels by the chord on projection, and no chord is below 0.012, so
+// its rounding stays below 1e-13 of a sum of thousands of pairs.  mt = -2 t.
+// 21 FP64 instructions against 29 of gref_near's plain branch.
+__device__ __forceinline__ void gref_far(const double (&mt)[3], const double4 &s, double (&A)[3]) {
+    const double mp = fma(mt[0], s.x, fma(mt[1], s.y, fma(mt[2], s.z, 2.0)));
+    const double v = val_chord<false>(mp) * s.w;
+    A[0] = fma(v, s.x, A[0]);
+    A[1] = fma(v, s.y, A[1]);
+    A[2] = fma(v, s.z, A[2]);
+}
+
+// val / kCons with its removable antipodal singularity cancelled analytically
+// (val_chord's form) for mp = q^2 from coordinate differences, not from
+// 2 - 2 t.s.  Pairs closer than 1e-3 keep the two + 1e-16 of the denominators
+// (a source on the target gives a finite value, times a zero displacement).
 __device__ __forceinline__ double vstable(double mp) {
-    double q = fast_sqrt(mp);
-    double d1 = q * mp + 1e-16;
-    double d2 = mp * (2.0 + q) + 1e-16;
-    double num = kC1 * d2 - 2.0 * kC2 * (1.0 + q) * d1;
-    return kCons * num * fast_rcp(d1 * d2);
+    if (mp >= 1e-6) return val_chord<true>(mp);
+    const double q = __dsqrt_rn(mp);
+    const double d1 = q * mp + 1e-16;
+    const double d2 = mp * (2.0 + q) + 1e-16;
+    return __ddiv_rn(kC1 * d2 - 2.0 * kC2 * (1.0 + q) * d1, d1 * d2);
 }
 
 // bli_coeffs, bli_module.f90:6-26 (0-based index i0 of degree d).
@@ -210,23 +280,53 @@ __device__ __forceinline__ void bli_basis(double x, const double *nodes, int n, 
     }
 }
 
+// bli_basis for N = d + 1 nodes in registers, with fast_rcp for the divisions.
+template <int N>
+__device__ __forceinline__ void bli_basis_n(double x, const double *nodes, double (&f)[N]) {
+    double denom = 0.0;
+    int at = -1;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const double dx = __dsub_rn(x, nodes[i]);
+        if (fabs(dx) < 1e-16) at = i;
+        const double c = (i & 1 ? -1.0 : 1.0) * (i == 0 || i == N - 1 ? 0.5 : 1.0);
+        f[i] = c * fast_rcp(dx);
+        denom += f[i];
+    }
+    const double r = fast_rcp(denom);
+#pragma unroll
+    for (int i = 0; i < N; ++i) f[i] = at < 0 ? f[i] * r : (i == at ? 1.0 : 0.0);
+}
+
 // ----------------------------------------------------------------- argument blocks
 struct EvalArgs {
-    const double4 *pool;     // sources: points then source proxies, (x, y, z, w)
-    const Group *groups;
-    const Item *items;
+    const double4 *pool;     // sources: points then source proxies, (x, y, z, w); leaf targets
+    const EvalUnit *units;   // of this launch, one CTA each
+    const EvalStage *stages;
+    const EvalItem *items;
     const uint32_t *masks;
-    const double4 *tgt;      // targets: the pool (leaf groups) or target proxies (proxy groups)
-    const double2 *xieta;    // per pool position (leaf groups)
-    const double *records;   // DOWN records, rec_stride doubles each
-    int rec_stride, d, P;
-    int kinds;               // bit k set: evaluate items of kind k (0 PP, 1 PC, 2 DOWN)
+    const double4 *tgt_proxy;   // P target proxies per target slot
+    int P;
+    int kinds;               // leaf units: bit k set evaluates sources of kind k (0 points, 1 proxies)
     const int32_t *perm;     // pool position -> caller index
-    double *out_x, *out_y;   // leaf groups: caller order, overwritten
-    double4 *partial;        // proxy groups: P outputs per unit
+    double *out_x, *out_y;   // caller order, overwritten (leaf units with out < 0)
+    double2 *leaf_part;      // leaf units' partial sums (x, y)
+    double4 *proxy_part;     // proxy units' partial sums, P per unit
     int *err;
     uint32_t polls;          // poll limit of every staging wait (0: kDefaultPolls)
-    int skip_last;           // fault injection: the last item's copy of every group is not issued
+    int skip_last;           // fault injection: the last stage's copies of every leaf unit are not issued
+};
+
+struct FinArgs {
+    const LeafFin *fin;
+    const int32_t *down_slots;
+    const double4 *pool;     // leaf targets
+    const double2 *xieta;    // per pool position
+    const double *records;   // DOWN records, rec_stride doubles each
+    int rec_stride;
+    const double2 *leaf_part;
+    const int32_t *perm;
+    double *out_x, *out_y;
 };
 
 struct UpArgs {
@@ -234,17 +334,17 @@ struct UpArgs {
     const double2 *xieta;
     const UpUnit *units;
     const double *nodes;     // per source slot 2(d+1) nodes
-    int d, P;
     double *partial;         // P per unit
 };
 
 // launches (implemented in kernels.cu)
 void launch_prep(const double4 *xyz, const double *area, const double *ssh, const int32_t *perm, int n, double4 *pool,
                  cudaStream_t st);
-void launch_upward(const UpArgs &a, int nunits, cudaStream_t st);
+void launch_upward(const UpArgs &a, int d, int nunits, cudaStream_t st);
 void launch_upward_finalize(const int32_t *unit_beg, const double *partial, int nslots, int d, int transposed,
                             double4 *pool_proxy, cudaStream_t st);
-void launch_eval(int tgt_kind, int form, const EvalArgs &a, int ngroups, cudaStream_t st);
+void launch_eval(int form, const EvalArgs &a, int nunits, cudaStream_t st);
+void launch_leaf_fin(int form, int d, const FinArgs &a, int nfin, cudaStream_t st);
 void launch_proxy_finalize(const int32_t *unit_beg, const double4 *partial, int nslots, int P, int rec_stride,
                            double *records, cudaStream_t st);
 void launch_direct(const double *xs, const double *ys, const double *zs, const double *w, int n,

@@ -76,8 +76,251 @@ static void push_range(std::vector<Item> &v, int64_t off, int64_t cnt, int kind,
     }
 }
 
-bool plan_build(const Tree &t, int d, int mode, const int32_t *list, int64_t nlist, const int32_t *pc, int64_t npc,
-                const int32_t *pp, int64_t npp, Plan *pl, std::string *err) {
+// A source of one target set in the FP64 pass: a panel's points (kind 0) or
+// proxies (kind 1), with the STT bitmask of the targets it acts on (-1: all).
+struct EvalSrc {
+    int32_t panel, kind, mask;
+};
+
+// Bounds that tell which panel pairs hold only plain pairs: per panel the
+// largest distance of its points and of its box (so of its proxies) from its
+// centre, and how far any |x|^2 is from 1.
+struct EvalBounds {
+    const Tree &t;
+    std::vector<double> rpts, rbox;
+    double eta = 0.0;
+    EvalBounds(const Tree &t_, const double *xs, const double *ys, const double *zs,
+               const std::vector<int32_t> &leaves, const std::vector<int64_t> &leaf_begin)
+        : t(t_) {
+        const int np = (int)t.p.size();
+        rpts.assign(np, 0.0);
+        rbox.assign(np, 0.0);
+        double worst = 0.0;
+        int bad = 0;
+#pragma omp parallel for schedule(static) reduction(max : worst) reduction(| : bad)
+        for (int64_t i = 0; i < (int64_t)t.n; ++i) {
+            const double e = std::fabs(xs[i] * xs[i] + ys[i] * ys[i] + zs[i] * zs[i] - 1.0);
+            if (e == e) worst = std::max(worst, e);
+            else bad |= 1;
+        }
+        eta = bad ? 1e300 : worst;
+#pragma omp parallel for schedule(dynamic, 64)
+        for (int k = 0; k < np; ++k) {
+            const Panel &q = t.p[k];
+            for (int c = 0; c < 4; ++c) {
+                double x, y, z;
+                xyz_from_xieta(c & 1 ? q.max_xi : q.min_xi, c & 2 ? q.max_eta : q.min_eta, q.face, &x, &y, &z);
+                rbox[k] = std::max(rbox[k], dist(k, x, y, z));
+            }
+            if (q.is_leaf)
+                for (int64_t p = q.begin; p < q.end; ++p) {
+                    const int32_t i = t.order[p];
+                    rpts[k] = std::max(rpts[k], dist(k, xs[i], ys[i], zs[i]));
+                }
+        }
+        // an inner panel's points are its leaves', contiguous in range order
+#pragma omp parallel for schedule(dynamic, 64)
+        for (int k = 0; k < np; ++k) {
+            const Panel &q = t.p[k];
+            if (q.is_leaf || q.count() == 0) continue;
+            const size_t lb = std::lower_bound(leaf_begin.begin(), leaf_begin.end(), q.begin) - leaf_begin.begin();
+            for (size_t l = lb; l < leaves.size() && leaf_begin[l] < q.end; ++l) {
+                const int c = leaves[l];
+                rpts[k] = std::max(rpts[k], rpts[c] + dist(k, t.cx[c], t.cy[c], t.cz[c]));
+            }
+        }
+    }
+    double dist(int k, double x, double y, double z) const {
+        const double a = x - t.cx[k], b = y - t.cy[k], c = z - t.cz[k];
+        return std::sqrt(a * a + b * b + c * c);
+    }
+    // 2 - 2 x.y = |x - y|^2 + (1 - |x|^2) + (1 - |y|^2): whether it can leave
+    // [1.5e-4, 3.96] for a target of panel kt (its points, or with `proxy` its
+    // proxies) and a source s.  Inside, the reference's operation order is not
+    // needed: a fused dot product's 2 - 2g is within 2e-16 / 1.5e-4 = 1.5e-12
+    // of the reference's at the nearest such pair (chord 0.012; with more than
+    // a thousand such pairs in a sum and nearer ones above them, below 2e-13
+    // of it), and neither the + 1e-16 nor the antipode is in reach.
+    bool near(int kt, bool proxy, const EvalSrc &s) const {
+        const double rt = proxy ? rbox[kt] : rpts[kt], rs = s.kind ? rbox[s.panel] : rpts[s.panel];
+        const double d = dist(kt, t.cx[s.panel], t.cy[s.panel], t.cz[s.panel]);
+        const double lo = d - rt - rs, hi = d + rt + rs;
+        return !(lo > 0.0 && lo * lo - 2.0 * eta >= 1.5e-4 && hi * hi + 2.0 * eta <= 3.96);
+    }
+};
+
+// Work of the FP64 evaluation pass: about kEvalUnits units of equal cost when
+// the grid is small (4 for each of 3 CTAs on 148 SMs, so the last wave is
+// short), but none below kEvalMinPairs pairs (a CTA's set-up costs about as
+// much as 4,000 pairs).
+static constexpr double kEvalUnits = 4.0 * 3 * 148, kEvalMinPairs = 16384.0;
+static constexpr double kEvalNearCost = 1.35;   // a near pair's cost in far pairs
+
+static void plan_build_eval(const Tree &t, const EvalBounds &bd, const std::vector<std::vector<EvalSrc>> &lsrc,
+                            const std::vector<std::vector<EvalSrc>> &tsrc,
+                            const std::vector<std::vector<int32_t>> &ldown, const std::vector<int32_t> &leaves,
+                            const std::vector<int32_t> &src_slot, Plan *pl) {
+    const int P = pl->P, ntgt = (int)tsrc.size();
+    const int64_t nl = (int64_t)leaves.size(), nsets = nl + ntgt;
+    const bool dtt = pl->mode == 0;
+    struct Set {
+        std::vector<EvalStage> stages;   // items relative to the set's own list
+        std::vector<EvalItem> items;
+        int32_t nt = 0, mid = 0;
+        double cost = 0.0;
+    };
+    auto cost_of = [&](const EvalStage &s, int32_t nt) {
+        return (double)s.cnt * nt * (s.flags & kEvalNear ? kEvalNearCost : 1.0);
+    };
+    std::vector<Set> sets(nsets);
+#pragma omp parallel for schedule(dynamic, 16)
+    for (int64_t x = 0; x < nsets; ++x) {
+        const bool proxy = x >= nl;
+        const int kt = proxy ? pl->tgt_slot_panel[x - nl] : leaves[x];
+        Set &S = sets[x];
+        S.nt = proxy ? P : (int32_t)t.p[kt].count();
+        struct Range { int32_t cls, off, cnt, mask; };
+        std::vector<Range> r;
+        for (const EvalSrc &e : proxy ? tsrc[x - nl] : lsrc[x]) {
+            const Panel &q = t.p[e.panel];
+            const int32_t off = e.kind ? (int32_t)(pl->n + (int64_t)src_slot[e.panel] * P) : (int32_t)q.begin;
+            const int32_t cnt = e.kind ? P : (int32_t)q.count();
+            // class: (STT: kind,) masked, near -- a stage holds one class, so
+            // that a solve can take one kind alone and a stage one kernel
+            const int32_t cls = (dtt ? 0 : 4 * e.kind) + (e.mask >= 0 ? 2 : 0) + (bd.near(kt, proxy, e) ? 1 : 0);
+            if (cnt > 0) r.push_back(Range{cls, off, cnt, e.mask});
+        }
+        std::sort(r.begin(), r.end(), [](const Range &a, const Range &b) {
+            return a.cls != b.cls ? a.cls < b.cls : a.off != b.off ? a.off < b.off : a.cnt < b.cnt;
+        });
+        EvalStage cur{0, 0, 0, 0};
+        int cls = -1;
+        auto flush = [&]() {
+            if (cur.ie > cur.ib) { S.stages.push_back(cur); S.cost += cost_of(cur, S.nt); }
+            cur = EvalStage{(int32_t)S.items.size(), (int32_t)S.items.size(), 0, 0};
+        };
+        for (const Range &g : r) {
+            if (g.cls != cls) {
+                flush();
+                if (cls < 4 && g.cls >= 4) S.mid = (int32_t)S.stages.size();
+                cls = g.cls;
+            }
+            int32_t off = g.off, left = g.cnt;
+            while (left > 0) {
+                if (cur.cnt == kMaxStage || cur.ie - cur.ib == kStageItems) flush();
+                cur.flags = (g.cls & 1 ? kEvalNear : 0) | (g.cls & 2 ? kEvalMasked : 0);
+                const int32_t c = std::min(left, kMaxStage - cur.cnt);
+                EvalItem *last = cur.ie > cur.ib ? &S.items.back() : nullptr;
+                if (last && g.mask < 0 && last->off + last->cnt == off) {
+                    last->cnt += c;   // the next range of the pool: one copy
+                } else {
+                    S.items.push_back(EvalItem{off, c, cur.cnt, g.mask});
+                    ++cur.ie;
+                }
+                cur.cnt += c;
+                off += c;
+                left -= c;
+            }
+        }
+        flush();
+        if (cls < 4) S.mid = (int32_t)S.stages.size();
+    }
+    double total = 0.0;
+    for (const Set &S : sets) total += S.cost;
+    const double target = std::max(kEvalMinPairs, total / kEvalUnits);
+    struct U { EvalUnit u; double cost; };
+    std::vector<U> pu, lu;
+    pl->eval_stages.clear();
+    pl->eval_items.clear();
+    pl->leaf_fin.clear();
+    pl->down_slots.clear();
+    pl->eval_proxy_unit_beg.assign(ntgt + 1, 0);
+    pl->leaf_part_rows = 0;
+    for (int64_t x = 0; x < nsets; ++x) {
+        const bool proxy = x >= nl;
+        const Set &S = sets[x];
+        const int32_t s0 = (int32_t)pl->eval_stages.size(), i0 = (int32_t)pl->eval_items.size();
+        const int32_t ns = (int32_t)S.stages.size();
+        for (EvalStage e : S.stages) {
+            e.ib += i0;
+            e.ie += i0;
+            pl->eval_stages.push_back(e);
+        }
+        pl->eval_items.insert(pl->eval_items.end(), S.items.begin(), S.items.end());
+        // units of about equal cost, whole stages each
+        const int32_t parts = std::max<int32_t>(proxy && ns == 0 ? 0 : 1,
+                                                (int32_t)std::min<double>(ns, std::floor(S.cost / target + 0.5)));
+        EvalUnit u{};
+        u.tgt = proxy ? (int32_t)(x - nl) : (int32_t)t.p[leaves[x]].begin;
+        u.nt = S.nt;
+        u.proxy = proxy;
+        LeafFin f{};
+        if (proxy) {
+            pl->eval_proxy_unit_beg[x - nl] = (int32_t)pu.size();
+        } else {
+            f.tgt = u.tgt;
+            f.nt = S.nt;
+            f.parts = parts;
+            f.db = (int32_t)pl->down_slots.size();
+            pl->down_slots.insert(pl->down_slots.end(), ldown[x].begin(), ldown[x].end());
+            f.de = (int32_t)pl->down_slots.size();
+            f.part = (int32_t)pl->leaf_part_rows;
+        }
+        const bool straight = !proxy && parts == 1 && f.db == f.de;
+        int32_t i = 0;
+        double done = 0.0;
+        for (int32_t k = 0; k < parts; ++k) {
+            const int32_t b = i;
+            double c = 0.0;
+            const double want = (S.cost - done) / (parts - k);
+            while (i < ns && (k == parts - 1 || ((c == 0.0 || c + 0.5 * cost_of(S.stages[i], S.nt) < want) &&
+                                                 ns - i > parts - 1 - k)))
+                c += cost_of(S.stages[i++], S.nt);
+            done += c;
+            u.sb = s0 + b;
+            u.se = s0 + i;
+            u.sm = s0 + std::min(std::max(S.mid, b), i);
+            if (proxy) {
+                u.out = (int32_t)pu.size();
+                pu.push_back(U{u, c});
+            } else {
+                u.out = straight ? -1 : f.part + k * S.nt;
+                lu.push_back(U{u, c});
+            }
+        }
+        if (!proxy && !straight) {
+            pl->leaf_fin.push_back(f);
+            pl->leaf_part_rows += (int64_t)parts * S.nt;
+        }
+    }
+    pl->eval_proxy_unit_beg[ntgt] = (int32_t)pu.size();
+    pl->n_proxy_eval = (int32_t)pu.size();
+    auto by_cost = [](const U &a, const U &b) { return a.cost > b.cost; };
+    std::stable_sort(pu.begin(), pu.end(), by_cost);
+    std::stable_sort(lu.begin(), lu.end(), by_cost);
+    pl->eval_units.clear();
+    for (const U &u : pu) pl->eval_units.push_back(u.u);
+    for (const U &u : lu) pl->eval_units.push_back(u.u);
+    // upward units: about the same number, 256 to 4096 points each
+    double rows = 0.0;
+    for (int32_t k : pl->src_slot_panel) rows += (double)t.p[k].count();
+    int64_t chunk = 256;
+    while (chunk < kUpChunk && rows / (double)chunk > kEvalUnits) chunk *= 2;
+    pl->up64_units.clear();
+    pl->up64_unit_beg.assign(pl->src_slot_panel.size() + 1, 0);
+    for (size_t s = 0; s < pl->src_slot_panel.size(); ++s) {
+        const Panel &q = t.p[pl->src_slot_panel[s]];
+        pl->up64_unit_beg[s] = (int32_t)pl->up64_units.size();
+        for (int64_t b = q.begin; b < q.end; b += chunk)
+            pl->up64_units.push_back(UpUnit{(int32_t)s, (int32_t)b, (int32_t)std::min<int64_t>(q.end, b + chunk),
+                                            pl->src_slot_panel[s]});
+    }
+    pl->up64_unit_beg[pl->src_slot_panel.size()] = (int32_t)pl->up64_units.size();
+}
+
+bool plan_build(const Tree &t, const double *xs, const double *ys, const double *zs, int d, int mode,
+                const int32_t *list, int64_t nlist, const int32_t *pc, int64_t npc, const int32_t *pp, int64_t npp,
+                Plan *pl, std::string *err) {
     if (d < 1 || d > kMaxDegree) { *err = "interp_degree must be in 1.." + std::to_string(kMaxDegree); return false; }
     const int n = t.n, np = (int)t.p.size(), nd = d + 1, P = nd * nd;
     pl->n = n; pl->d = d; pl->P = P; pl->mode = mode; pl->npanels = np;
@@ -150,6 +393,8 @@ bool plan_build(const Tree &t, int d, int mode, const int32_t *list, int64_t nli
     auto proxy_off = [&](int k) { return pool_proxy0 + (int64_t)src_slot[k] * P; };
     std::vector<std::vector<Item>> litems(leaves.size()), titems(ntgt);
     std::vector<double> lcost(leaves.size(), 0.0), tcost(ntgt, 0.0);
+    std::vector<std::vector<EvalSrc>> lsrc(leaves.size()), tsrc(ntgt);
+    std::vector<std::vector<int32_t>> ldown(leaves.size());
     pl->masks.clear();
     if (dtt) {
         for (int64_t i = 0; i < nlist; ++i) {
@@ -162,6 +407,7 @@ bool plan_build(const Tree &t, int d, int mode, const int32_t *list, int64_t nli
                 for (int32_t l = lb; l < le; ++l) {
                     if (ty == 0) push_range(litems[l], S.begin, S.count(), 0, -1);
                     else push_range(litems[l], proxy_off(k_s), P, 1, -1);
+                    lsrc[l].push_back(EvalSrc{k_s, ty, -1});
                     lcost[l] += (double)(ty == 0 ? S.count() : P) * t.p[leaves[l]].count();
                 }
                 pl->pairs[ty] += (double)T.count() * (ty == 0 ? S.count() : P);
@@ -169,6 +415,7 @@ bool plan_build(const Tree &t, int d, int mode, const int32_t *list, int64_t nli
                 int32_t ts = tgt_slot[k_t];
                 if (ty == 2) push_range(titems[ts], S.begin, S.count(), 0, -1);
                 else push_range(titems[ts], proxy_off(k_s), P, 1, -1);
+                tsrc[ts].push_back(EvalSrc{k_s, ty - 2, -1});
                 tcost[ts] += (double)P * (ty == 2 ? S.count() : P);
                 pl->pairs[ty] += (double)P * (ty == 2 ? S.count() : P);
             }
@@ -179,6 +426,7 @@ bool plan_build(const Tree &t, int d, int mode, const int32_t *list, int64_t nli
             leaf_range(pl->tgt_slot_panel[s], &lb, &le);
             for (int32_t l = lb; l < le; ++l) {
                 litems[l].push_back(Item{s, 0, -1, 2});
+                ldown[l].push_back(s);
                 lcost[l] += (double)P * t.p[leaves[l]].count() * 0.5;
             }
             pl->macs_down += (double)t.p[pl->tgt_slot_panel[s]].count() * P;
@@ -240,6 +488,11 @@ bool plan_build(const Tree &t, int d, int mode, const int32_t *list, int64_t nli
             double c = 0;
             for (int32_t a : ordk) {
                 int32_t k_s = keys[a] / 2, kind = keys[a] % 2;
+                // an item that every target of the leaf takes needs no mask
+                bool all = true;
+                for (int w = 0; w < words && all; ++w)
+                    all = mk[(size_t)a * words + w] == (w + 1 < words || nt % 32 == 0 ? ~0u : (1u << (nt % 32)) - 1u);
+                lsrc[l].push_back(EvalSrc{k_s, kind, all ? -1 : a * words});
                 if (kind == 0) push_range(litems[l], t.p[k_s].begin, t.p[k_s].count(), 0, a * words);
                 else push_range(litems[l], proxy_off(k_s), P, 1, a * words);
                 c += (double)(kind == 0 ? t.p[k_s].count() : P) * nt;
@@ -249,6 +502,8 @@ bool plan_build(const Tree &t, int d, int mode, const int32_t *list, int64_t nli
         for (size_t l = 0; l < leaves.size(); ++l) {
             int32_t base = (int32_t)pl->masks.size();
             for (auto &it : litems[l]) it.mask += base;
+            for (auto &e : lsrc[l])
+                if (e.mask >= 0) e.mask += base;
             pl->masks.insert(pl->masks.end(), lmask[l].begin(), lmask[l].end());
         }
         for (int64_t i = 0; i < npc; ++i) pl->pairs[1] += P;
@@ -310,6 +565,7 @@ bool plan_build(const Tree &t, int d, int mode, const int32_t *list, int64_t nli
         std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return ucost[a] > ucost[b]; });
         for (int32_t u : ord) pl->proxy_groups.push_back(units[u]);
     }
+    plan_build_eval(t, EvalBounds(t, xs, ys, zs, leaves, leaf_begin), lsrc, tsrc, ldown, leaves, src_slot, pl);
     pl->leaf_panel = leaves;
     pl->mix_built = false;
     if (dtt && !plan_build_tc(t, pl, TcOptions{}, err)) return false;

@@ -76,6 +76,32 @@ struct Group {           // a set of targets with one work list
     int32_t pad0, pad1, pad2;
 };
 
+// FP64 evaluation pass (kernels.cu eval_kernel).  A unit is a set of targets
+// (a leaf's points, or a target slot's proxies) with a run of stages; a stage
+// is up to kMaxStage sources gathered from up to kStageItems pool ranges,
+// which one CTA stages with that many bulk copies and consumes together.
+struct EvalItem {        // sources: pool rows [off, off + cnt), at position dst of the stage
+    int32_t off, cnt, dst;
+    int32_t mask;        // STT: word offset of the per-target bitmask, or -1 (every target)
+};
+struct EvalStage {
+    int32_t ib, ie;      // item range
+    int32_t cnt;         // sources
+    int32_t flags;       // kEvalNear | kEvalMasked
+};
+constexpr int32_t kEvalNear = 1;     // pairs that need the reference's operation order can be among these
+constexpr int32_t kEvalMasked = 2;   // items with bitmasks
+struct EvalUnit {
+    int32_t tgt, nt;     // first pool row (leaf) or target slot (proxies), number of targets
+    int32_t sb, sm, se;  // stages [sb, se); STT: [sb, sm) are point sources, [sm, se) proxies
+    int32_t out;         // leaf: row of the partial sums (-1: straight to the outputs); proxies: unit number
+    int32_t proxy;       // 1: proxy targets
+    int32_t pad0;
+};
+struct LeafFin {         // a leaf's end: partial sums of `parts` units, then DOWN interpolation from its slots
+    int32_t tgt, nt, part, parts, db, de;
+};
+
 struct UpUnit {          // upward-pass work unit
     int32_t slot, beg, end, panel;
 };
@@ -144,6 +170,19 @@ struct Plan {
     std::vector<Group> leaf_groups;               // one per leaf with targets, sorted by cost
     std::vector<Item> leaf_items;
     std::vector<uint32_t> masks;                  // STT per-target bitmasks
+    // FP64 passes: evaluation units (n_proxy_eval proxy units, then leaf
+    // units, each by descending cost), their stages and items, the leaves'
+    // ends with their DOWN slots, and the upward pass's own cut
+    std::vector<EvalUnit> eval_units;
+    std::vector<EvalStage> eval_stages;
+    std::vector<EvalItem> eval_items;
+    std::vector<LeafFin> leaf_fin;
+    std::vector<int32_t> down_slots;
+    std::vector<int32_t> eval_proxy_unit_beg;     // tgt slot -> first proxy unit (ntgt + 1)
+    int32_t n_proxy_eval = 0;
+    int64_t leaf_part_rows = 0;                   // rows of the leaves' partial sums
+    std::vector<UpUnit> up64_units;
+    std::vector<int32_t> up64_unit_beg;           // source slot -> first unit (nsrc + 1)
     // batched form: items of at most kMixStage sources (DOWN items: rows of
     // a target slot's potentials, off = slot, cnt = rows, mask = first row)
     std::vector<MixGroup> mix_leaf_groups, mix_proxy_groups, mix_up_groups;
@@ -206,8 +245,9 @@ struct Plan {
 };
 
 // Builds the plan of a DTT list (triplets) or STT lists (pairs).
-bool plan_build(const Tree &t, int d, int mode, const int32_t *list, int64_t nlist, const int32_t *pc, int64_t npc,
-                const int32_t *pp, int64_t npp, Plan *plan, std::string *err);
+bool plan_build(const Tree &t, const double *xs, const double *ys, const double *zs, int d, int mode,
+                const int32_t *list, int64_t nlist, const int32_t *pc, int64_t npc, const int32_t *pp, int64_t npp,
+                Plan *plan, std::string *err);
 // (Re)builds the tcgen05 part of a DTT plan for the given options.
 bool plan_build_tc(const Tree &t, Plan *plan, const TcOptions &opt, std::string *err);
 // the kernel-tile store's per-group offsets for one stored item in `every`
@@ -215,7 +255,8 @@ void plan_tile_offsets(Plan *plan, int every);
 // The 32-field (mma.sync) groups of the batched form, from a built plan.
 void plan_build_mix(const Tree &t, Plan *plan);
 
-constexpr int kMaxStage = 256;   // sources staged per item (items are split to fit)
+constexpr int kMaxStage = 256;   // sources per stage of the FP64 pass; plan items are split to fit
+constexpr int kStageItems = 32;  // pool ranges per stage of the FP64 pass (one lane of a warp copies each)
 constexpr int kMixStage = 64;    // sources (or DOWN rows) staged per batched item
 constexpr int kMixRows = 64;     // targets per batched CTA
 constexpr int kTcRows = 128;     // targets per tcgen05 leaf group (the MMA's M)

@@ -187,9 +187,7 @@ __device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
+using dev::mbar_arrive;
 // Bounded wait on an mbarrier phase; on time-out raises the error flag and
 // the CTA-wide abort flag (later waits then give up after one poll).  A phase
 // that has already completed costs one poll and no read of the flag: every
