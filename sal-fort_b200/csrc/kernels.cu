@@ -158,16 +158,26 @@ void launch_upward_finalize(const int32_t *unit_beg, const double *partial, int 
 // ranges; lane i of warp 0 copies range i (one bulk copy each, completing on
 // the stage's mbarrier) into a ring of kRing buffers, two stages ahead, so a
 // warp that is through with a stage goes on without a CTA-wide barrier.
-// Targets and source splits fill the threads without gaps: thread tid has
-// target tid % nt and sources tid / nt, tid / nt + nsplit, ...; the splits are
-// summed in a fixed order at the end, so results are deterministic.  Stages
+// Every warp has the same share of the unit's pairs: each target is taken F
+// times, each time for one residue of the sources mod F (F from the plan, so
+// that the nt F lanes fill up to one chunk of 32 lanes a warp with little
+// waste), and a last chunk of m <= 16 lanes takes 32 / m residues more.  The
+// (chunk, source) plane is cut into one equal run per warp: a fraction of the
+// sources of at most two chunks, the same ones in every stage, whose sums the
+// warp keeps.  (One thread per target and whole source splits left a leaf of
+// 148 targets with 5 of 8 warps at work, two of them on one scheduler: 62 % of
+// the FP64 pipe.)  The sums are added in a fixed order at the end, so results
+// are deterministic.  Stages
 // are near (gref_near: the reference's operation order where its rounding
 // noise counts) or far (gref_far).
 //   Leaf units and FORM 0 proxies: the reference kernel.  FORM 1 proxies: the
 //   Cartesian sum val (s - x) w with the antipode-stable val.
-// Bound by the FP64 pipe (two cycles an instruction and warp on each of the
-// four schedulers).
-constexpr int kEvalThreads = 256, kEvalCtas = 3, kIlp = 2, kNearIlp = 2, kRing = 4, kAhead = 2;
+// Bound by the FP64 pipe: an instruction with three register operands takes
+// about 2.5 cycles of a scheduler's pipe (50 for a far pair's 20, in a loop of
+// nothing else), and 8 pairs at a time on 4 warps a scheduler come closest to
+// that (24 warps of 80 registers and 4 pairs: 3 % slower).
+constexpr int kEvalThreads = 256, kEvalCtas = 2, kIlp = 8, kNearIlp = 4, kRing = 4, kAhead = 2, kSlots = 2;
+constexpr int kEvalWarps = kEvalThreads / 32;
 
 template <int FORM>
 __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs a) {
@@ -177,31 +187,52 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs 
     volatile int *abort = &abort_;
     const EvalUnit U = a.units[blockIdx.x];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nt = U.nt, nsplit = kEvalThreads / nt;
-    const int ti = tid % nt, sp = tid / nt;
-    const bool active = sp < nsplit;
     const bool cart = FORM == 1 && U.proxy;
     const int sb = (U.proxy || (a.kinds & 1)) ? U.sb : U.sm, se = (U.proxy || (a.kinds & 2)) ? U.se : U.sm;
     const int ns = se - sb;
     const uint32_t polls = a.polls ? a.polls : kDefaultPolls;
     const int nissue = (a.skip_last && !U.proxy) ? ns - 1 : ns;
-    Tgt T;
-    double mt[3] = {0.0, 0.0, 0.0};
-    if (active) {
-        const double4 c = U.proxy ? a.tgt_proxy[(size_t)U.tgt * a.P + ti] : a.pool[U.tgt + ti];
-        tgt_init(T, c.x, c.y, c.z);
-    } else {
-        tgt_init(T, 0.0, 0.0, 0.5);
-        T.live = false;
+    // chunks of 32 (target, residue) lanes; the last one's weight is 1 / (its
+    // residues side by side)
+    const int F = U.fold, nid = U.nt * F, nch = (nid + 31) >> 5, nlast = nid - 32 * (nch - 1), rlast = 32 / nlast;
+    const float wlast = 1.f / (float)rlast, per = ((float)(nch - 1) + wlast) * (1.f / kEvalWarps);
+    // this warp's run of the plane
+    const float lo = per * (float)warp, hi = per * (float)(warp + 1);
+    const int c0 = min((int)lo, nch - 1);
+    // the slots' state; a stage's range takes one slot into registers
+    struct Slot {
+        double x, y, z;            // the target
+        double A[3], ax, ay;       // sums: far pairs Sum val w s (Cartesian proxies Sum val w (s - x)); near pairs
+        float f0, f1, rstep;       // this run's fraction of the chunk's sources, 1 / step
+        int ti, res, step, work;   // target, residue and modulus of its sources
+    } slot[kSlots];
+#pragma unroll 1
+    for (int i = 0; i < kSlots; ++i) {
+        const int c = c0 + i;
+        const bool last = c == nch - 1;
+        const int n = last ? nlast : 32, l = lane % n, id = 32 * c + l;
+        const float base = (float)c, wc = last ? wlast : 1.f;
+        Slot w{};
+        w.step = last ? F * rlast : F;
+        w.rstep = 1.f / (float)w.step;
+        w.ti = id % U.nt;
+        w.res = id / U.nt + F * (lane / n);
+        // neighbouring warps compute a shared boundary from the same numbers
+        w.f0 = lo <= base ? 0.f : fminf((lo - base) / wc, 1.f);
+        w.f1 = (warp == kEvalWarps - 1 || hi >= base + wc) ? 1.f : fmaxf((hi - base) / wc, 0.f);
+        if (c < nch && w.res < w.step && w.f0 < w.f1) {
+            const double4 q = U.proxy ? a.tgt_proxy[(size_t)U.tgt * a.P + w.ti] : a.pool[U.tgt + w.ti];
+            w.x = q.x;
+            w.y = q.y;
+            w.z = q.z;
+            w.work = cart || tgt_live(q.z);
+        }
+        slot[i] = w;
     }
-    mt[0] = -2.0 * T.x;
-    mt[1] = -2.0 * T.y;
-    mt[2] = -2.0 * T.z;
-    const bool work = active && (T.live || cart);
     if (tid == 0) {
         for (int i = 0; i < kRing; ++i) {
             mbar_init(&full[i], 1);
-            mbar_init(&empty[i], kEvalThreads / 32);
+            mbar_init(&empty[i], kEvalWarps);
         }
         fence_mbar_init();
         abort_ = 0;
@@ -231,67 +262,91 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs 
     };
     if (warp == 0)
         for (int k = 0; k < kAhead && k < ns; ++k) issue(k);
-    double A[3] = {0.0, 0.0, 0.0};   // far pairs: Sum val w s; Cartesian proxies: Sum val w (s - x)
-    double ax = 0.0, ay = 0.0;       // near pairs
     for (int k = 0; k < ns; ++k) {
         if (warp == 0 && k + kAhead < ns) issue(k + kAhead);
         const int b = k % kRing;
         const EvalStage S = a.stages[sb + k];
         if (!*abort && !mbar_wait_bounded(&full[b], (uint32_t)((k / kRing) & 1), a.err, polls)) *abort = 1;
         const double4 *src = buf[b];
-        // several pairs at a time: independent chains
-        auto range = [&](int beg, int end) {
-            int s = beg + sp;
-            if (cart) {
-                for (; s < end; s += nsplit) {
-                    const double4 q = src[s];
-                    const double dx = q.x - T.x, dy = q.y - T.y, dz = q.z - T.z;
-                    const double v = vstable(fma(dx, dx, fma(dy, dy, dz * dz))) * q.w;
-                    A[0] = fma(v, dx, A[0]);
-                    A[1] = fma(v, dy, A[1]);
-                    A[2] = fma(v, dz, A[2]);
+        const bool near = S.flags & kEvalNear, masked = S.flags & kEvalMasked;
+#pragma unroll 1
+        for (int i = 0; i < kSlots; ++i) {
+            if (!slot[i].work) continue;
+            const double x = slot[i].x, y = slot[i].y, z = slot[i].z;
+            const float f0 = slot[i].f0, f1 = slot[i].f1;
+            const int res = slot[i].res, step = slot[i].step, ti = slot[i].ti;
+            const float rstep = slot[i].rstep;
+            double A[3] = {slot[i].A[0], slot[i].A[1], slot[i].A[2]}, ax = slot[i].ax, ay = slot[i].ay;
+            // an unmasked stage is one run of sources, a masked one a run per item
+#pragma unroll 1
+            for (int v = masked ? S.ib : S.ie - 1; v < S.ie; ++v) {
+                int beg = 0, n = S.cnt;
+                if (masked) {
+                    const EvalItem it = a.items[v];
+                    if (!((a.masks[it.mask + (ti >> 5)] >> (ti & 31)) & 1u)) continue;
+                    beg = it.dst;
+                    n = it.cnt;
                 }
-            } else if (S.flags & kEvalNear) {
-                for (; s + (kNearIlp - 1) * nsplit < end; s += kNearIlp * nsplit) gref_near<kNearIlp>(T, src + s, nsplit, ax, ay);
-                for (; s < end; s += nsplit) gref_near<1>(T, src + s, nsplit, ax, ay);
-            } else {
-                for (; s + (kIlp - 1) * nsplit < end; s += kIlp * nsplit) {
-#pragma unroll
-                    for (int u = 0; u < kIlp; ++u) gref_far(mt, src[s + u * nsplit], A);
+                // this run's share of the blocks of `step` sources
+                const float nb = floorf(((float)(n + step) - 0.5f) * rstep);   // ceil(n / step), exact for n <= 256
+                int s = beg + (int)(nb * f0) * step + res;
+                const int e = min(beg + (int)(nb * f1) * step, beg + n);
+                if (cart) {
+                    for (; s + (kNearIlp - 1) * step < e; s += kNearIlp * step)
+                        cart_pairs<kNearIlp>(x, y, z, src + s, step, A);
+                    for (; s < e; s += step) cart_pairs<1>(x, y, z, src + s, step, A);
+                } else if (near) {
+                    Tgt T;
+                    T.x = x;
+                    T.y = y;
+                    T.z = z;
+                    T.omx32 = tgt_omx32(z);
+                    for (; s + (kNearIlp - 1) * step < e; s += kNearIlp * step) gref_near<kNearIlp>(T, src + s, step, ax, ay);
+                    for (; s < e; s += step) gref_near<1>(T, src + s, step, ax, ay);
+                } else {
+                    // several pairs at a time: independent chains
+                    const double mt[3] = {-2.0 * x, -2.0 * y, -2.0 * z};
+                    for (; s + (kIlp - 1) * step < e; s += kIlp * step) gref_far<kIlp>(mt, src + s, step, A);
+                    if (s + (kIlp / 2 - 1) * step < e) {
+                        gref_far<kIlp / 2>(mt, src + s, step, A);
+                        s += kIlp / 2 * step;
+                    }
+                    for (; s < e; s += step) gref_far<1>(mt, src + s, step, A);
                 }
-                for (; s < end; s += nsplit) gref_far(mt, src[s], A);
             }
-        };
-        if (!(S.flags & kEvalMasked)) {
-            if (work) range(0, S.cnt);
-        } else {
-            for (int i = S.ib; i < S.ie; ++i) {
-                const EvalItem it = a.items[i];
-                if (work && ((a.masks[it.mask + (ti >> 5)] >> (ti & 31)) & 1u)) range(it.dst, it.dst + it.cnt);
-            }
+            slot[i].A[0] = A[0];
+            slot[i].A[1] = A[1];
+            slot[i].A[2] = A[2];
+            slot[i].ax = ax;
+            slot[i].ay = ay;
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[b]);
     }
-    // the kernel's constant; leaves and reference proxies: the projection of
-    // the far pairs' vector and the target factor 1/sqrt(1 - tz^2) (zero
-    // inside the pole guard)
-    if (cart) {
-        ax = kCons * A[0];
-        ay = kCons * A[1];
-        A[2] *= kCons;
-    } else {
-        const double tf = T.live ? kCons * T.inv_mp2 : 0.0;
-        ax = tf * (ax + (T.x * A[1] - T.y * A[0]));
-        ay = tf * (ay + (T.omx32 * A[2] - T.z * (T.x * A[0] + T.y * A[1])));
-        A[2] = 0.0;
-    }
-    __syncthreads();   // every stage is consumed: the ring holds the reduction
-    double *red = reinterpret_cast<double *>(buf);
-    if (active) {
-        red[3 * tid] = ax;
-        red[3 * tid + 1] = ay;
-        red[3 * tid + 2] = A[2];
+    __syncthreads();   // every stage is consumed: the ring holds the warps' sums
+    double *red = reinterpret_cast<double *>(buf);   // [warp][slot][component][lane]
+#pragma unroll 1
+    for (int i = 0; i < kSlots; ++i) {
+        // the kernel's constant; leaves and reference proxies: the projection
+        // of the far pairs' vector and the target factor 1/sqrt(1 - tz^2)
+        // (zero inside the pole guard, and in slots without work)
+        const Slot &w = slot[i];
+        double rx = 0.0, ry = 0.0, rz = 0.0;
+        if (cart) {
+            rx = kCons * w.A[0];
+            ry = kCons * w.A[1];
+            rz = kCons * w.A[2];
+        } else if (w.work) {
+            Tgt T;
+            tgt_init(T, w.x, w.y, w.z);
+            const double tf = kCons * T.inv_mp2;
+            rx = tf * (w.ax + (T.x * w.A[1] - T.y * w.A[0]));
+            ry = tf * (w.ay + (T.omx32 * w.A[2] - T.z * (T.x * w.A[0] + T.y * w.A[1])));
+        }
+        double *o = red + ((warp * kSlots + i) * 3) * 32 + lane;
+        o[0] = rx;
+        o[32] = ry;
+        o[64] = rz;
     }
     if (*abort && tid == 0) {
         // a wait gave up: copies still in flight get a last bounded wait
@@ -300,25 +355,52 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs 
             mbar_wait_bounded(&full[k % kRing], (uint32_t)((k / kRing) & 1), a.err, kDefaultPolls);
     }
     __syncthreads();
-    if (active && sp == 0) {
-        double rx = 0.0, ry = 0.0, rz = 0.0;
-        for (int s = 0; s < nsplit; ++s) {
-            rx += red[3 * (s * nt + ti)];
-            ry += red[3 * (s * nt + ti) + 1];
-            rz += red[3 * (s * nt + ti) + 2];
+    // lane tid of the folded set: the warps whose runs meet its chunk, in
+    // order; then each target's F lanes, in order
+    double *fold = red + 3 * 32 * kSlots * kEvalWarps;
+    double rx = 0.0, ry = 0.0, rz = 0.0;
+    if (tid < nid) {
+        const int c = tid >> 5, n = c == nch - 1 ? nlast : 32, r = c == nch - 1 ? rlast : 1;
+        for (int v = 0; v < kEvalWarps; ++v) {
+            const int i = c - min((int)(per * (float)v), nch - 1);
+            if (i < 0 || i >= kSlots) continue;
+            const double *o = red + ((v * kSlots + i) * 3) * 32 + lane;
+            for (int k = 0; k < r; ++k) {
+                rx += o[k * n];
+                ry += o[k * n + 32];
+                rz += o[k * n + 64];
+            }
         }
+    }
+    if (F > 1) {
+        fold[tid] = rx;
+        fold[kEvalThreads + tid] = ry;
+        fold[2 * kEvalThreads + tid] = rz;
+        __syncthreads();
+        if (tid < U.nt)
+            for (int id = tid + U.nt; id < nid; id += U.nt) {
+                rx += fold[id];
+                ry += fold[kEvalThreads + id];
+                rz += fold[2 * kEvalThreads + id];
+            }
+    }
+    if (tid < U.nt) {
         if (U.proxy) {
-            a.proxy_part[(size_t)U.out * a.P + ti] = make_double4(rx, ry, rz, 0.0);
+            a.proxy_part[(size_t)U.out * a.P + tid] = make_double4(rx, ry, rz, 0.0);
         } else if (U.out >= 0) {
-            a.leaf_part[(size_t)U.out + ti] = make_double2(rx, ry);
+            a.leaf_part[(size_t)U.out + tid] = make_double2(rx, ry);
         } else {
-            const int idx = a.perm[U.tgt + ti];
+            const int idx = a.perm[U.tgt + tid];
             a.out_x[idx] = rx;
             a.out_y[idx] = ry;
         }
     }
 }
-static_assert(sizeof(double) * 3 * kEvalThreads <= sizeof(double4) * kRing * kMaxStage, "the reduction fits the ring");
+static_assert(sizeof(double) * 3 * (kSlots + 1) * kEvalThreads <= sizeof(double4) * kRing * kMaxStage,
+              "the warps' sums and the folded lanes' fit the ring");
+static_assert(kEvalMaxChunks <= kEvalWarps && kSlots == 2, "a warp's run is a chunk at most: it meets two");
+static_assert(32 * kEvalMaxChunks <= kEvalThreads, "a thread per lane of the folded set");
+static_assert(kEvalThreads >= kMaxStage, "a thread per target at the end (leaves and proxy sets hold at most 256)");
 
 void launch_eval(int form, const EvalArgs &a, int nunits, cudaStream_t st) {
     if (nunits <= 0) return;
@@ -331,38 +413,46 @@ void launch_eval(int form, const EvalArgs &a, int nunits, cudaStream_t st) {
 // interpolation of its target slots' proxy potentials (interp_vals_bli and
 // the loops of fast_sum_module.f90:186-199).  FORM 0 interpolates east/north
 // components, FORM 1 the Cartesian vector, projected on the target's frame.
-// Thread tid has target tid % nt and the eta rows tid / nt, + nsplit, ... of
-// every slot, whose record (potentials, nodes) the CTA copies to shared
-// memory.
-constexpr int kFinThreads = 256;
+// The records (potentials, nodes) of up to kFinSlots slots come to shared
+// memory at a time; thread tid has target tid % nt and every (256 / nt)-th
+// (slot, eta row) of them, so that small leaves' slots run side by side.
+constexpr int kFinThreads = 256, kFinSlots = 4;
 template <int N, int FORM>
 __global__ void __launch_bounds__(kFinThreads) leaf_fin_kernel(FinArgs a) {
-    constexpr int P = N * N;
-    __shared__ double4 rec[P + (2 * N + 3) / 4];
+    constexpr int P = N * N, R = P + (2 * N + 3) / 4;   // double4 per record
+    __shared__ double4 rec[kFinSlots][R];
     __shared__ double red[3][kFinThreads];
     const LeafFin L = a.fin[blockIdx.x];
     const int tid = threadIdx.x, nt = L.nt, nsplit = kFinThreads / nt, ti = tid % nt, sp = tid / nt;
     const bool active = sp < nsplit;
     const double2 xe = active ? a.xieta[L.tgt + ti] : make_double2(0.0, 0.0);
     double ux = 0.0, uy = 0.0, uz = 0.0;
-    for (int e = L.db; e < L.de; ++e) {
-        const double4 *src = reinterpret_cast<const double4 *>(a.records + (size_t)a.down_slots[e] * a.rec_stride);
+    for (int e0 = L.db; e0 < L.de; e0 += kFinSlots) {
+        const int ne = min(kFinSlots, L.de - e0);
         __syncthreads();
-        for (int i = tid; i < a.rec_stride / 4; i += kFinThreads) rec[i] = src[i];
+        for (int i = tid; i < ne * R; i += kFinThreads)
+            rec[i / R][i % R] = reinterpret_cast<const double4 *>(
+                a.records + (size_t)a.down_slots[e0 + i / R] * a.rec_stride)[i % R];
         __syncthreads();
-        if (active) {
-            const double *nodes = reinterpret_cast<const double *>(rec + P);
+        if (!active) continue;
+        int turn = sp;   // the next (slot, eta row) is this thread's when turn is 0
+        for (int e = 0; e < ne; ++e) {
+            if (turn >= N) {   // none of this slot's rows
+                turn -= N;
+                continue;
+            }
+            const double4 *rc = rec[e];
+            const double *nodes = reinterpret_cast<const double *>(rc + P);
             double fx[N], fe[N];
             bli_basis_n<N>(xe.x, nodes, fx);
             bli_basis_n<N>(xe.y, nodes + N, fe);
-            int turn = sp;   // eta row k is this thread's when turn is 0
 #pragma unroll
             for (int k = 0; k < N; ++k) {
                 if (turn == 0) {
                     double rx = 0.0, ry = 0.0, rz = 0.0;
 #pragma unroll
                     for (int j = 0; j < N; ++j) {
-                        const double4 ph = rec[j + k * N];
+                        const double4 ph = rc[j + k * N];
                         rx = fma(fx[j], ph.x, rx);
                         ry = fma(fx[j], ph.y, ry);
                         if (FORM == 1) rz = fma(fx[j], ph.z, rz);

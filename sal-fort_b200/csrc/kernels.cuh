@@ -93,12 +93,15 @@ struct Tgt {
     bool live;  // outside the pole guard
 };
 
+__device__ __forceinline__ double tgt_omx32(double z) { return __dsub_rn(1.0, __dmul_rn(z, z)); }
+__device__ __forceinline__ bool tgt_live(double z) {
+    return (fabs(__dsub_rn(z, 1.0)) > 1e-15) && (fabs(__dadd_rn(z, 1.0)) > 1e-15);
+}
 __device__ __forceinline__ void tgt_init(Tgt &t, double x, double y, double z) {
     t.x = x; t.y = y; t.z = z;
-    double x32 = __dmul_rn(z, z);
-    t.omx32 = __dsub_rn(1.0, x32);
+    t.omx32 = tgt_omx32(z);
     t.inv_mp2 = __ddiv_rn(1.0, __dsqrt_rn(t.omx32));
-    t.live = (fabs(__dsub_rn(z, 1.0)) > 1e-15) && (fabs(__dadd_rn(z, 1.0)) > 1e-15);
+    t.live = tgt_live(z);
 }
 
 // sal_grad_gfunc (fast_sum_module.f90:9-31) for a live target, operation for
@@ -122,51 +125,61 @@ __device__ __forceinline__ void gref_exact(const Tgt &t, double sx, double sy, d
     gx = __dmul_rn(__dmul_rn(nx, t.inv_mp2), val);
 }
 
-// Reciprocal and inverse square root for the treecode's inner loops: the
-// hardware's FP64 approximation (about 20 good bits, no conversion to FP32 and
-// back, which costs four conversions a pair on the SFU's pipe), refined by one
-// step of Householder's third-order iteration, whose error is the cube of the
-// seed's: for 1/x, r (1 + e + e^2) with e = 1 - x r; for 1/sqrt(x),
-// y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2.  Accurate to about one ulp for
-// normal x whose reciprocal (square root) is normal; 0, infinities and NaN do
-// not give IEEE results, and callers keep them away.
-__device__ __forceinline__ double fast_rcp(double x) {
+// Reciprocal and square root for the treecode's inner loops: the hardware's
+// FP64 approximation (about 20 good bits, no conversion to FP32 and back, which
+// costs four conversions a pair on the SFU's pipe), refined by one step of
+// Householder's third-order iteration, whose error is the cube of the seed's:
+// for 1/x, r (1 + e + e^2) with e = 1 - x r; for sqrt(x) = x y with
+// y ~ 1/sqrt(x), g (1 + e/2 + 3 e^2/8) with g = x y and e = 1 - g y.  Accurate
+// to about one ulp for normal x whose reciprocal (inverse square root) is
+// normal; 0, infinities and NaN do not give IEEE results, and callers keep
+// them away.
+__device__ __forceinline__ double rcp_seed(double x) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    const double e = fma(-x, r, 1.0);
+    return r;
+}
+__device__ __forceinline__ double fast_rcp(double x) {
+    const double r = rcp_seed(x), e = fma(-x, r, 1.0);
     return fma(r, fma(e, e, e), r);
 }
-__device__ __forceinline__ double fast_rsqrt(double x) {
+__device__ __forceinline__ double fast_sqrt(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
-    return fma(fma(e, 0.375, 0.5), y * e, y);
+    const double g = x * y, e = fma(-g, y, 1.0);
+    return fma(g * e, fma(e, 0.375, 0.5), g);
 }
 
-// The kernel's scalar val / kCons as a function of mp = 2 - 2g alone.  With
+// The kernel's scalar val w / kCons as a function of mp = 2 - 2g alone.  With
 // q = sqrt(mp): 2g + q = (2 - q)(1 + q) and 2(g^2 - 1) = -mp (2 - q)(2 + q)/2,
-// so p1 + p2 = [kC1 - 2 kC2 q (1 + q)/(2 + q)] / q^3 and
-// q (1 + q)/(2 + q) = q - 1 + 2/(2 + q): one inverse square root and one
-// reciprocal, and no cancellation.  kReg: p1's + 1e-16 to first order
-// (1/(q^3 + c) = 1/q^3 - c/q^6); p2's is below 2e-13 of the value for
-// q > 1e-3.  22 FP64 instructions against 31 of the two denominators' form.
+// so p1 + p2 = N / D with
+//   N = kC1 (2 + q) - 2 kC2 (q + mp),  D = q^3 (2 + q) = mp (2 q + mp):
+// one square root, one reciprocal, no cancellation.  kReg: p1's + 1e-16,
+// folded into D: c (2 + b q) there takes c kC1/q^6 off N / D up to 4 c/q of it
+// (c = 1e-16, b = 1 + 2 kC2/kC1); p2's is below 2e-13 of the value for
+// q > 1e-3.  15 FP64 instructions (16 with kReg) against 31 of the two
+// denominators' form with its FP32 seeds.
 template <bool kReg>
-__device__ __forceinline__ double val_chord(double mp) {
-    const double y = fast_rsqrt(mp);
-    const double q = mp * y;
-    const double r = fast_rcp(q + 2.0);
-    double f = fma(-2.0 * kC2, q, kC1 + 2.0 * kC2);
-    f = fma(-4.0 * kC2, r, f);
-    const double y3 = y * y * y;
-    if (kReg) f = fma(-1e-16 * kC1, y3, f);
-    return f * y3;
+__device__ __forceinline__ double val_chord(double mp, double w) {
+    const double q = fast_sqrt(mp);
+    const double n = fma(-2.0 * kC2, mp, fma(kC1 - 2.0 * kC2, q, 2.0 * kC1));
+    const double t = fma(2.0, q, mp);
+    const double d = kReg ? fma(mp, t, fma(1e-16 * (1.0 + 2.0 * kC2 / kC1), q, 2e-16)) : mp * t;
+    const double r = rcp_seed(d), e = fma(-d, r, 1.0);
+    const double u = n * w * r;
+    return fma(u, fma(e, e, e), u);
 }
 
 // Where val_chord<true> stands for the reference's expressions: q >= 1e-3
 // (the second-order term of the + 1e-16 is below 1e-14 of the value) and off
 // the antipode, where the reference's (2g + q) and (g^2 - 1) cancel to
 // rounding noise that has to be reproduced.  False for NaN.
-__device__ __forceinline__ bool chord_plain(double mp) { return mp >= 1e-6 && mp <= 3.99; }
+// On the value's upper word, a positive double's order: the ALU's work, not
+// two comparisons on the FP64 pipe.
+__device__ __forceinline__ bool chord_plain(double mp) {
+    constexpr unsigned kLo = 0x3EB0C6F7u + 1u, kHi = 0x400FEB85u;   // above 1e-6's, 3.99's
+    return (unsigned)__double2hiint(mp) - kLo < kHi - kLo;
+}
 
 // sal_grad_gfunc's val / kCons in the reference's operation order: g clamped,
 // mp = 2 - 2g, the two denominators and the two numerators (these carry the
@@ -206,7 +219,7 @@ __device__ __forceinline__ void gref_near(const Tgt &t, const double4 *s, int st
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const double4 q = s[k * stride];
-            const double val = val_chord<true>(mp[k]) * q.w;
+            const double val = val_chord<true>(mp[k], q.w);
             ax = fma(fma(-t.y, q.x, t.x * q.y), val, ax);
             ay = fma(fma(-t.z, gxy[k], q.z * t.omx32), val, ay);
         }
@@ -216,7 +229,7 @@ __device__ __forceinline__ void gref_near(const Tgt &t, const double4 *s, int st
             const double4 q = s[k * stride];
             const double gk = __dadd_rn(__dadd_rn(__dmul_rn(t.x, q.x), __dmul_rn(t.y, q.y)), __dmul_rn(t.z, q.z));
             const double m = fma(-2.0, gk, 2.0);
-            const double val = (chord_plain(m) ? val_chord<true>(m) : val_ref(gk)) * q.w;
+            const double val = chord_plain(m) ? val_chord<true>(m, q.w) : val_ref(gk) * q.w;
             const double nx = __dsub_rn(__dmul_rn(t.x, q.y), __dmul_rn(t.y, q.x));
             const double ny = __dsub_rn(__dmul_rn(q.z, t.omx32),
                                         __dmul_rn(t.z, __dadd_rn(__dmul_rn(t.x, q.x), __dmul_rn(t.y, q.y))));
@@ -231,25 +244,66 @@ __device__ __forceinline__ void gref_near(const Tgt &t, const double4 *s, int st
 // target (nx = tx Ay - ty Ax, ny = (1 - tz^2) Az - tz (tx Ax + ty Ay)).  The
 // vector cancels by the chord on projection, and no chord is below 0.012, so
 // its rounding stays below 1e-13 of a sum of thousands of pairs.  mt = -2 t.
-// 21 FP64 instructions against 29 of gref_near's plain branch.
-__device__ __forceinline__ void gref_far(const double (&mt)[3], const double4 &s, double (&A)[3]) {
-    const double mp = fma(mt[0], s.x, fma(mt[1], s.y, fma(mt[2], s.z, 2.0)));
-    const double v = val_chord<false>(mp) * s.w;
-    A[0] = fma(v, s.x, A[0]);
-    A[1] = fma(v, s.y, A[1]);
-    A[2] = fma(v, s.z, A[2]);
+// 20 FP64 instructions against 28 of gref_near's plain branch.
+// K sources s[0], s[stride], ...: independent chains side by side.
+template <int K>
+__device__ __forceinline__ void gref_far(const double (&mt)[3], const double4 *s, int stride, double (&A)[3]) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const double4 q = s[k * stride];
+        const double mp = fma(mt[0], q.x, fma(mt[1], q.y, fma(mt[2], q.z, 2.0)));
+        const double v = val_chord<false>(mp, q.w);
+        A[0] = fma(v, q.x, A[0]);
+        A[1] = fma(v, q.y, A[1]);
+        A[2] = fma(v, q.z, A[2]);
+    }
 }
 
-// val / kCons with its removable antipodal singularity cancelled analytically
-// (val_chord's form) for mp = q^2 from coordinate differences, not from
-// 2 - 2 t.s.  Pairs closer than 1e-3 keep the two + 1e-16 of the denominators
-// (a source on the target gives a finite value, times a zero displacement).
-__device__ __forceinline__ double vstable(double mp) {
-    if (mp >= 1e-6) return val_chord<true>(mp);
-    const double q = __dsqrt_rn(mp);
-    const double d1 = q * mp + 1e-16;
-    const double d2 = mp * (2.0 + q) + 1e-16;
-    return __ddiv_rn(kC1 * d2 - 2.0 * kC2 * (1.0 + q) * d1, d1 * d2);
+// K pairs of a Cartesian proxy target (x, y, z) with sources s[0], s[stride],
+// ...: adds val w (s - x) / kCons, with val's removable antipodal singularity
+// cancelled analytically (val_chord's form) and mp = |s - x|^2 from coordinate
+// differences, not from 2 - 2 t.s.  Independent chains side by side; with a
+// pair closer than 1e-3 among them, which keeps the two + 1e-16 of the
+// denominators (a source on the target gives a finite value, times a zero
+// displacement), one after another.
+template <int K>
+__device__ __forceinline__ void cart_pairs(double x, double y, double z, const double4 *s, int stride,
+                                           double (&A)[3]) {
+    double mp[K];
+    bool plain = true;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const double4 q = s[k * stride];
+        const double dx = q.x - x, dy = q.y - y, dz = q.z - z;
+        mp[k] = fma(dx, dx, fma(dy, dy, dz * dz));
+        plain = plain && mp[k] >= 1e-6;
+    }
+    if (plain) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const double4 q = s[k * stride];
+            const double v = val_chord<true>(mp[k], q.w);
+            A[0] = fma(v, q.x - x, A[0]);
+            A[1] = fma(v, q.y - y, A[1]);
+            A[2] = fma(v, q.z - z, A[2]);
+        }
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < K; ++k) {
+            const double4 q = s[k * stride];
+            const double dx = q.x - x, dy = q.y - y, dz = q.z - z, m = fma(dx, dx, fma(dy, dy, dz * dz));
+            double v;
+            if (m >= 1e-6) {
+                v = val_chord<true>(m, q.w);
+            } else {
+                const double c = __dsqrt_rn(m), d1 = c * m + 1e-16, d2 = m * (2.0 + c) + 1e-16;
+                v = __ddiv_rn(kC1 * d2 - 2.0 * kC2 * (1.0 + c) * d1, d1 * d2) * q.w;
+            }
+            A[0] = fma(v, dx, A[0]);
+            A[1] = fma(v, dy, A[1]);
+            A[2] = fma(v, dz, A[2]);
+        }
+    }
 }
 
 // bli_coeffs, bli_module.f90:6-26 (0-based index i0 of degree d).

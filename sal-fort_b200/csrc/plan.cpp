@@ -150,11 +150,30 @@ struct EvalBounds {
 };
 
 // Work of the FP64 evaluation pass: about kEvalUnits units of equal cost when
-// the grid is small (4 for each of 3 CTAs on 148 SMs, so the last wave is
-// short), but none below kEvalMinPairs pairs (a CTA's set-up costs about as
-// much as 4,000 pairs).
-static constexpr double kEvalUnits = 4.0 * 3 * 148, kEvalMinPairs = 16384.0;
+// the grid is small (8 for each of 2 CTAs on 148 SMs, so the last wave is
+// short; 4 cost 3 % at 163,842 cells), but none below kEvalMinPairs pairs (a
+// CTA's set-up and end cost about as much as 10,000; half of it costs 4 % at
+// 3,000 cells).
+static constexpr double kEvalUnits = 8.0 * 2 * 148, kEvalMinPairs = 32768.0;
 static constexpr double kEvalNearCost = 1.35;   // a near pair's cost in far pairs
+
+// How often a set of nt targets is taken (EvalUnit::fold): the number that
+// leaves the fewest idle lanes in chunks of 32, up to one chunk a warp (81
+// proxies: 3 x 81 lanes fill 8 chunks to 95 %, 84 % unfolded).  More chunks
+// than warps were no faster at 2.3M cells (148 targets in 19 chunks: 19.9 ms
+// for the leaf units, as unfolded): what the lanes gain, the state that a warp
+// swaps per chunk and stage takes back.
+static int32_t eval_fold(int32_t nt) {
+    int32_t best = 1;
+    double least = 1e30;
+    for (int32_t f = 1; f <= 8; ++f) {
+        const int32_t nid = nt * f, nch = (nid + 31) / 32, nlast = nid - 32 * (nch - 1);
+        if (nch > kEvalMaxChunks && f > 1) break;
+        const double c = (nch - 1 + 1.0 / (32 / nlast)) * 32.0 / nid;   // the last chunk takes 32 / nlast residues at once
+        if (c < least - 1e-12) { least = c; best = f; }
+    }
+    return best;
+}
 
 static void plan_build_eval(const Tree &t, const EvalBounds &bd, const std::vector<std::vector<EvalSrc>> &lsrc,
                             const std::vector<std::vector<EvalSrc>> &tsrc,
@@ -254,6 +273,7 @@ static void plan_build_eval(const Tree &t, const EvalBounds &bd, const std::vect
         u.tgt = proxy ? (int32_t)(x - nl) : (int32_t)t.p[leaves[x]].begin;
         u.nt = S.nt;
         u.proxy = proxy;
+        u.fold = eval_fold(S.nt);
         LeafFin f{};
         if (proxy) {
             pl->eval_proxy_unit_beg[x - nl] = (int32_t)pu.size();
