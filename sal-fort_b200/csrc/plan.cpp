@@ -389,12 +389,14 @@ bool plan_build(const Tree &t, const double *xs, const double *ys, const double 
     pl->src_proxy_xyz.resize((size_t)nsrc * P * 3);
     pl->src_nodes.resize((size_t)nsrc * 2 * nd);
     pl->src_box.resize((size_t)nsrc * 4);
+#pragma omp parallel for schedule(static)
     for (int32_t s = 0; s < nsrc; ++s)
         panel_proxies(t.p[pl->src_slot_panel[s]], d, &pl->src_proxy_xyz[(size_t)s * P * 3], &pl->src_nodes[(size_t)s * 2 * nd],
                       &pl->src_box[(size_t)s * 4]);
     pl->tgt_proxy_xyz.resize((size_t)ntgt * P * 3);
     pl->tgt_nodes.resize((size_t)ntgt * 2 * nd);
     pl->tgt_box.resize((size_t)ntgt * 4);
+#pragma omp parallel for schedule(static)
     for (int32_t s = 0; s < ntgt; ++s)
         panel_proxies(t.p[pl->tgt_slot_panel[s]], d, &pl->tgt_proxy_xyz[(size_t)s * P * 3], &pl->tgt_nodes[(size_t)s * 2 * nd],
                       &pl->tgt_box[(size_t)s * 4]);
@@ -424,20 +426,26 @@ bool plan_build(const Tree &t, const double *xs, const double *ys, const double 
             if (ty == 0 || ty == 1) {
                 int32_t lb, le;
                 leaf_range(k_t, &lb, &le);
-                for (int32_t l = lb; l < le; ++l) {
-                    if (ty == 0) push_range(litems[l], S.begin, S.count(), 0, -1);
-                    else push_range(litems[l], proxy_off(k_s), P, 1, -1);
-                    lsrc[l].push_back(EvalSrc{k_s, ty, -1});
-                    lcost[l] += (double)(ty == 0 ? S.count() : P) * t.p[leaves[l]].count();
-                }
+                for (int32_t l = lb; l < le; ++l) lsrc[l].push_back(EvalSrc{k_s, ty, -1});
                 pl->pairs[ty] += (double)T.count() * (ty == 0 ? S.count() : P);
             } else {
-                int32_t ts = tgt_slot[k_t];
-                if (ty == 2) push_range(titems[ts], S.begin, S.count(), 0, -1);
-                else push_range(titems[ts], proxy_off(k_s), P, 1, -1);
-                tsrc[ts].push_back(EvalSrc{k_s, ty - 2, -1});
-                tcost[ts] += (double)P * (ty == 2 ? S.count() : P);
+                tsrc[tgt_slot[k_t]].push_back(EvalSrc{k_s, ty - 2, -1});
                 pl->pairs[ty] += (double)P * (ty == 2 ? S.count() : P);
+            }
+        }
+        // the same as work-list items, each set in list order
+        const int64_t nl = (int64_t)leaves.size();
+#pragma omp parallel for schedule(dynamic, 16)
+        for (int64_t x = 0; x < nl + ntgt; ++x) {
+            const bool proxy = x >= nl;
+            std::vector<Item> &v = proxy ? titems[x - nl] : litems[x];
+            double &c = proxy ? tcost[x - nl] : lcost[x];
+            const double nt = proxy ? (double)P : (double)t.p[leaves[x]].count();
+            for (const EvalSrc &e : proxy ? tsrc[x - nl] : lsrc[x]) {
+                const Panel &S = t.p[e.panel];
+                if (e.kind == 0) push_range(v, S.begin, S.count(), 0, -1);
+                else push_range(v, proxy_off(e.panel), P, 1, -1);
+                c += (e.kind == 0 ? (double)S.count() : (double)P) * nt;
             }
         }
         // DOWN items: every leaf under a target slot interpolates its potentials
