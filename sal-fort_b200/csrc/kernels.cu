@@ -532,15 +532,21 @@ void launch_proxy_finalize(const int32_t *unit_beg, const double4 *partial, int 
 }
 
 // ------------------------------------------------------------------ direct sum
-// FP64 direct O(N^2) sum at sampled targets with the reference kernel, sources
-// split into chunks (blockIdx.y) whose partial sums are added in chunk order.
-constexpr int kDirectTile = 128;
-__global__ void __launch_bounds__(kDirectTile) direct_kernel(const double *__restrict__ xs, const double *__restrict__ ys,
-                                                             const double *__restrict__ zs, const double *__restrict__ w,
-                                                             int n, const int32_t *__restrict__ targets, int nt,
-                                                             int chunk, double *__restrict__ partial) {
-    __shared__ double4 S[kDirectTile];
-    const int k = blockIdx.x * kDirectTile + threadIdx.x;
+// FP64 direct O(N^2) sum at sampled targets with the reference kernel: one
+// target per thread, sources staged through shared memory, gref_near 4 pairs
+// at a time (g in the reference's operation order, val_ref for the self pair
+// and the other pairs whose value is rounding noise).  Bound by the FP64 pipe:
+// 27 instructions a pair (10,000 targets x 655,362 sources: 12.5 ms, 72 cycles
+// a pair and scheduler of the 68 that a loop of nothing else takes), where
+// IEEE division and square root took about 110 (31.4 ms).  The sources are split into
+// chunks (blockIdx.y) whose partial sums are added in a fixed order.
+constexpr int kDirectThreads = 128, kDirectTile = 256, kDirectCtas = 5, kDirectIlp = 4;
+__global__ void __launch_bounds__(kDirectThreads, kDirectCtas)
+    direct_kernel(const double *__restrict__ xs, const double *__restrict__ ys, const double *__restrict__ zs,
+                  const double *__restrict__ w, int n, const int32_t *__restrict__ targets, int nt, int chunk,
+                  double *__restrict__ partial) {
+    __shared__ __align__(16) double4 S2[2][kDirectTile];
+    const int k = blockIdx.x * kDirectThreads + threadIdx.x;
     const int s0 = blockIdx.y * chunk, s1 = min(n, s0 + chunk);
     Tgt T;
     if (k < nt) {
@@ -551,51 +557,78 @@ __global__ void __launch_bounds__(kDirectTile) direct_kernel(const double *__res
         T.live = false;
     }
     double ax = 0.0, ay = 0.0;
-    for (int b = s0; b < s1; b += kDirectTile) {
-        const int m = min(kDirectTile, s1 - b);
-        if (threadIdx.x < m) {
-            const int s = b + threadIdx.x;
-            S[threadIdx.x] = make_double4(xs[s], ys[s], zs[s], w[s]);
+    // the next tile is copied (8 bytes at a time: the four arrays have no other
+    // common alignment) while this one is summed
+    auto fetch = [&](int b, int buf) {
+        for (int i = threadIdx.x; i < min(kDirectTile, s1 - b); i += kDirectThreads) {
+            double *o = reinterpret_cast<double *>(&S2[buf][i]);
+            cp_async8(o, xs + b + i);
+            cp_async8(o + 1, ys + b + i);
+            cp_async8(o + 2, zs + b + i);
+            cp_async8(o + 3, w + b + i);
         }
-        __syncthreads();
-        if (T.live)
-            for (int s = 0; s < m; ++s) {
-                double gx, gy;
-                gref_exact(T, S[s].x, S[s].y, S[s].z, gx, gy);
-                ax += gx * S[s].w;
-                ay += gy * S[s].w;
-            }
-        __syncthreads();
+        cp_async_commit();
+    };
+    fetch(s0, 0);
+    int buf = 0;
+    for (int b = s0; b < s1; b += kDirectTile, buf ^= 1) {
+        cp_async_wait_all();
+        __syncthreads();   // this tile is here, and every warp is through with the other buffer
+        if (b + kDirectTile < s1) fetch(b + kDirectTile, buf ^ 1);
+        if (T.live) {
+            const double4 *S = S2[buf];
+            const int m = min(kDirectTile, s1 - b);
+            int s = 0;
+            for (; s + kDirectIlp <= m; s += kDirectIlp) gref_near<kDirectIlp>(T, S + s, 1, ax, ay);
+            for (; s < m; ++s) gref_near<1>(T, S + s, 1, ax, ay);
+        }
     }
+    cp_async_wait_all();
     if (k < nt) {
-        partial[((size_t)blockIdx.y * nt + k) * 2] = ax;
-        partial[((size_t)blockIdx.y * nt + k) * 2 + 1] = ay;
+        const double tf = T.live ? kCons * T.inv_mp2 : 0.0;
+        partial[((size_t)blockIdx.y * nt + k) * 2] = ax * tf;
+        partial[((size_t)blockIdx.y * nt + k) * 2 + 1] = ay * tf;
     }
 }
 
-__global__ void direct_reduce_kernel(const double *__restrict__ partial, int nt, int nchunks, double *__restrict__ ox,
+// One warp per target: lane l adds chunks l, l + 32, ..., then the lanes' sums.
+__global__ void direct_reduce_kernel(const double2 *__restrict__ partial, int nt, int nchunks, double *__restrict__ ox,
                                      double *__restrict__ oy) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (k >= nt) return;
     double x = 0.0, y = 0.0;
-    for (int c = 0; c < nchunks; ++c) {
-        x += partial[((size_t)c * nt + k) * 2];
-        y += partial[((size_t)c * nt + k) * 2 + 1];
+    for (int c = lane; c < nchunks; c += 32) {
+        const double2 v = partial[(size_t)c * nt + k];
+        x += v.x;
+        y += v.y;
     }
-    ox[k] = x;
-    oy[k] = y;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        x += __shfl_xor_sync(0xffffffffu, x, o);
+        y += __shfl_xor_sync(0xffffffffu, y, o);
+    }
+    if (lane == 0) {
+        ox[k] = x;
+        oy[k] = y;
+    }
 }
 
-int direct_chunks(int n) { return max(1, min(64, (n + 32767) / 32768)); }
+// Source chunks of a direct sum: up to 8 waves of CTAs, the last one nearly
+// full, and chunks of 1,024 sources at least.
+int direct_chunks(int n, int nt) {
+    const int tb = max(1, (nt + kDirectThreads - 1) / kDirectThreads);
+    return max(1, min(8 * 148 * kDirectCtas / tb, n / 1024));
+}
 
 void launch_direct(const double *xs, const double *ys, const double *zs, const double *w, int n,
                    const int32_t *targets, int nt, double *out_x, double *out_y, double *scratch, int nchunks,
                    cudaStream_t st) {
     if (nt <= 0) return;
     const int chunk = (n + nchunks - 1) / nchunks;
-    dim3 grid((nt + kDirectTile - 1) / kDirectTile, nchunks);
-    direct_kernel<<<grid, kDirectTile, 0, st>>>(xs, ys, zs, w, n, targets, nt, chunk, scratch);
-    direct_reduce_kernel<<<(nt + 255) / 256, 256, 0, st>>>(scratch, nt, nchunks, out_x, out_y);
+    dim3 grid((nt + kDirectThreads - 1) / kDirectThreads, nchunks);
+    direct_kernel<<<grid, kDirectThreads, 0, st>>>(xs, ys, zs, w, n, targets, nt, chunk, scratch);
+    direct_reduce_kernel<<<(nt + 7) / 8, 256, 0, st>>>(reinterpret_cast<const double2 *>(scratch), nt, nchunks, out_x,
+                                                       out_y);
 }
 
 // ------------------------------------------------------------------ proxy weight transfer

@@ -36,6 +36,11 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // Bulk (non-tensor) TMA copy global -> this CTA's shared memory, completing
 // on an mbarrier.  No multicast.  Both addresses 16-byte aligned, bytes a
 // multiple of 16.
@@ -107,8 +112,8 @@ __device__ __forceinline__ void tgt_init(Tgt &t, double x, double y, double z) {
 // sal_grad_gfunc (fast_sum_module.f90:9-31) for a live target, operation for
 // operation with IEEE division and square root and without contraction, so the
 // singular self pair s == t rounds exactly as the reference's does.  The
-// division by sqrt(1-tz^2) is a multiply by its hoisted reciprocal.  Used by
-// the direct sum, the accuracy judge.
+// division by sqrt(1-tz^2) is a multiply by its hoisted reciprocal.  Used for
+// the batched form's self pairs.
 __device__ __forceinline__ void gref_exact(const Tgt &t, double sx, double sy, double sz, double &gx, double &gy) {
     double gxy = __dadd_rn(__dmul_rn(t.x, sx), __dmul_rn(t.y, sy));
     double g = __dadd_rn(gxy, __dmul_rn(t.z, sz));
@@ -171,13 +176,16 @@ __device__ __forceinline__ double val_chord(double mp, double w) {
 }
 
 // Where val_chord<true> stands for the reference's expressions: q >= 1e-3
-// (the second-order term of the + 1e-16 is below 1e-14 of the value) and off
-// the antipode, where the reference's (2g + q) and (g^2 - 1) cancel to
-// rounding noise that has to be reproduced.  False for NaN.
-// On the value's upper word, a positive double's order: the ALU's work, not
-// two comparisons on the FP64 pipe.
+// (the + 1e-16 terms it leaves out are below 4e-13 of the value), and
+// 2e-6 off mp = 4: at the antipode the reference's (2g + q) and (g^2 - 1)
+// cancel to rounding noise (4e-10 of p2 at this line, in pairs whose value is
+// among the smallest; the line is as close as the test below can draw it,
+// because with a band of 0.01 a warp of scattered targets meets it with one
+// source in twelve: 17.7 ms for 10,000 targets x 655,362 sources).  False for
+// NaN.  On the value's upper word, a positive double's order: the ALU's work,
+// not two comparisons on the FP64 pipe.
 __device__ __forceinline__ bool chord_plain(double mp) {
-    constexpr unsigned kLo = 0x3EB0C6F7u + 1u, kHi = 0x400FEB85u;   // above 1e-6's, 3.99's
+    constexpr unsigned kLo = 0x3EB0C6F7u + 1u, kHi = 0x400FFFFFu;   // above 1e-6's, the last below 4's
     return (unsigned)__double2hiint(mp) - kLo < kHi - kLo;
 }
 
@@ -404,7 +412,7 @@ void launch_proxy_finalize(const int32_t *unit_beg, const double4 *partial, int 
 void launch_direct(const double *xs, const double *ys, const double *zs, const double *w, int n,
                    const int32_t *targets, int nt, double *out_x, double *out_y, double *scratch, int nchunks,
                    cudaStream_t st);
-int direct_chunks(int n);
+int direct_chunks(int n, int nt);
 void launch_extract_w(const double4 *pool_proxy, int count, double *out, cudaStream_t st);
 void launch_insert_w(const double *w, int count, double4 *pool_proxy, cudaStream_t st);
 

@@ -70,7 +70,7 @@ extern "C" int sal_direct_sum_noalloc(const double *xs, const double *ys, const 
     // as many source chunks as the scratch holds for nt targets, at most the
     // count the allocating entry point uses
     const int cap = (int)((int64_t)SAL_NOALLOC_SCRATCH_DOUBLES / (2 * (int64_t)nt));
-    int nch = sal::dev::direct_chunks(n);
+    int nch = sal::dev::direct_chunks(n, nt);
     if (nch > cap) nch = cap;
     sal::dev::launch_direct(xs, ys, zs, w, n, targets, nt, out_x, out_y, scratch, nch, (cudaStream_t)stream);
     e = cudaGetLastError();

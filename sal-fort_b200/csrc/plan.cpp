@@ -135,7 +135,7 @@ struct EvalBounds {
         return std::sqrt(a * a + b * b + c * c);
     }
     // 2 - 2 x.y = |x - y|^2 + (1 - |x|^2) + (1 - |y|^2): whether it can leave
-    // [1.5e-4, 3.96] for a target of panel kt (its points, or with `proxy` its
+    // [1.5e-4, 3.999] for a target of panel kt (its points, or with `proxy` its
     // proxies) and a source s.  Inside, the reference's operation order is not
     // needed: a fused dot product's 2 - 2g is within 2e-16 / 1.5e-4 = 1.5e-12
     // of the reference's at the nearest such pair (chord 0.012; with more than
@@ -145,7 +145,7 @@ struct EvalBounds {
         const double rt = proxy ? rbox[kt] : rpts[kt], rs = s.kind ? rbox[s.panel] : rpts[s.panel];
         const double d = dist(kt, t.cx[s.panel], t.cy[s.panel], t.cz[s.panel]);
         const double lo = d - rt - rs, hi = d + rt + rs;
-        return !(lo > 0.0 && lo * lo - 2.0 * eta >= 1.5e-4 && hi * hi + 2.0 * eta <= 3.96);
+        return !(lo > 0.0 && lo * lo - 2.0 * eta >= 1.5e-4 && hi * hi + 2.0 * eta <= 3.999);
     }
 };
 

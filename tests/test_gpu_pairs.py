@@ -1,4 +1,4 @@
-"""GPU test of the FP64 pair kernel over the chords where its evaluation
+"""GPU tests of the FP64 pair kernel over the chords where its evaluation
 changes: self pairs, near duplicates, the switch from the reference's operation
 order to the chord form (chord 1e-3), close and distant neighbours, and
 (near-)antipodes, where the reference's value is rounding noise.
@@ -44,3 +44,31 @@ def test_pair_kernel_over_chords_matches_oracle(chord, antipodal):
     gx, gy = np.zeros(80), np.zeros(80)
     S.fast_sum(gx, gy, L, t, xs, ys, zs, area, h, 80, 8)
     assert rel_l2(gx, gy, ox, oy) <= 1e-12
+
+
+@pytest.mark.parametrize("n,nt", [(1, 1), (4, 3), (255, 127), (256, 128), (257, 129), (1023, 33), (2048, 200),
+                                  (2049, 2049), (9001, 1), (40000, 300)])
+def test_direct_sum_at_tile_and_chunk_edges_matches_oracle(n, nt):
+    """sal_direct_sum and its allocation-free form at the edges of the target
+    blocks (128), source tiles (256) and source chunks (1,024 and more), on
+    random points, whose close pairs reach chords of about 1e-2 / sqrt(n): the
+    same 1e-12 bar as the pair kernel's."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import salgpu as S
+    from oracle import oracle as O
+    rng = np.random.default_rng(n + nt)
+    p = rng.standard_normal((n, 3))
+    p /= np.linalg.norm(p, axis=1, keepdims=True)
+    xs, ys, zs = (np.ascontiguousarray(p[:, k]) for k in range(3))
+    area, h = rng.uniform(0.9, 1.1, n), rng.standard_normal(n)
+    tg = np.sort(rng.choice(n, nt, replace=False)).astype(np.int32)
+    rx, ry = O.direct_sum(xs, ys, zs, area, h, tg)
+    dev = [torch.tensor(v, device="cuda") for v in (xs, ys, zs, area * h, tg)]
+    ox, oy = S.direct_sum(*dev)
+    nx, ny = torch.full_like(ox, float("nan")), torch.full_like(ox, float("nan"))
+    S.direct_sum_noalloc(*dev, nx, ny)
+    torch.cuda.synchronize()
+    for x, y in ((ox, oy), (nx, ny)):
+        assert rel_l2(x.cpu().numpy(), y.cpu().numpy(), rx, ry) <= 1e-12
