@@ -12,11 +12,16 @@
 // into stages of 32 K columns (four k-steps of 8).  The contraction is
 //     D[field part, target component] += W[field part, k] * T[k, target component]
 // with M = 128 weight rows (64 fields, TF32 hi and lo parts, ordered so that
-// field f's hi row 32(f/16) + f%16 and lo row +16 share a warp) and N = 256
-// kernel-tile columns (east of the 128 targets, then north).  One tcgen05.mma
-// costs the same whatever its N, so N = 256 keeps the tensor cores at full
-// width: per k-step two MMAs, W * T_hi and W * T_lo, give all four hi/lo
-// cross products.
+// field f's hi row 32(f/16) + f%16 and lo row +16 share a warp) and N = 2 half
+// kernel-tile columns (east of the group's targets, rounded up to half, a
+// multiple of 16, then north): per k-step two MMAs, W * T_hi and W * T_lo, give
+// all four hi/lo cross products.  An MMA of N = 256 takes 128 cycles, a small
+// group's in proportion, if one elected thread issues it with descriptors from
+// uniform registers; issued under `lane == 0` each cost 144 cycles and more
+// (207 in this kernel, whatever N: half of the MMA warp's time).  Elected
+// issue and narrow groups: leaf pass 34.9 -> 33.5 ms at 2.3M cells x 64
+// fields, where the producers' tile arithmetic is what the MMA warp then waits
+// for.
 // Warp roles:
 //   warps 0-7   producers.  A task is one k-step of a 32-target row block:
 //               8 kernel-tile entries per component and row in FP32, split
@@ -98,11 +103,11 @@ constexpr float kTwoC2F = (float)(2.0 * dev::kC2);
 
 static_assert(kTcChunk % kStageK == 0, "items are whole stages");
 
-// instruction descriptor: D F32, A/B TF32, both K-major, N = 256, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(256 >> 3) << 17) |
-                            ((uint32_t)(128 >> 4) << 24);
-// the same for kind::f16 with A/B FP16 (format 0), 16 sources per MMA
-constexpr uint32_t kIdescF16 = (1u << 4) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+// instruction descriptor: D F32, A/B TF32 (or FP16, format 0, 16 sources per
+// MMA), both K-major, M = 128; N (columns, a multiple of 16) by idesc_n
+constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(128 >> 4) << 24);
+constexpr uint32_t kIdescF16 = (1u << 4) | ((uint32_t)(128 >> 4) << 24);
+__device__ __forceinline__ uint32_t idesc_n(uint32_t idesc, int n) { return idesc | ((uint32_t)(n >> 3) << 17); }
 // FP16 leaf pass: a stage is 64 sources, eight units of 8 (a unit is one
 // TF32 k-step: the split store's granularity); a unit of the FP16 weight store
 // is 128 rows x 8 halves, 8-row groups 128 B apart (2 KB)
@@ -192,14 +197,15 @@ using dev::mbar_arrive;
 // the CTA-wide abort flag (later waits then give up after one poll).  A phase
 // that has already completed costs one poll and no read of the flag: every
 // shared-memory round trip is on the producers' critical path.
-__device__ __forceinline__ void wait_bounded(uint64_t *bar, uint32_t parity, volatile int *abort, int *err) {
-    if (dev::mbar_try_wait(bar, parity)) return;
+__device__ __forceinline__ bool wait_bounded(uint64_t *bar, uint32_t parity, volatile int *abort, int *err) {
+    if (dev::mbar_try_wait(bar, parity)) return true;
     for (uint32_t it = 0; it < kWaitPolls; ++it) {
-        if (*abort) return;
-        if (dev::mbar_try_wait(bar, parity)) return;
+        if (*abort) return false;
+        if (dev::mbar_try_wait(bar, parity)) return true;
     }
     *abort = 1;
     atomicExch(err, dev::kErrTimeout);
+    return false;
 }
 // Bounded wait that ignores the abort flag (drains copies and MMAs in flight
 // before the CTA exits).
@@ -224,20 +230,29 @@ __device__ __forceinline__ uint64_t smem_desc(const void *p) {
            (1ull << 46);
 }
 
+// One thread of the (converged) warp.  MMAs issued under it take their
+// descriptors from uniform registers; under `lane == 0` each issue cost 144
+// cycles (measured, whatever M and N), more than the MMA itself (N = 256: 128).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 // D[tmem] (+)= A[smem] * B[smem]
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t accumulate) {
+__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(kIdesc), "r"(accumulate)
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // D[tmem] (+)= A[smem] * B[smem], FP16 operands, 16 sources
-__device__ __forceinline__ void mma_ss_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t accumulate) {
+__device__ __forceinline__ void mma_ss_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
+                                           uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(kIdescF16), "r"(accumulate)
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // Descriptor of an FP16 weight tile of two store units (16 sources): K core
@@ -362,8 +377,7 @@ __device__ __forceinline__ void emit_chunk(const float (&x)[16], int c0, int f, 
 // writes them out after the accumulator has been handed back to the MMA
 // warp, so the next group's first chain overlaps the output writes.
 // MODE 0 (leaf): columns half c + t are component c (east, north) of target
-// t (half = 128, or the group's rows rounded up to 16 for the packed tiles of
-// a replayed kernel-tile store).  MODE 1 (proxy): columns 85c + r are
+// t (half = the group's rows rounded up to 16).  MODE 1 (proxy): columns 85c + r are
 // Cartesian component c of proxy r.  MODE 2 (upward): columns j < 128 are
 // proxies row0 + j.
 //
@@ -633,14 +647,16 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             const int row = 32 * wb + lane;
             const bool active = 32 * wb < G.nt, rvalid = row < G.nt;
             // canonical offsets (floats) of this thread's rows in a kernel tile:
-            // leaf east / north at rows t, 128 + t; proxy x / y / z at 85c + r
+            // leaf east / north at rows t, half + t (half: the targets rounded
+            // up to 16); proxy x / y / z at 85c + r
+            const int half = (G.nt + 15) & ~15;
             const int oe = canon(row, 0) >> 2;
-            const int on = canon(MODE == 0 ? kTcRows + row : kTcProxyRows + row, 0) >> 2;
+            const int on = canon(MODE == 0 ? half + row : kTcProxyRows + row, 0) >> 2;
             const int oz = canon(MODE == 0 ? 0 : 2 * kTcProxyRows + row, 0) >> 2;
-            const bool row_in_tile = MODE != 1 || row < kTcProxyRows;   // proxy components hold 85 rows
+            const bool row_in_tile = row < (MODE == 0 ? half : MODE == 1 ? kTcProxyRows : kTcRows);
             // FP16 tiles: byte offset of the row's first K core matrix (8-row
             // groups 256 B apart, the two K halves 128 B apart)
-            const int oe16 = (row >> 3) * 256 + (row & 7) * 16, on16 = oe16 + (kTcRows / 8) * 256;
+            const int oe16 = (row >> 3) * 256 + (row & 7) * 16, on16 = oe16 + half * 32;
             // the row's target relative to the leaf centre and its east /
             // north unit vectors (zero at the poles, as the reference's guard)
             float tl0 = 0.f, tl1 = 0.f, tl2 = 0.f, el0 = 0.f, el1 = 0.f, ep0 = 0.f, ep1 = 0.f, ep2 = 0.f;
@@ -684,8 +700,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             // record: the group's tiles in the store, stage after stage; per
             // MMA step four chunks (hi, lo x east, north) of the group's rows
             // rounded up to 16, each the bytes of the ring's rows
-            const int nr16 = (G.nt + 15) & ~15;
-            const size_t cb = (size_t)nr16 * 32;
+            const size_t cb = (size_t)half * 32;
             unsigned char *gtile = (TS == 1 || TS == 3) ? a.ktile + a.ktile_off[gi - J.beg[gk]] : nullptr;
             // item records are read one item ahead, so their latency hides
             // behind the current item's stages
@@ -709,7 +724,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                         __syncwarp();
                         if (lane < nq && !*abort)
                             dev::bulk_g2s_hint(reinterpret_cast<unsigned char *>(sm.Kt(slot, lane >> 2, (lane >> 1) & 1)) +
-                                                   (lane & 1) * (kTcRows / 8) * 256,
+                                                   (lane & 1) * cb,
                                                gtile + (size_t)lane * cb, (uint32_t)cb, &sm.kfull[slot], dev::l2_evict_first());
                     } else if (lane == 0) {
                         mbar_arrive(&sm.kfull[slot]);
@@ -849,11 +864,13 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                                 split_f16x2(vn[2], vn[3], nh.y, nl.y);
                                 split_f16x2(vn[4], vn[5], nh.z, nl.z);
                                 split_f16x2(vn[6], vn[7], nh.w, nl.w);
-                                *reinterpret_cast<uint4 *>(th + oe16 + hb) = eh;
-                                *reinterpret_cast<uint4 *>(tlo + oe16 + hb) = el;
-                                *reinterpret_cast<uint4 *>(th + on16 + hb) = nh;
-                                *reinterpret_cast<uint4 *>(tlo + on16 + hb) = nl;
-                                if (TS == 1 && stored && row < nr16) {
+                                if (row_in_tile) {
+                                    *reinterpret_cast<uint4 *>(th + oe16 + hb) = eh;
+                                    *reinterpret_cast<uint4 *>(tlo + oe16 + hb) = el;
+                                    *reinterpret_cast<uint4 *>(th + on16 + hb) = nh;
+                                    *reinterpret_cast<uint4 *>(tlo + on16 + hb) = nl;
+                                }
+                                if (TS == 1 && stored && row_in_tile) {
                                     unsigned char *g = gtile + (size_t)(kk >> 1) * 4 * cb + oe16 + hb;
                                     *reinterpret_cast<uint4 *>(g) = eh;
                                     *reinterpret_cast<uint4 *>(g + cb) = nh;
@@ -947,48 +964,60 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             const MixGroup G = a.groups[gi - J.beg[gk]];
             ItemWindow w;
             w.start(a.items, G.ib, G.ie, lane);
+            // the group's columns: component c of target t is column half c + t
+            // (half: the targets rounded up to 16), so small groups' MMAs are
+            // narrow; the proxy pass has three components of 85 rows, the
+            // upward pass one of 128
+            const int half = (G.nt + 15) & ~15;
+            const uint32_t idesc = idesc_n(F16 ? kIdescF16 : kIdesc, MODE == 0 ? 2 * half : MODE == 1 ? 256 : 128);
             // replay: bytes of one packed tile (east rows, then north rows)
-            const uint32_t ptile = 2u * (uint32_t)((G.nt + 15) & ~15) * 32u;
+            const uint32_t ptile = 2u * (uint32_t)half * 32u;
             for (int k = G.ib; k < G.ie; ++k) {
                 const TcItem it = w.get(k, lane);
                 const int nst = (it.cnt + SK - 1) / SK;
                 for (int j = 0; j < nst; ++j, ++st) {
                     const uint32_t slot = st % KS, jb = st % WS;
                     // replay: the stage's one barrier covers its weight and kernel tiles
-                    if (TS != 2) wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err);
-                    wait_bounded(&sm.kfull[slot], (st / KS) & 1, abort, err);
+                    bool ok = true;
+                    if (TS != 2) ok = wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err);
+                    ok = wait_bounded(&sm.kfull[slot], (st / KS) & 1, abort, err) && ok;
                     // a new chain overwrites the accumulator, whose last chain
                     // (cc - 1) the fold warps must have read
-                    if (!chain_open && cc >= 1) wait_bounded(&sm.accfree, (cc - 1) & 1, abort, err);
+                    if (!chain_open && cc >= 1) ok = wait_bounded(&sm.accfree, (cc - 1) & 1, abort, err) && ok;
+                    ok = __all_sync(0xffffffffu, ok);
                     tc_fence_after();
-                    if (lane == 0) {
-                        if (!*abort) {
-                            const int nks = (min(SK, it.cnt - SK * j) + 7) >> 3;
+                    const int nks = (min(SK, it.cnt - SK * j) + 7) >> 3;
+                    const uint32_t open = chain_open ? 1u : 0u;
+                    if (elect_one()) {
+                        if (ok) {
                             if constexpr (TS == 2) {
                                 // packed tiles of MMA step s: hi at (2s) ptile, lo at (2s + 1) ptile
-                                const unsigned char *tb = sm.ring + sm.toff[slot];
-                                const unsigned char *wb = sm.ring + TcSmem<TS>::kKtBytes + sm.woff[slot];
-                                for (int s = 0; 2 * s < nks; ++s) {
-                                    const uint64_t aw = smem_desc_w16(wb + s * 2 * kW16UnitBytes);
-                                    const uint64_t bh = smem_desc(tb + 2 * s * ptile), bl = smem_desc(tb + (2 * s + 1) * ptile);
-                                    mma_ss_f16(tmem, aw, bh, (chain_open || s > 0) ? 1u : 0u);
-                                    mma_ss_f16(tmem, aw, bl, 1u);
-                                }
-                            } else if constexpr (F16) {
-                                // 16 sources per MMA: weight units 2s and 2s + 1
-                                for (int s = 0; 2 * s < nks; ++s) {
-                                    const uint64_t aw = smem_desc_w16(sm.Wt(jb) + s * (2 * kW16UnitBytes / 4));
-                                    const uint64_t bh = smem_desc(sm.Kt(slot, s, 0)), bl = smem_desc(sm.Kt(slot, s, 1));
-                                    mma_ss_f16(tmem, aw, bh, (chain_open || s > 0) ? 1u : 0u);
-                                    mma_ss_f16(tmem, aw, bl, 1u);
-                                }
+                                const uint64_t aw = smem_desc_w16(sm.ring + TcSmem<TS>::kKtBytes + sm.woff[slot]);
+                                const uint64_t bt = smem_desc(sm.ring + sm.toff[slot]);
+#pragma unroll
+                                for (int s = 0; s < SK / 16; ++s)
+                                    if (2 * s < nks) {
+                                        const uint64_t a = aw + s * (2 * kW16UnitBytes >> 4), bh = bt + 2 * s * (ptile >> 4);
+                                        mma_ss_f16(tmem, a, bh, idesc, s ? 1u : open);
+                                        mma_ss_f16(tmem, a, bh + (ptile >> 4), idesc, 1u);
+                                    }
                             } else {
-                                for (int s = 0; s < nks; ++s) {
-                                    const uint64_t aw = smem_desc(sm.Wt(jb) + s * kWStepFloats);
-                                    const uint64_t bh = smem_desc(sm.Kt(slot, s, 0)), bl = smem_desc(sm.Kt(slot, s, 1));
-                                    mma_ss(tmem, aw, bh, (chain_open || s > 0) ? 1u : 0u);
-                                    mma_ss(tmem, aw, bl, 1u);
-                                }
+                                // FP16: 16 sources per MMA (weight units 2s and 2s + 1); TF32: 8
+                                constexpr uint32_t kStepW = kWStepFloats * 4 >> 4, kStepT = kTileFloats * 4 >> 4;
+                                const uint64_t aw = F16 ? smem_desc_w16(sm.Wt(jb)) : smem_desc(sm.Wt(jb));
+                                const uint64_t bt = smem_desc(sm.Kt(slot, 0, 0));
+#pragma unroll
+                                for (int s = 0; s < kStageKs; ++s)
+                                    if ((F16 ? 2 : 1) * s < nks) {
+                                        const uint64_t a = aw + s * kStepW, bh = bt + 2 * s * kStepT;
+                                        if (F16) {
+                                            mma_ss_f16(tmem, a, bh, idesc, s ? 1u : open);
+                                            mma_ss_f16(tmem, a, bh + kStepT, idesc, 1u);
+                                        } else {
+                                            mma_ss(tmem, a, bh, idesc, s ? 1u : open);
+                                            mma_ss(tmem, a, bh + kStepT, idesc, 1u);
+                                        }
+                                    }
                             }
                         }
                         mma_commit(&sm.kempty[slot]);
@@ -998,7 +1027,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     __syncwarp();
                 }
                 if (it.kind & kTcFlush) {
-                    if (lane == 0) mma_commit(&sm.accfull);
+                    if (elect_one()) mma_commit(&sm.accfull);
                     __syncwarp();
                     chain_open = false;
                     ++cc;
@@ -1006,10 +1035,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             }
         }
         // every MMA issued by this CTA completes before tensor memory is freed
-        if (lane == 0) {
-            mma_commit(&sm.fin);
-            wait_drain(&sm.fin, 0, err);
-        }
+        if (elect_one()) mma_commit(&sm.fin);
+        if (lane == 0) wait_drain(&sm.fin, 0, err);
         __syncwarp();
     } else if (warp == kLoadWarp) {
         // ============================================================ loads
@@ -1032,7 +1059,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     const TcItem nxt = w.get(k + 1, lane);
                     // the next item's weight tiles (and source coordinates)
                     // into L2 while this item's stages run
-                    if (lane == 0 && MODE != 2) {
+                    if (MODE != 2 && elect_one()) {
                         const uint32_t nks = (uint32_t)(nxt.cnt + 7) >> 3;
                         if (F16)
                             prefetch_l2(static_cast<const char *>(a.bstore16) + (size_t)nxt.kb * kW16UnitBytes,
@@ -1067,7 +1094,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                             ++oldest;
                         }
                         const uint32_t slot = st % KS;
-                        if (lane == 0) {
+                        if (elect_one()) {
                             sm.toff[slot] = tpos;
                             sm.tlen[slot] = sb;
                             sm.woff[slot] = wpos;
@@ -1090,7 +1117,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     } else {
                         const uint32_t jb = st % WS, ub = st / WS;
                         if (ub > 0) wait_bounded(&sm.wempty[jb], (ub - 1) & 1, abort, err);
-                        if (lane == 0) {
+                        if (elect_one()) {
                             // FP16: whole 16-source MMA steps (the store has a spare unit at its end)
                             const uint32_t wbytes = F16 ? (uint32_t)((nks + 1) & ~1) * kW16UnitBytes
                                                         : (uint32_t)nks * kWStepFloats * 4;
@@ -1146,7 +1173,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                 continue;
             }
             bool first = true;
-            const int half = TS == 2 ? (G.nt + 15) & ~15 : 128;   // columns per component
+            const int half = MODE == 0 ? (G.nt + 15) & ~15 : 128;   // columns per component
             ItemWindow w;
             w.start(a.items, G.ib, G.ie, lane);
             for (int k = G.ib; k < G.ie; ++k) {
