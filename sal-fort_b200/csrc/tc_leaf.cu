@@ -81,12 +81,12 @@ using dev::smem_u32;
 
 namespace {
 
-constexpr int kProdWarps = 8;
-constexpr int kProducers = kProdWarps * 32;
-constexpr int kMmaWarp = kProdWarps;
-constexpr int kLoadWarp = kProdWarps + 1;
 constexpr int kFoldWarps = 4;                     // one per tensor memory lane quarter
-constexpr int kThreads = (kProdWarps + 2 + kFoldWarps) * 32;   // 448
+// Producer warps of a launch (the MMA, loader and fold warps follow them).
+template <bool F16, int TS>
+constexpr int kProdWarpsOf = 8;
+template <bool F16, int TS>
+constexpr int kThreadsOf = (kProdWarpsOf<F16, TS> + 2 + kFoldWarps) * 32;
 constexpr int kF = 64;                            // fields
 constexpr int kStageK = 32;                       // K columns per stage (four k-steps of 8)
 constexpr int kStageKs = kStageK / 8;             // k-steps per stage
@@ -97,7 +97,8 @@ constexpr int kTileFloats = 2048;                 // kernel tile of one k-step: 
 constexpr int kWStepFloats = 1024;                // weight tile of one k-step: 128 rows x 8
 constexpr int kTmemCols = 512;
 constexpr int kKmap = 3 * (kMaxDegree + 1) * (kMaxDegree + 1) + 64;
-constexpr uint32_t kWaitPolls = 1u << 22;
+constexpr uint32_t kWaitPolls = 1u << 24, kPollNs = 20000;
+constexpr uint64_t kWaitNs = 2000000000ull;
 constexpr float kC1F = (float)dev::kC1;
 constexpr float kTwoC2F = (float)(2.0 * dev::kC2);
 
@@ -116,6 +117,10 @@ constexpr int kW16UnitBytes = 2048;
 // FP16 operands are scaled by powers of two to at most 2^12 (FP16 max 65504)
 constexpr int kF16TopExp = 12;
 static_assert(kStageKF16 == kTcChunk, "an FP16 stage is one item: the tile store's layout");
+// TcSmem::rec flags: units (8 sources) of the stage, its item's kind << 4
+// (kRecDown: 2), the end of an accumulator chain, the group's own points among
+// the sources
+constexpr int kRecUnits = 15, kRecDown = 32, kRecFlush = 64, kRecSelf = 128;
 
 // Replay of the kernel-tile store: the stages' kernel tiles and weight tiles
 // go into two byte rings (a stage takes its own size, so the small groups'
@@ -145,6 +150,10 @@ struct TcSmem {
     float fx[kReplay ? 1 : kTcRows][kMaxDegree + 1];              // per target row: BLI bases in the current DOWN slot
     float fe[kReplay ? 1 : kTcRows][kMaxDegree + 1];
     int kmap[kReplay ? 1 : kKmap];
+    // FP16 computing launches, per weight stage, its item as the loader saw it:
+    // (dx, dy, dz, flags: kRec*) and (off, row0)
+    float4 rec[kReplay ? 1 : kWStages];
+    int2 rec2[kReplay ? 1 : kWStages];
     uint32_t toff[KS], tlen[KS], woff[KS], wlen[KS];             // replay: each stage slot's ranges in the rings
     uint64_t kfull[KS], kempty[KS], wfull[WS], wempty[WS], accfull, accfree, fin;
     uint32_t tmem_base;
@@ -194,14 +203,19 @@ __device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
 
 using dev::mbar_arrive;
 // Bounded wait on an mbarrier phase; on time-out raises the error flag and
-// the CTA-wide abort flag (later waits then give up after one poll).  A phase
-// that has already completed costs one poll and no read of the flag: every
-// shared-memory round trip is on the producers' critical path.
+// the CTA-wide abort flag (later waits then give up at once).  A phase that
+// has already completed costs one poll and no read of the flag: every
+// shared-memory round trip is on the producers' critical path.  After that a
+// poll suspends the warp for up to kPollNs: polls without a time hint come back
+// early, and the six waiting warps' loops took more issue slots than the
+// producers' arithmetic.  The limits are kWaitNs and kWaitPolls.
 __device__ __forceinline__ bool wait_bounded(uint64_t *bar, uint32_t parity, volatile int *abort, int *err) {
     if (dev::mbar_try_wait(bar, parity)) return true;
+    const uint64_t t0 = dev::global_ns();
     for (uint32_t it = 0; it < kWaitPolls; ++it) {
         if (*abort) return false;
-        if (dev::mbar_try_wait(bar, parity)) return true;
+        if (dev::mbar_try_wait_ns(bar, parity, kPollNs)) return true;
+        if (dev::global_ns() - t0 > kWaitNs) break;
     }
     *abort = 1;
     atomicExch(err, dev::kErrTimeout);
@@ -210,13 +224,16 @@ __device__ __forceinline__ bool wait_bounded(uint64_t *bar, uint32_t parity, vol
 // Bounded wait that ignores the abort flag (drains copies and MMAs in flight
 // before the CTA exits).
 __device__ __forceinline__ void wait_drain(uint64_t *bar, uint32_t parity, int *err) {
-    for (uint32_t it = 0; it < kWaitPolls; ++it)
-        if (dev::mbar_try_wait(bar, parity)) return;
+    const uint64_t t0 = dev::global_ns();
+    for (uint32_t it = 0; it < kWaitPolls; ++it) {
+        if (dev::mbar_try_wait_ns(bar, parity, kPollNs)) return;
+        if (dev::global_ns() - t0 > kWaitNs) break;
+    }
     atomicExch(err, dev::kErrTimeout);
 }
 
 // Named barrier 1 over the producer warps.
-__device__ __forceinline__ void producers_sync() { asm volatile("bar.sync 1, %0;" ::"r"(kProducers) : "memory"); }
+__device__ __forceinline__ void producers_sync(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -557,7 +574,9 @@ struct ItemWindow {
 // 2 the loader copies them from the store into the kernel-tile ring and the
 // producers only write the outputs of groups without sources.
 template <int MODE, bool JOINT, bool F16, int TS = 0>
-__global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_constant__ TcJoint J, int *err) {
+__global__ void __launch_bounds__(kThreadsOf<F16, TS>, 1) tc_leaf_kernel(const __grid_constant__ TcJoint J, int *err) {
+    constexpr int kProdWarps = kProdWarpsOf<F16, TS>, kMmaWarp = kProdWarps, kLoadWarp = kProdWarps + 1;
+    constexpr int kThreads = kThreadsOf<F16, TS>;
     static_assert(!F16 || MODE == 0, "FP16 operands in the leaf pass only");
     static_assert(TS == 0 || (MODE == 0 && F16 && !JOINT), "kernel-tile store: FP16 leaf pass of one grid");
     constexpr int SK = F16 ? kStageKF16 : kStageK;   // sources per stage
@@ -643,7 +662,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             const int rb = (G.nt + 31) >> 5;
             const int wb = rb >= 3 ? (warp & 3) : rb == 2 ? (warp & 1) : 0;            // row block
             const int kfirst = rb >= 3 ? (warp >> 2) : rb == 2 ? (warp >> 1) : warp;    // first k-step
-            const int kstride = rb >= 3 ? 2 : rb == 2 ? 4 : 8;
+            const int kstride = rb >= 3 ? kProdWarps / 4 : rb == 2 ? kProdWarps / 2 : kProdWarps;
             const int row = 32 * wb + lane;
             const bool active = 32 * wb < G.nt, rvalid = row < G.nt;
             // canonical offsets (floats) of this thread's rows in a kernel tile:
@@ -656,7 +675,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             const bool row_in_tile = row < (MODE == 0 ? half : MODE == 1 ? kTcProxyRows : kTcRows);
             // FP16 tiles: byte offset of the row's first K core matrix (8-row
             // groups 256 B apart, the two K halves 128 B apart)
-            const int oe16 = (row >> 3) * 256 + (row & 7) * 16, on16 = oe16 + half * 32;
+            const int oe16 = (row >> 3) * 256 + (row & 7) * 16;
             // the row's target relative to the leaf centre and its east /
             // north unit vectors (zero at the poles, as the reference's guard)
             float tl0 = 0.f, tl1 = 0.f, tl2 = 0.f, el0 = 0.f, el1 = 0.f, ep0 = 0.f, ep1 = 0.f, ep2 = 0.f;
@@ -702,6 +721,187 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             // rounded up to 16, each the bytes of the ring's rows
             const size_t cb = (size_t)half * 32;
             unsigned char *gtile = (TS == 1 || TS == 3) ? a.ktile + a.ktile_off[gi - J.beg[gk]] : nullptr;
+            if constexpr (F16) {
+                // FP16: an item is one stage, and its record comes to shared
+                // memory with its weights: the loop costs a warp about as much
+                // per stage as a task does, so it holds nothing else
+#pragma unroll 1
+                for (int k = 0; k < ni; ++k, ++st) {
+                    const uint32_t slot = st % KS, kpar = ((st / KS) - 1) & 1, jb = st % WS;
+                    bool slot_free = st < (uint32_t)KS;
+                    // an item the kernel-tile store holds (one in tile_every)
+                    const bool stored = (TS == 1 || TS == 3) && k % a.tile_every == a.tile_every - 1;
+                    wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err);
+                    const float4 rec = sm.rec[jb];
+                    const int flags = __float_as_int(rec.w), nks = flags & kRecUnits;
+                    if (TS == 3 && stored) {
+                        // replay: warp 0 copies the stage's chunks (MMA step q / 4, hi / lo,
+                        // east / north) into the ring slot once the MMAs that last read it
+                        // are done; its arrival carries the bytes
+                        const int nq = 4 * ((nks + 1) >> 1);
+                        if (!slot_free) wait_bounded(&sm.kempty[slot], kpar, abort, err);
+                        if (warp == 0) {
+                            if (lane == 0) dev::mbar_expect_tx(&sm.kfull[slot], (uint32_t)(nq * cb));
+                            __syncwarp();
+                            if (lane < nq && !*abort)
+                                dev::bulk_g2s_hint(
+                                    reinterpret_cast<unsigned char *>(sm.Kt(slot, lane >> 2, (lane >> 1) & 1)) + (lane & 1) * cb,
+                                    gtile + (size_t)lane * cb, (uint32_t)cb, &sm.kfull[slot], dev::l2_evict_first());
+                        } else if (lane == 0) {
+                            mbar_arrive(&sm.kfull[slot]);
+                        }
+                        __syncwarp();
+                        gtile += (size_t)nq * cb;
+                        continue;
+                    }
+                    const float2 tx2 = f2(tl0 - rec.x), ty2 = f2(tl1 - rec.y), tz2 = f2(tl2 - rec.z);
+                    // the sources' x[8] y[8] z[8] per unit (the same address in every
+                    // lane: shared-memory broadcasts), and this row's place in the tile
+                    const float2 *crd = reinterpret_cast<const float2 *>(sm.aux[jb]);
+                    char *tile = reinterpret_cast<char *>(sm.Kt(slot, 0, 0)) + oe16;
+                    // a K task's kernel values (units kk, kk + dk, ...), two columns per
+                    // packed instruction, as FP16 hi + lo words o[task] = {east hi, east
+                    // lo, north hi, north lo}, packed as they are computed: 4 K
+                    // independent chains in one block of code
+                    auto pairs16 = [&]<int K>(int kk, int dk, uint32_t (&o)[K][4][4]) {
+#pragma unroll
+                        for (int c2 = 0; c2 < 4; ++c2)
+#pragma unroll
+                            for (int t = 0; t < K; ++t) {
+                                const float2 *cr = crd + 12 * (kk + t * dk) + c2;
+                                const float2 dx = sub2(cr[0], tx2), dy = sub2(cr[4], ty2), dz = sub2(cr[8], tz2);
+                                // + 1e-20: mp = 0 only for a source on the target itself (or
+                                // a repeated point), and the floor keeps the value finite;
+                                // chords of neighbours (mp >= 1e-12) do not see it
+                                const float2 mp = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, f2(1e-20f))));
+                                const float2 r = make_float2(rsqrt_approx(mp.x), rsqrt_approx(mp.y));
+                                const float2 w = __fadd2_rn(__fmul2_rn(mp, r), f2(2.f));
+                                const float2 u = make_float2(rcp_approx(w.x), rcp_approx(w.y));
+                                const float2 inner = __ffma2_rn(f2(kC1F), r, __ffma2_rn(f2(kTwoC2F), u, f2(-kTwoC2F)));
+                                const float2 v = __fmul2_rn(inner, __fmul2_rn(r, r));
+                                const float2 pe = __ffma2_rn(el1v, dy, __fmul2_rn(el0v, dx));
+                                const float2 pn = __ffma2_rn(ep2v, dz, __ffma2_rn(ep1v, dy, __fmul2_rn(ep0v, dx)));
+                                const float2 e2 = __fmul2_rn(v, pe), n2 = __fmul2_rn(v, pn);
+                                split_f16x2(e2.x, e2.y, o[t][0][c2], o[t][1][c2]);
+                                split_f16x2(n2.x, n2.y, o[t][2][c2], o[t][3][c2]);
+                            }
+                    };
+                    // unit kk is K half kk & 1 of MMA step kk / 2, the row's 8 values
+                    // one 16-byte core-matrix row
+                    auto store16 = [&](int kk, const uint32_t (&o)[4][4]) {
+                        if (!row_in_tile) return;
+                        char *t = tile + (kk >> 1) * (2 * kTileFloats * 4) + 128 * (kk & 1);
+                        const uint4 eh = make_uint4(o[0][0], o[0][1], o[0][2], o[0][3]), el = make_uint4(o[1][0], o[1][1], o[1][2], o[1][3]);
+                        const uint4 nh = make_uint4(o[2][0], o[2][1], o[2][2], o[2][3]), nl = make_uint4(o[3][0], o[3][1], o[3][2], o[3][3]);
+                        *reinterpret_cast<uint4 *>(t) = eh;
+                        *reinterpret_cast<uint4 *>(t + kTileFloats * 4) = el;
+                        *reinterpret_cast<uint4 *>(t + half * 32) = nh;
+                        *reinterpret_cast<uint4 *>(t + half * 32 + kTileFloats * 4) = nl;
+                        if (TS == 1 && stored) {
+                            unsigned char *g = gtile + (size_t)(kk >> 1) * 4 * cb + oe16 + 128 * (kk & 1);
+                            *reinterpret_cast<uint4 *>(g) = eh;
+                            *reinterpret_cast<uint4 *>(g + cb) = nh;
+                            *reinterpret_cast<uint4 *>(g + 2 * cb) = el;
+                            *reinterpret_cast<uint4 *>(g + 3 * cb) = nl;
+                        }
+                    };
+                    // the MMAs that last read the slot must be done before the first
+                    // store into it
+                    auto claim = [&]() {
+                        if (!slot_free) wait_bounded(&sm.kempty[slot], kpar, abort, err);
+                        slot_free = true;
+                    };
+                    int kk = active ? kfirst : nks + 1;
+                    if (!(flags & (kRecDown | kRecSelf))) {
+#pragma unroll 1
+                        for (; kk + kstride < nks; kk += 2 * kstride) {
+                            uint32_t o[2][4][4];
+                            pairs16(kk, kstride, o);
+                            claim();
+                            store16(kk, o[0]);
+                            store16(kk + kstride, o[1]);
+                        }
+                    } else if (flags & kRecDown) {
+                        const int slot_id = sm.rec2[jb].x;
+                        if (slot_id != cur_slot) {
+                            // BLI bases of every target row in the new slot: thread
+                            // t < 128 the xi basis of target t, thread 128 + t its
+                            // eta basis
+                            cur_slot = slot_id;
+                            producers_sync(32 * kProdWarps);
+                            const int brow = tid & (kTcRows - 1);
+                            if (brow < G.nt) {
+                                const double2 e = a.xieta[G.tgt + brow];
+                                const double *nodes = a.tgt_nodes + (size_t)slot_id * 2 * n;
+                                if (tid < kTcRows) down_basis(e.x, nodes, n, sm.fx[brow]);
+                                else down_basis(e.y, nodes + n, n, sm.fe[brow]);
+                            }
+                            producers_sync(32 * kProdWarps);
+                        }
+                    }
+#pragma unroll 1
+                    for (; kk < ((nks + 1) & ~1); kk += kstride) {
+                        uint32_t o[1][4][4];
+                        if (kk >= nks) {
+                            // an odd last unit's partner in its 16-source MMA step
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) o[0][0][c] = o[0][1][c] = o[0][2][c] = o[0][3][c] = 0u;
+                        } else if (flags & kRecDown) {
+                            // BLI basis of the target x its unit vector's component of the
+                            // Cartesian row
+                            const int *km0 = sm.kmap + sm.rec2[jb].y + 8 * kk;
+                            const float *fxr = sm.fx[row], *fer = sm.fe[row];
+#pragma unroll
+                            for (int c2 = 0; c2 < 4; ++c2) {
+                                float e[2], nn[2];
+#pragma unroll
+                                for (int c = 0; c < 2; ++c) {
+                                    const int km = km0[2 * c2 + c];
+                                    const float b = fxr[km & 255] * fer[(km >> 8) & 255];
+                                    const int comp = km >> 16;
+                                    e[c] = comp == 2 ? 0.f : b * (comp == 0 ? el0 : el1);
+                                    nn[c] = b * (comp == 0 ? ep0 : (comp == 1 ? ep1 : ep2));
+                                }
+                                split_f16x2(e[0], e[1], o[0][0][c2], o[0][1][c2]);
+                                split_f16x2(nn[0], nn[1], o[0][2][c2], o[0][3][c2]);
+                            }
+                        } else {
+                            pairs16(kk, 0, o);
+                        }
+                        claim();
+                        store16(kk, o[0]);
+                        if (flags & kRecSelf) {
+                            // the target itself among these 8 sources: the self pair's
+                            // halves over the tile entry just stored
+                            const int cs = my_pos - (sm.rec2[jb].x + 8 * kk);
+                            if (row_in_tile && kk < nks && (unsigned)cs < 8u) {
+                                uint32_t h, l;
+                                split_f16x2(self_e, self_n, h, l);
+                                char *t = tile + (kk >> 1) * (2 * kTileFloats * 4) + 128 * (kk & 1) + 2 * cs;
+                                *reinterpret_cast<uint16_t *>(t) = (uint16_t)h;
+                                *reinterpret_cast<uint16_t *>(t + kTileFloats * 4) = (uint16_t)l;
+                                *reinterpret_cast<uint16_t *>(t + half * 32) = (uint16_t)(h >> 16);
+                                *reinterpret_cast<uint16_t *>(t + half * 32 + kTileFloats * 4) = (uint16_t)(l >> 16);
+                                if (TS == 1 && stored) {
+                                    unsigned char *g = gtile + (size_t)(kk >> 1) * 4 * cb + oe16 + 128 * (kk & 1) + 2 * cs;
+                                    *reinterpret_cast<uint16_t *>(g) = (uint16_t)h;
+                                    *reinterpret_cast<uint16_t *>(g + cb) = (uint16_t)(h >> 16);
+                                    *reinterpret_cast<uint16_t *>(g + 2 * cb) = (uint16_t)l;
+                                    *reinterpret_cast<uint16_t *>(g + 3 * cb) = (uint16_t)(l >> 16);
+                                }
+                            }
+                        }
+                    }
+                    // warps that wrote nothing: their arrival must still not run a
+                    // ring phase ahead of the MMAs
+                    claim();
+                    dev::fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sm.kfull[slot]);
+                    if (TS == 1 && stored) gtile += (size_t)4 * ((nks + 1) >> 1) * cb;
+                }
+                continue;
+            }
             // item records are read one item ahead, so their latency hides
             // behind the current item's stages
             TcItem nxt = a.items[G.ib];
@@ -710,44 +910,20 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                 if (k + 1 < ni) nxt = a.items[G.ib + k + 1];
                 const int kind = it.kind & 3;
                 const int nst = (it.cnt + SK - 1) / SK;
-                // an item the kernel-tile store holds (one in tile_every)
-                const bool stored = (TS == 1 || TS == 3) && k % a.tile_every == a.tile_every - 1;
-                if (TS == 3 && stored) {
-                    // replay: warp 0 copies the stage's chunks (MMA step q / 4, hi / lo,
-                    // east / north) into the ring slot once the MMAs that last read it
-                    // are done; its arrival carries the bytes
-                    const uint32_t slot = st % KS, kpar = ((st / KS) - 1) & 1;
-                    const int nq = 4 * (((min(SK, it.cnt) + 7) / 8 + 1) / 2);
-                    if (st >= (uint32_t)KS) wait_bounded(&sm.kempty[slot], kpar, abort, err);
-                    if (warp == 0) {
-                        if (lane == 0) dev::mbar_expect_tx(&sm.kfull[slot], (uint32_t)(nq * cb));
-                        __syncwarp();
-                        if (lane < nq && !*abort)
-                            dev::bulk_g2s_hint(reinterpret_cast<unsigned char *>(sm.Kt(slot, lane >> 2, (lane >> 1) & 1)) +
-                                                   (lane & 1) * cb,
-                                               gtile + (size_t)lane * cb, (uint32_t)cb, &sm.kfull[slot], dev::l2_evict_first());
-                    } else if (lane == 0) {
-                        mbar_arrive(&sm.kfull[slot]);
-                    }
-                    __syncwarp();
-                    gtile += (size_t)nq * cb;
-                    ++st;
-                    continue;
-                }
                 if (MODE == 0 && kind == 2 && it.off != cur_slot) {
                     // BLI bases of every target row in the new slot: thread
                     // t < 128 the xi basis of target t, thread 128 + t its
                     // eta basis
                     cur_slot = it.off;
-                    producers_sync();
+                    producers_sync(32 * kProdWarps);
                     const int brow = tid & (kTcRows - 1);
-                    if (brow < G.nt) {
+                    if (brow < G.nt && tid < 2 * kTcRows) {
                         const double2 e = a.xieta[G.tgt + brow];
                         const double *nodes = a.tgt_nodes + (size_t)it.off * 2 * n;
                         if (tid < kTcRows) down_basis(e.x, nodes, n, sm.fx[brow]);
                         else down_basis(e.y, nodes + n, n, sm.fe[brow]);
                     }
-                    producers_sync();
+                    producers_sync(32 * kProdWarps);
                 }
                 const float2 tx2 = f2(tl0 - it.dx), ty2 = f2(tl1 - it.dy), tz2 = f2(tl2 - it.dz);
                 // only the item whose sources are the group's own points holds
@@ -849,36 +1025,6 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     };
                     // its TF32 hi + lo split, stored into the kernel tile
                     auto store = [&](int kk, const float (&ve)[8], const float (&vn)[8], const float (&vz)[8]) {
-                            if constexpr (F16) {
-                                // FP16 hi + lo: unit kk is K half kk & 1 of MMA step kk / 2,
-                                // the row's 8 values one 16-byte core-matrix row
-                                char *th = reinterpret_cast<char *>(sm.Kt(slot, kk >> 1, 0));
-                                char *tlo = reinterpret_cast<char *>(sm.Kt(slot, kk >> 1, 1));
-                                const int hb = 128 * (kk & 1);
-                                uint4 eh, el, nh, nl;
-                                split_f16x2(ve[0], ve[1], eh.x, el.x);
-                                split_f16x2(ve[2], ve[3], eh.y, el.y);
-                                split_f16x2(ve[4], ve[5], eh.z, el.z);
-                                split_f16x2(ve[6], ve[7], eh.w, el.w);
-                                split_f16x2(vn[0], vn[1], nh.x, nl.x);
-                                split_f16x2(vn[2], vn[3], nh.y, nl.y);
-                                split_f16x2(vn[4], vn[5], nh.z, nl.z);
-                                split_f16x2(vn[6], vn[7], nh.w, nl.w);
-                                if (row_in_tile) {
-                                    *reinterpret_cast<uint4 *>(th + oe16 + hb) = eh;
-                                    *reinterpret_cast<uint4 *>(tlo + oe16 + hb) = el;
-                                    *reinterpret_cast<uint4 *>(th + on16 + hb) = nh;
-                                    *reinterpret_cast<uint4 *>(tlo + on16 + hb) = nl;
-                                }
-                                if (TS == 1 && stored && row_in_tile) {
-                                    unsigned char *g = gtile + (size_t)(kk >> 1) * 4 * cb + oe16 + hb;
-                                    *reinterpret_cast<uint4 *>(g) = eh;
-                                    *reinterpret_cast<uint4 *>(g + cb) = nh;
-                                    *reinterpret_cast<uint4 *>(g + 2 * cb) = el;
-                                    *reinterpret_cast<uint4 *>(g + 3 * cb) = nl;
-                                }
-                                return;
-                            }
                             // TF32 hi + lo (the tensor cores read lo's top 11 bits)
                             float *th = sm.Kt(slot, kk, 0), *tlo = sm.Kt(slot, kk, 1);
 #pragma unroll
@@ -911,35 +1057,26 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                                 }
                             }
                     };
-                    // FP16: an odd last unit's partner in its 16-source MMA
-                    // step is written as zeros
-                    const int nut = F16 ? ((nks + 1) & ~1) : nks;
-                    auto compute = [&](int k, float (&ve)[8], float (&vn)[8], float (&vz)[8]) {
-                        if (!F16 || k < nks) {
-                            values(k, ve, vn, vz);   // FP16: kernel values come scaled
-                        } else {
-#pragma unroll
-                            for (int c = 0; c < 8; ++c) ve[c] = vn[c] = vz[c] = 0.f;
-                        }
-                    };
-                    // The proxy pass takes two tasks at a time (their values are
-                    // independent, so the second's arithmetic fills the first's
-                    // latencies; measured 5 % on that pass).  The leaf pass gains
-                    // nothing from it and keeps its registers.
-                    constexpr int kPair = MODE == 1 ? 2 : 1;
+                    {
+                        // The proxy pass takes two tasks at a time (their values are
+                        // independent, so the second's arithmetic fills the first's
+                        // latencies; measured 5 % on that pass).  The leaf pass gains
+                        // nothing from it and keeps its registers.
+                        constexpr int kPair = MODE == 1 ? 2 : 1;
 #pragma unroll 1
-                    for (int kk = kfirst; active && kk < nut; kk += kPair * kstride) {
-                        float ve[8], vn[8], vz[8], ve2[8], vn2[8], vz2[8];
-                        const int k2 = kk + kstride;
-                        const bool two = kPair == 2 && k2 < nut;
-                        compute(kk, ve, vn, vz);
-                        if (kPair == 2) compute(two ? k2 : kk, ve2, vn2, vz2);
-                        if (!slot_free) {
-                            wait_bounded(&sm.kempty[slot], kpar, abort, err);
-                            slot_free = true;
+                        for (int kk = kfirst; active && kk < nks; kk += kPair * kstride) {
+                            float ve[8], vn[8], vz[8], ve2[8], vn2[8], vz2[8];
+                            const int k2 = kk + kstride;
+                            const bool two = kPair == 2 && k2 < nks;
+                            values(kk, ve, vn, vz);
+                            if (kPair == 2) values(two ? k2 : kk, ve2, vn2, vz2);
+                            if (!slot_free) {
+                                wait_bounded(&sm.kempty[slot], kpar, abort, err);
+                                slot_free = true;
+                            }
+                            store(kk, ve, vn, vz);
+                            if (two) store(k2, ve2, vn2, vz2);
                         }
-                        store(kk, ve, vn, vz);
-                        if (two) store(k2, ve2, vn2, vz2);
                     }
                     if (!slot_free) {
                         // warps that wrote nothing: their arrival must still
@@ -950,7 +1087,6 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     }
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sm.kfull[slot]);
-                    if (TS == 1 && stored) gtile += (size_t)4 * ((nks + 1) >> 1) * cb;
                 }
             }
         }
@@ -962,8 +1098,11 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             const int gk = grid_of(gi);
             const TcArgs &a = J.g[gk];
             const MixGroup G = a.groups[gi - J.beg[gk]];
+            // FP16 computing launches take an item's units and chain end from the
+            // loader's record
+            constexpr bool kRec = F16 && TS != 2;
             ItemWindow w;
-            w.start(a.items, G.ib, G.ie, lane);
+            if (!kRec) w.start(a.items, G.ib, G.ie, lane);
             // the group's columns: component c of target t is column half c + t
             // (half: the targets rounded up to 16), so small groups' MMAs are
             // narrow; the proxy pass has three components of 85 rows, the
@@ -973,8 +1112,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             // replay: bytes of one packed tile (east rows, then north rows)
             const uint32_t ptile = 2u * (uint32_t)half * 32u;
             for (int k = G.ib; k < G.ie; ++k) {
-                const TcItem it = w.get(k, lane);
-                const int nst = (it.cnt + SK - 1) / SK;
+                TcItem it{};
+                if (!kRec) it = w.get(k, lane);
+                bool flush = it.kind & kTcFlush;
+                const int nst = kRec ? 1 : (it.cnt + SK - 1) / SK;
                 for (int j = 0; j < nst; ++j, ++st) {
                     const uint32_t slot = st % KS, jb = st % WS;
                     // replay: the stage's one barrier covers its weight and kernel tiles
@@ -986,7 +1127,12 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     if (!chain_open && cc >= 1) ok = wait_bounded(&sm.accfree, (cc - 1) & 1, abort, err) && ok;
                     ok = __all_sync(0xffffffffu, ok);
                     tc_fence_after();
-                    const int nks = (min(SK, it.cnt - SK * j) + 7) >> 3;
+                    int nks = (min(SK, it.cnt - SK * j) + 7) >> 3;
+                    if (kRec) {
+                        const int flags = __float_as_int(sm.rec[jb].w);
+                        nks = flags & kRecUnits;
+                        flush = flags & kRecFlush;
+                    }
                     const uint32_t open = chain_open ? 1u : 0u;
                     if (elect_one()) {
                         if (ok) {
@@ -1026,7 +1172,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     chain_open = true;
                     __syncwarp();
                 }
-                if (it.kind & kTcFlush) {
+                if (flush) {
                     if (elect_one()) mma_commit(&sm.accfull);
                     __syncwarp();
                     chain_open = false;
@@ -1126,6 +1272,14 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                             // k-step; DOWN rows need none)
                             const uint32_t lbytes = MODE == 2 ? (uint32_t)nks * 64 * n
                                                     : (it.kind & 3) != 2 ? (uint32_t)nks * 96u : 0u;
+                            if constexpr (F16) {
+                                // written before the arrival that its readers wait for
+                                const bool self = (it.kind & 3) == 0 && it.off < G.tgt + G.nt && G.tgt < it.off + it.cnt;
+                                const int flags = nks | (it.kind & 3) << 4 | ((it.kind & kTcFlush) ? kRecFlush : 0) |
+                                                  (self ? kRecSelf : 0);
+                                sm.rec[jb] = make_float4(it.dx, it.dy, it.dz, __int_as_float(flags));
+                                sm.rec2[jb] = make_int2(it.off, it.row0);
+                            }
                             dev::mbar_expect_tx(&sm.wfull[jb], wbytes + lbytes);
                             if (!*abort) {
                                 if (lbytes)
@@ -1448,7 +1602,7 @@ static void launch_tc(const TcJoint &J, int nsm, int cta_groups, int *err, cudaS
     const int per = cta_groups > 0 ? cta_groups : 1;
     int grid = (total + per - 1) / per;
     if (grid < nsm) grid = total < nsm ? total : nsm;
-    tc_leaf_kernel<MODE, JOINT, F16, TS><<<grid, kThreads, smem, st>>>(J, err);
+    tc_leaf_kernel<MODE, JOINT, F16, TS><<<grid, kThreadsOf<F16, TS>, smem, st>>>(J, err);
 }
 
 template <int MODE, bool F16 = false, int TS = 0>
