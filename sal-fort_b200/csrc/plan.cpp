@@ -979,10 +979,14 @@ bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *e
         const int kt = leaves[g.out];
         const int32_t ib = range[x].first, ie = range[x].second;
         if (tree && leaf_phi_block[g.out] >= 0) pl->tc_macs_down += (double)g.nt * P;
+        // DOWN items end the list (the work lists hold them after all others)
+        int32_t ndown = 0;
+        while (ndown < ie - ib && (pl->tc_items[ie - 1 - ndown].kind & 3) == 2) ++ndown;
         for (int32_t r = 0; r < g.nt; r += kTcRows) {
             MixGroup m{};
             m.tgt = g.tgt + r; m.nt = std::min(kTcRows, g.nt - r); m.ib = ib; m.ie = ie; m.out = g.out;
             m.cx = t.cx[kt]; m.cy = t.cy[kt]; m.cz = t.cz[kt];
+            m.ndown = ndown;
             pl->tc_leaf_groups.push_back(m);
         }
     }

@@ -110,9 +110,9 @@ struct UpUnit {          // upward-pass work unit
 // Target group of the batched (mixed-precision) kernels: at most 64 targets
 // (four 16-row tensor-core tiles) with a local coordinate origin (cx, cy, cz)
 // near them.  row0: first target row of the group within its panel (proxy
-// groups) or 0.
+// groups) or 0.  ndown: DOWN items at the end of the list (tcgen05 leaf groups).
 struct MixGroup {
-    int32_t tgt, nt, ib, ie, out, row0, pad0, pad1;
+    int32_t tgt, nt, ib, ie, out, row0, ndown, pad1;
     double cx, cy, cz, pad2;
 };
 

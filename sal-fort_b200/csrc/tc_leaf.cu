@@ -82,11 +82,9 @@ using dev::smem_u32;
 namespace {
 
 constexpr int kFoldWarps = 4;                     // one per tensor memory lane quarter
-// Producer warps of a launch (the MMA, loader and fold warps follow them).
-template <bool F16, int TS>
-constexpr int kProdWarpsOf = 8;
-template <bool F16, int TS>
-constexpr int kThreadsOf = (kProdWarpsOf<F16, TS> + 2 + kFoldWarps) * 32;
+constexpr int kProdWarps = 8;
+constexpr int kMmaWarp = kProdWarps, kLoadWarp = kProdWarps + 1;
+constexpr int kThreads = (kProdWarps + 2 + kFoldWarps) * 32;   // 448
 constexpr int kF = 64;                            // fields
 constexpr int kStageK = 32;                       // K columns per stage (four k-steps of 8)
 constexpr int kStageKs = kStageK / 8;             // k-steps per stage
@@ -233,6 +231,9 @@ __device__ __forceinline__ void wait_drain(uint64_t *bar, uint32_t parity, int *
 }
 
 // Named barrier 1 over the producer warps.
+__device__ __forceinline__ void mbar_arrive_n(uint64_t *bar, uint32_t n) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
+}
 __device__ __forceinline__ void producers_sync(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -328,6 +329,32 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) 
         "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) {
+    uint32_t r[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(v[i]);
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+        "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+        "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // BLI basis (FP64, stored as FP32) of one coordinate of a target over one
@@ -417,6 +444,11 @@ __device__ __forceinline__ int fold_per(bool end, int nt, int half) {
     return (MODE != 1 && end) ? (nt + 15) / 16 : (MODE == 0 ? half / 16 : 8);
 }
 
+// The MMA warp waits for the fold, so it is short: the chunks are contiguous
+// columns (16 i), taken 32 at a time; a kernel chain's factor is a power of
+// two, so factor and add are one packed fused multiply-add with the same bits;
+// and the next chain columns are on their way while a result is stored (full
+// group: 4,300 -> FOLDNEW cycles a chain).
 template <int MODE>
 __device__ __noinline__ void fold_chain(uint32_t td, int lane, bool end, bool first, int tgt, int nt, bool scaled,
                                         float fsc, bool down, const float *__restrict__ tscale, int half, int part_i,
@@ -426,45 +458,57 @@ __device__ __noinline__ void fold_chain(uint32_t td, int lane, bool end, bool fi
     if (MODE == 0 && scaled && down)
 #pragma unroll
         for (int k = 0; k < 4; ++k) csd[k] = 32 * k + lane < nt ? tscale[tgt + 32 * k + lane] : 1.f;
-    // the chain into the running sums' domain, on a 16-column chunk starting at column c
-    auto unscale = [&](float (&x)[16], int c) {
-        if (!scaled) return;
+    const int per = fold_per<MODE>(end, nt, half);
+    const int ncol = 16 * (MODE == 2 ? per : 2 * per);   // component c's chunk j is columns half c + 16 j, half = 16 per
+    const float2 f2v = f2(scaled && !down ? fsc : 1.f);
+    // DOWN chains: the field's factor, then the column's
+    auto unscale = [&](float *x, int c) {
 #pragma unroll
         for (int m = 0; m < 16; ++m) x[m] *= fsc;
-        if (down) {
-            const int b = c >= half ? c - half : c, k = b >> 5;
-            const float src = k == 0 ? csd[0] : k == 1 ? csd[1] : k == 2 ? csd[2] : csd[3];
+        const int b = c >= half ? c - half : c, k = b >> 5;
+        const float src = k == 0 ? csd[0] : k == 1 ? csd[1] : k == 2 ? csd[2] : csd[3];
 #pragma unroll
-            for (int m = 0; m < 16; ++m) x[m] *= __shfl_sync(0xffffffffu, src, (b & 31) + m);
-        }
+        for (int m = 0; m < 16; ++m) x[m] *= __shfl_sync(0xffffffffu, src, (b & 31) + m);
     };
-    const int per = fold_per<MODE>(end, nt, half);
-    const int nchunk = MODE == 2 ? per : 2 * per;   // upward: one component, columns 0..127
-    auto col = [&](int i) { return (i / per) * half + (i % per) * 16; };
-    // two chunks' loads in flight per wait: the MMA warp waits for this fold
-    float x0[16], x1[16], r0[16], r1[16];
-#pragma unroll 1
-    for (int i = 2 * part_i; i < nchunk; i += 2 * nparts) {
-        const bool two = i + 1 < nchunk;   // a group's end in the upward pass can leave one
-        const int c0 = col(i), c1 = col(two ? i + 1 : i);
-        tmem_ld16(td + c0, x0);
-        tmem_ld16(td + c1, x1);
-        if (!first) {
-            tmem_ld16(td + 256 + c0, r0);
-            tmem_ld16(td + 256 + c1, r1);
-        }
-        tmem_wait_ld();
-        unscale(x0, c0);
-        unscale(x1, c1);
-        if (!first) {
+    auto add = [&](float *x, const float *r) {   // 2 columns
+        float2 v = make_float2(x[0], x[1]);
+        v = first ? __fmul2_rn(v, f2v) : __ffma2_rn(v, f2v, make_float2(r[0], r[1]));
+        x[0] = v.x;
+        x[1] = v.y;
+    };
+    float x[32], r[32];
 #pragma unroll
-            for (int m = 0; m < 16; ++m) {
-                x0[m] += r0[m];
-                x1[m] += r1[m];
-            }
+    for (int m = 0; m < 32; ++m) r[m] = 0.f;
+    int c = 32 * part_i;
+    if (c + 32 <= ncol) tmem_ld32(td + c, x);
+#pragma unroll 1
+    for (; c + 32 <= ncol; c += 32 * nparts) {
+        if (!first) tmem_ld32(td + 256 + c, r);
+        tmem_wait_ld();
+        if (MODE == 0 && scaled && down) {
+            unscale(x, c);
+            unscale(x + 16, c + 16);
         }
-        tmem_st16(td + 256 + c0, x0);
-        if (two) tmem_st16(td + 256 + c1, x1);
+        float y[32];
+#pragma unroll
+        for (int m = 0; m < 32; ++m) y[m] = x[m];
+#pragma unroll
+        for (int m = 0; m < 32; m += 2) add(y + m, r + m);
+        if (c + 32 * nparts + 32 <= ncol) tmem_ld32(td + c + 32 * nparts, x);
+        tmem_st32(td + 256 + c, y);
+    }
+    if (c < ncol) {   // an odd chunk left
+        float x1[16], r1[16];
+        tmem_ld16(td + c, x1);
+        if (!first) tmem_ld16(td + 256 + c, r1);
+        else
+#pragma unroll
+            for (int m = 0; m < 16; ++m) r1[m] = 0.f;
+        tmem_wait_ld();
+        if (MODE == 0 && scaled && down) unscale(x1, c);
+#pragma unroll
+        for (int m = 0; m < 16; m += 2) add(x1 + m, r1 + m);
+        tmem_st16(td + 256 + c, x1);
     }
     tmem_wait_st();
 }
@@ -574,9 +618,7 @@ struct ItemWindow {
 // 2 the loader copies them from the store into the kernel-tile ring and the
 // producers only write the outputs of groups without sources.
 template <int MODE, bool JOINT, bool F16, int TS = 0>
-__global__ void __launch_bounds__(kThreadsOf<F16, TS>, 1) tc_leaf_kernel(const __grid_constant__ TcJoint J, int *err) {
-    constexpr int kProdWarps = kProdWarpsOf<F16, TS>, kMmaWarp = kProdWarps, kLoadWarp = kProdWarps + 1;
-    constexpr int kThreads = kThreadsOf<F16, TS>;
+__global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_constant__ TcJoint J, int *err) {
     static_assert(!F16 || MODE == 0, "FP16 operands in the leaf pass only");
     static_assert(TS == 0 || (MODE == 0 && F16 && !JOINT), "kernel-tile store: FP16 leaf pass of one grid");
     constexpr int SK = F16 ? kStageKF16 : kStageK;   // sources per stage
@@ -661,8 +703,8 @@ __global__ void __launch_bounds__(kThreadsOf<F16, TS>, 1) tc_leaf_kernel(const _
             const int ni = G.ie - G.ib;
             const int rb = (G.nt + 31) >> 5;
             const int wb = rb >= 3 ? (warp & 3) : rb == 2 ? (warp & 1) : 0;            // row block
-            const int kfirst = rb >= 3 ? (warp >> 2) : rb == 2 ? (warp >> 1) : warp;    // first k-step
-            const int kstride = rb >= 3 ? kProdWarps / 4 : rb == 2 ? kProdWarps / 2 : kProdWarps;
+            const int kfirst8 = rb >= 3 ? (warp >> 2) : rb == 2 ? (warp >> 1) : warp;    // first k-step
+            const int kstride8 = rb >= 3 ? 2 : rb == 2 ? 4 : 8;
             const int row = 32 * wb + lane;
             const bool active = 32 * wb < G.nt, rvalid = row < G.nt;
             // canonical offsets (floats) of this thread's rows in a kernel tile:
@@ -724,31 +766,47 @@ __global__ void __launch_bounds__(kThreadsOf<F16, TS>, 1) tc_leaf_kernel(const _
             if constexpr (F16) {
                 // FP16: an item is one stage, and its record comes to shared
                 // memory with its weights: the loop costs a warp about as much
-                // per stage as a task does, so it holds nothing else
+                // per stage as a task does, so it holds nothing else.  The
+                // group's point and proxy items (all before its DOWN items) are
+                // dealt to two teams of four warps, stage by stage: a team's
+                // warps take twice the tasks of every other stage, and pay
+                // for half the stages.  DOWN items are every warp's.  A
+                // team's warp counts for two arrivals.
+                const int team = warp >> 2, tw = warp & 3;
+                const int ndown = G.ndown;   // DOWN items, at the list's end
 #pragma unroll 1
                 for (int k = 0; k < ni; ++k, ++st) {
-                    const uint32_t slot = st % KS, kpar = ((st / KS) - 1) & 1, jb = st % WS;
-                    bool slot_free = st < (uint32_t)KS;
+                    const bool down = k >= ni - ndown;
                     // an item the kernel-tile store holds (one in tile_every)
                     const bool stored = (TS == 1 || TS == 3) && k % a.tile_every == a.tile_every - 1;
+                    if (!down && (st & 1) != (uint32_t)team) {
+                        if (stored) gtile += (size_t)4 * ((((a.items[G.ib + k].cnt + 7) >> 3) + 1) >> 1) * cb;
+                        continue;
+                    }
+                    const uint32_t arrivals = down ? 1 : 2;
+                    const uint32_t slot = st % KS, kpar = ((st / KS) - 1) & 1, jb = st % WS;
+                    bool slot_free = st < (uint32_t)KS;
                     wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err);
                     const float4 rec = sm.rec[jb];
                     const int flags = __float_as_int(rec.w), nks = flags & kRecUnits;
                     if (TS == 3 && stored) {
-                        // replay: warp 0 copies the stage's chunks (MMA step q / 4, hi / lo,
-                        // east / north) into the ring slot once the MMAs that last read it
-                        // are done; its arrival carries the bytes
+                        // replay: the stage's first warp copies its chunks (MMA step
+                        // q / 4, hi / lo, east / north) into the ring slot once the MMAs
+                        // that last read it are done; its arrival carries the bytes
                         const int nq = 4 * ((nks + 1) >> 1);
                         if (!slot_free) wait_bounded(&sm.kempty[slot], kpar, abort, err);
-                        if (warp == 0) {
-                            if (lane == 0) dev::mbar_expect_tx(&sm.kfull[slot], (uint32_t)(nq * cb));
+                        if (down ? warp == 0 : tw == 0) {
+                            if (lane == 0) {
+                                dev::mbar_expect_tx(&sm.kfull[slot], (uint32_t)(nq * cb));
+                                if (!down) mbar_arrive(&sm.kfull[slot]);
+                            }
                             __syncwarp();
                             if (lane < nq && !*abort)
                                 dev::bulk_g2s_hint(
                                     reinterpret_cast<unsigned char *>(sm.Kt(slot, lane >> 2, (lane >> 1) & 1)) + (lane & 1) * cb,
                                     gtile + (size_t)lane * cb, (uint32_t)cb, &sm.kfull[slot], dev::l2_evict_first());
                         } else if (lane == 0) {
-                            mbar_arrive(&sm.kfull[slot]);
+                            mbar_arrive_n(&sm.kfull[slot], arrivals);
                         }
                         __syncwarp();
                         gtile += (size_t)nq * cb;
@@ -811,7 +869,10 @@ __global__ void __launch_bounds__(kThreadsOf<F16, TS>, 1) tc_leaf_kernel(const _
                         if (!slot_free) wait_bounded(&sm.kempty[slot], kpar, abort, err);
                         slot_free = true;
                     };
-                    int kk = active ? kfirst : nks + 1;
+                    // units: a team's warp w takes row block w (w % 2, 0), units i (w / 2
+                    // + 2i, w + 4i) of a group of 3-4 (2, 1) row blocks
+                    const int kstride = down ? kstride8 : rb >= 3 ? 1 : rb == 2 ? 2 : 4;
+                    int kk = !active ? nks + 1 : down ? kfirst8 : rb >= 3 ? 0 : rb == 2 ? tw >> 1 : tw;
                     if (!(flags & (kRecDown | kRecSelf))) {
 #pragma unroll 1
                         for (; kk + kstride < nks; kk += 2 * kstride) {
@@ -897,7 +958,7 @@ __global__ void __launch_bounds__(kThreadsOf<F16, TS>, 1) tc_leaf_kernel(const _
                     claim();
                     dev::fence_proxy_async();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&sm.kfull[slot]);
+                    if (lane == 0) mbar_arrive_n(&sm.kfull[slot], arrivals);
                     if (TS == 1 && stored) gtile += (size_t)4 * ((nks + 1) >> 1) * cb;
                 }
                 continue;
@@ -937,7 +998,7 @@ __global__ void __launch_bounds__(kThreadsOf<F16, TS>, 1) tc_leaf_kernel(const _
                     bool slot_free = st < (uint32_t)KS;
                     // the stage's upward factors (MODE 2) or source
                     // coordinates (point and proxy sources) are in aux
-                    if ((MODE == 2 || kind != 2) && active && kfirst < nks)
+                    if ((MODE == 2 || kind != 2) && active && kfirst8 < nks)
                         wait_bounded(&sm.wfull[st % WS], (st / WS) & 1, abort, err);
                     const float4 *crd = reinterpret_cast<const float4 *>(sm.aux[st % WS]);
                     // one task: the kernel-tile values of k-step kk for this
@@ -1064,9 +1125,9 @@ __global__ void __launch_bounds__(kThreadsOf<F16, TS>, 1) tc_leaf_kernel(const _
                         // nothing from it and keeps its registers.
                         constexpr int kPair = MODE == 1 ? 2 : 1;
 #pragma unroll 1
-                        for (int kk = kfirst; active && kk < nks; kk += kPair * kstride) {
+                        for (int kk = kfirst8; active && kk < nks; kk += kPair * kstride8) {
                             float ve[8], vn[8], vz[8], ve2[8], vn2[8], vz2[8];
-                            const int k2 = kk + kstride;
+                            const int k2 = kk + kstride8;
                             const bool two = kPair == 2 && k2 < nks;
                             values(kk, ve, vn, vz);
                             if (kPair == 2) values(two ? k2 : kk, ve2, vn2, vz2);
@@ -1119,9 +1180,12 @@ __global__ void __launch_bounds__(kThreadsOf<F16, TS>, 1) tc_leaf_kernel(const _
                 for (int j = 0; j < nst; ++j, ++st) {
                     const uint32_t slot = st % KS, jb = st % WS;
                     // replay: the stage's one barrier covers its weight and kernel tiles
+                    // (polled together: the one's latency hides the other's)
                     bool ok = true;
-                    if (TS != 2) ok = wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err);
-                    ok = wait_bounded(&sm.kfull[slot], (st / KS) & 1, abort, err) && ok;
+                    const bool wf = TS == 2 || dev::mbar_try_wait(&sm.wfull[jb], (st / WS) & 1);
+                    const bool kf = dev::mbar_try_wait(&sm.kfull[slot], (st / KS) & 1);
+                    if (!kf) ok = wait_bounded(&sm.kfull[slot], (st / KS) & 1, abort, err);
+                    if (!wf) ok = wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err) && ok;
                     // a new chain overwrites the accumulator, whose last chain
                     // (cc - 1) the fold warps must have read
                     if (!chain_open && cc >= 1) ok = wait_bounded(&sm.accfree, (cc - 1) & 1, abort, err) && ok;
@@ -1199,6 +1263,48 @@ __global__ void __launch_bounds__(kThreadsOf<F16, TS>, 1) tc_leaf_kernel(const _
             // rows, rounded up to 16 rows of 32 bytes)
             const unsigned char *tsrc = TS == 2 ? a.ktile + a.ktile_off[gi - J.beg[gk]] : nullptr;
             const uint32_t cb = (uint32_t)((G.nt + 15) & ~15) * 32u;
+            if constexpr (F16 && TS != 2) {
+                // FP16 computing launches: an item is one stage.  Lane l holds item
+                // k0 + l of the window: it writes the item's record itself, and the
+                // copies need two of its numbers only.  (The whole record by
+                // shuffles, twice, and an L2 prefetch of the next item's tiles, made
+                // this warp the slowest of a small group's stage: 1,240 cycles.)
+#pragma unroll 1
+                for (int k = G.ib; k < G.ie; ++k, ++st) {
+                    w.seek(k, lane);
+                    const int l = k - w.k0;
+                    const uint32_t jb = st % WS, ub = st / WS;
+                    const TcItem &it = w.cur;
+                    const int units = (it.cnt + 7) >> 3;
+                    const bool self = (it.kind & 3) == 0 && it.off < G.tgt + G.nt && G.tgt < it.off + it.cnt;
+                    const int flags = units | (it.kind & 3) << 4 | ((it.kind & kTcFlush) ? kRecFlush : 0) | (self ? kRecSelf : 0);
+                    const int kb = __shfl_sync(0xffffffffu, it.kb, l), fl = __shfl_sync(0xffffffffu, flags, l);
+                    bool ok = true;
+                    if (ub > 0) ok = wait_bounded(&sm.wempty[jb], (ub - 1) & 1, abort, err);
+                    if (lane == l) {
+                        // before the arrival that its readers wait for
+                        sm.rec[jb] = make_float4(it.dx, it.dy, it.dz, __int_as_float(flags));
+                        sm.rec2[jb] = make_int2(it.off, it.row0);
+                    }
+                    ok = __all_sync(0xffffffffu, ok);
+                    __syncwarp();
+                    if (elect_one()) {
+                        // whole 16-source MMA steps (the store has a spare unit at its
+                        // end), and the point and proxy sources' coordinates (24 floats
+                        // per unit; DOWN rows need none)
+                        const uint32_t nks = fl & kRecUnits, wbytes = ((nks + 1) & ~1u) * kW16UnitBytes;
+                        const uint32_t lbytes = (fl & kRecDown) ? 0u : nks * 96u;
+                        dev::mbar_expect_tx(&sm.wfull[jb], wbytes + lbytes);
+                        if (ok) {
+                            if (lbytes) dev::bulk_g2s(sm.aux[jb], a.sxyz + (size_t)kb * 24, lbytes, &sm.wfull[jb]);
+                            dev::bulk_g2s(sm.Wt(jb), static_cast<const char *>(a.bstore16) + (size_t)kb * kW16UnitBytes, wbytes,
+                                          &sm.wfull[jb]);
+                        }
+                    }
+                    __syncwarp();
+                }
+                continue;
+            }
             for (int k = G.ib; k < G.ie; ++k) {
                 const TcItem it = w.get(k, lane);
                 if (k + 1 < G.ie) {
@@ -1272,14 +1378,6 @@ __global__ void __launch_bounds__(kThreadsOf<F16, TS>, 1) tc_leaf_kernel(const _
                             // k-step; DOWN rows need none)
                             const uint32_t lbytes = MODE == 2 ? (uint32_t)nks * 64 * n
                                                     : (it.kind & 3) != 2 ? (uint32_t)nks * 96u : 0u;
-                            if constexpr (F16) {
-                                // written before the arrival that its readers wait for
-                                const bool self = (it.kind & 3) == 0 && it.off < G.tgt + G.nt && G.tgt < it.off + it.cnt;
-                                const int flags = nks | (it.kind & 3) << 4 | ((it.kind & kTcFlush) ? kRecFlush : 0) |
-                                                  (self ? kRecSelf : 0);
-                                sm.rec[jb] = make_float4(it.dx, it.dy, it.dz, __int_as_float(flags));
-                                sm.rec2[jb] = make_int2(it.off, it.row0);
-                            }
                             dev::mbar_expect_tx(&sm.wfull[jb], wbytes + lbytes);
                             if (!*abort) {
                                 if (lbytes)
@@ -1602,7 +1700,7 @@ static void launch_tc(const TcJoint &J, int nsm, int cta_groups, int *err, cudaS
     const int per = cta_groups > 0 ? cta_groups : 1;
     int grid = (total + per - 1) / per;
     if (grid < nsm) grid = total < nsm ? total : nsm;
-    tc_leaf_kernel<MODE, JOINT, F16, TS><<<grid, kThreadsOf<F16, TS>, smem, st>>>(J, err);
+    tc_leaf_kernel<MODE, JOINT, F16, TS><<<grid, kThreads, smem, st>>>(J, err);
 }
 
 template <int MODE, bool F16 = false, int TS = 0>
