@@ -80,6 +80,7 @@ struct GridImpl {
     float *bstore = nullptr;          // split weight store of the tcgen05 leaf pass
     void *bstore16 = nullptr;         // FP16 leaf pass: its FP16 hi/lo weight store (one spare unit at the end)
     float *tscale = nullptr, *tinv = nullptr;   // FP16 leaf pass: per target, its kernel values' scale
+    float *dbasis = nullptr;          // FP16 leaf pass, tree passes: per target, its BLI bases in its DOWN slot
     unsigned *fmax = nullptr;         // FP16 leaf pass: the block's field maxima (source weights, potentials)
     unsigned char *ktile = nullptr;   // FP16 leaf pass with sal_tune.tile_store: its kernel tiles
     int64_t *ktile_off = nullptr;     // per leaf group, the byte offset of its tiles
@@ -430,6 +431,7 @@ static int64_t mixed_bytes_needed(const GridImpl &g, int FT) {
              (int64_t)sizeof(float4) * (n + (int64_t)g.nsrc * P) + (int64_t)sizeof(double2) * n +
              4 * pl.tc_src_ksteps * 24;
         if (pl.tc_opt.f16) b += ((int64_t)pl.bsrc.size() / 8 + 1) * 2048 + 128 * 4 + 2 * 4 * n;
+        if (pl.tc_opt.f16 && pl.tc_opt.tree_passes) b += 4 * n * 2 * (pl.d + 1);
         if (pl.tc_opt.f16 && pl.tc_opt.tile_store) b += pl.tc_tile_off.back() + vb(pl.tc_tile_off);
     }
     return b;
@@ -662,6 +664,7 @@ static int ensure_mixed(GridImpl &g, int FT) {
             if (!rc) rc = malloc_mix(g, &g.fmax, (size_t)128);
             if (!rc) rc = malloc_mix(g, &g.tscale, n);
             if (!rc) rc = malloc_mix(g, &g.tinv, n);
+            if (!rc && pl.tc_opt.tree_passes) rc = malloc_mix(g, &g.dbasis, n * 2 * (pl.d + 1));
             if (!rc) {
                 // zeros in every row no pass writes, so the per-field maxima can
                 // read the weight and potential rows whole
@@ -670,6 +673,7 @@ static int ensure_mixed(GridImpl &g, int FT) {
                 CK(cudaMemsetAsync(g.bstore16, 0, units * 2048, g.stream));
                 mix::TcArgs t = leaf_args(g, nullptr, nullptr, 0, 0, 0);
                 mix::launch_target_scales(t, g.tscale, g.tinv, g.stream);
+                if (g.dbasis) mix::launch_down_basis(t, g.dbasis, g.stream);
                 CK(cudaStreamSynchronize(g.stream));
                 CK(cudaGetLastError());
             }
@@ -718,6 +722,7 @@ static mix::TcArgs leaf_args(GridImpl &g, double *ox, double *oy, int64_t ld_out
         t.tscale = g.tscale;
         t.tinv = g.tinv;
         t.fmax = g.fmax;
+        t.dbasis = g.dbasis;
         t.ktile = g.ktile;
         t.ktile_off = g.ktile_off;
         t.tile_every = g.plan.tc_opt.tile_store > 1 ? g.plan.tc_opt.tile_store : 1;

@@ -73,6 +73,7 @@ struct TcArgs {
     const void *bstore16;
     const float *tscale, *tinv;
     const unsigned *fmax;
+    const float *dbasis;      // FP16 leaf pass, tree passes: per pool position 2(d+1) BLI bases over its DOWN slot's nodes
     // FP16 leaf pass with a kernel-tile store: the store, per group the byte
     // offset of its tiles (ngroups + 1 entries), and which items it holds:
     // items every-1, 2 every-1, ... of each group (all with every = 1)
@@ -96,6 +97,7 @@ void launch_tc_leaf(const TcArgs &a, int nsm, int cta_groups, int *err, cudaStre
 void launch_tc_leaf_joint(const TcArgs *grids, int ngrids, int nsm, int cta_groups, int *err, cudaStream_t st);
 void launch_tc_proxy(const TcArgs &a, int nsm, int cta_groups, int *err, cudaStream_t st);
 void launch_tc_upward(const TcArgs &a, int nsm, int cta_groups, int *err, cudaStream_t st);
+void launch_down_basis(const TcArgs &a, float *out, cudaStream_t st);
 void launch_basis_store(const int32_t *bas, int64_t nbk, const double2 *xieta, const double *src_nodes, int n,
                         float *basis, cudaStream_t st);
 size_t tc_smem_bytes();

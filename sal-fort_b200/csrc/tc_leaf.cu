@@ -150,6 +150,7 @@ struct TcSmem {
     int kmap[kReplay ? 1 : kKmap];
     // FP16 computing launches, per weight stage, its item as the loader saw it:
     // (dx, dy, dz, flags: kRec*) and (off, row0)
+    alignas(16) float cs[kTcRows];                                // folds: the group's column scales (DOWN chains)
     float4 rec[kReplay ? 1 : kWStages];
     int2 rec2[kReplay ? 1 : kWStages];
     uint32_t toff[KS], tlen[KS], woff[KS], wlen[KS];             // replay: each stage slot's ranges in the rings
@@ -451,24 +452,28 @@ __device__ __forceinline__ int fold_per(bool end, int nt, int half) {
 // group: 4,300 -> FOLDNEW cycles a chain).
 template <int MODE>
 __device__ __noinline__ void fold_chain(uint32_t td, int lane, bool end, bool first, int tgt, int nt, bool scaled,
-                                        float fsc, bool down, const float *__restrict__ tscale, int half, int part_i,
-                                        int nparts) {
-    // per target slot 32k + lane: its scale (DOWN chains)
-    float csd[4] = {1.f, 1.f, 1.f, 1.f};
-    if (MODE == 0 && scaled && down)
+                                        float fsc, bool down, const float *__restrict__ tscale, float *cs, int half,
+                                        int part_i, int nparts) {
+    // DOWN chains: the targets' scales, which every fold warp writes to shared
+    // memory for itself (the same values; the next such chain's are written
+    // after every warp has handed this one's accumulator back)
+    if (MODE == 0 && scaled && down) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) csd[k] = 32 * k + lane < nt ? tscale[tgt + 32 * k + lane] : 1.f;
+        for (int k = 0; k < 4; ++k) cs[32 * k + lane] = 32 * k + lane < nt ? tscale[tgt + 32 * k + lane] : 1.f;
+        __syncwarp();
+    }
     const int per = fold_per<MODE>(end, nt, half);
     const int ncol = 16 * (MODE == 2 ? per : 2 * per);   // component c's chunk j is columns half c + 16 j, half = 16 per
     const float2 f2v = f2(scaled && !down ? fsc : 1.f);
     // DOWN chains: the field's factor, then the column's
     auto unscale = [&](float *x, int c) {
+        const float2 *sc = reinterpret_cast<const float2 *>(cs + (c >= half ? c - half : c));
 #pragma unroll
-        for (int m = 0; m < 16; ++m) x[m] *= fsc;
-        const int b = c >= half ? c - half : c, k = b >> 5;
-        const float src = k == 0 ? csd[0] : k == 1 ? csd[1] : k == 2 ? csd[2] : csd[3];
-#pragma unroll
-        for (int m = 0; m < 16; ++m) x[m] *= __shfl_sync(0xffffffffu, src, (b & 31) + m);
+        for (int m = 0; m < 16; m += 2) {
+            const float2 v = __fmul2_rn(__fmul2_rn(make_float2(x[m], x[m + 1]), f2(fsc)), sc[m >> 1]);
+            x[m] = v.x;
+            x[m + 1] = v.y;
+        }
     };
     auto add = [&](float *x, const float *r) {   // 2 columns
         float2 v = make_float2(x[0], x[1]);
@@ -892,10 +897,17 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                             producers_sync(32 * kProdWarps);
                             const int brow = tid & (kTcRows - 1);
                             if (brow < G.nt) {
-                                const double2 e = a.xieta[G.tgt + brow];
-                                const double *nodes = a.tgt_nodes + (size_t)slot_id * 2 * n;
-                                if (tid < kTcRows) down_basis(e.x, nodes, n, sm.fx[brow]);
-                                else down_basis(e.y, nodes + n, n, sm.fe[brow]);
+                                float *o = tid < kTcRows ? sm.fx[brow] : sm.fe[brow];
+                                if (a.dbasis) {
+                                    // tree passes: a target has one slot, its bases are in the
+                                    // plan's store
+                                    const float *src = a.dbasis + (size_t)(G.tgt + brow) * 2 * n + (tid < kTcRows ? 0 : n);
+                                    for (int i = 0; i < n; ++i) o[i] = src[i];
+                                } else {
+                                    const double2 e = a.xieta[G.tgt + brow];
+                                    const double *nodes = a.tgt_nodes + (size_t)slot_id * 2 * n;
+                                    down_basis(tid < kTcRows ? e.x : e.y, tid < kTcRows ? nodes : nodes + n, n, o);
+                                }
                             }
                             producers_sync(32 * kProdWarps);
                         }
@@ -909,23 +921,35 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                             for (int c = 0; c < 4; ++c) o[0][0][c] = o[0][1][c] = o[0][2][c] = o[0][3][c] = 0u;
                         } else if (flags & kRecDown) {
                             // BLI basis of the target x its unit vector's component of the
-                            // Cartesian row
-                            const int *km0 = sm.kmap + sm.rec2[jb].y + 8 * kk;
-                            const float *fxr = sm.fx[row], *fer = sm.fe[row];
+                            // Cartesian row: the unit's rows r0 .. r0 + 7 are components
+                            // r % 3 of proxies r / 3, four proxies at most (rows past
+                            // 3 P meet zero weights)
+                            const int r0 = sm.rec2[jb].y + 8 * kk, p0 = r0 / 3, ph = r0 - 3 * p0;
+                            float bv[4];
 #pragma unroll
-                            for (int c2 = 0; c2 < 4; ++c2) {
-                                float e[2], nn[2];
-#pragma unroll
-                                for (int c = 0; c < 2; ++c) {
-                                    const int km = km0[2 * c2 + c];
-                                    const float b = fxr[km & 255] * fer[(km >> 8) & 255];
-                                    const int comp = km >> 16;
-                                    e[c] = comp == 2 ? 0.f : b * (comp == 0 ? el0 : el1);
-                                    nn[c] = b * (comp == 0 ? ep0 : (comp == 1 ? ep1 : ep2));
-                                }
-                                split_f16x2(e[0], e[1], o[0][0][c2], o[0][1][c2]);
-                                split_f16x2(nn[0], nn[1], o[0][2][c2], o[0][3][c2]);
+                            for (int q = 0; q < 4; ++q) {
+                                const int km = sm.kmap[3 * (p0 + q < P ? p0 + q : 0)];
+                                bv[q] = sm.fx[row][km & 255] * sm.fe[row][(km >> 8) & 255];
                             }
+                            auto fill = [&]<int PH>() {
+#pragma unroll
+                                for (int c2 = 0; c2 < 4; ++c2) {
+                                    float e[2], nn[2];
+#pragma unroll
+                                    for (int c = 0; c < 2; ++c) {
+                                        constexpr int kThree = 3;
+                                        const int x = PH + 2 * c2 + c, comp = x % kThree;
+                                        const float b = bv[x / kThree];
+                                        e[c] = comp == 2 ? 0.f : b * (comp == 0 ? el0 : el1);
+                                        nn[c] = b * (comp == 0 ? ep0 : (comp == 1 ? ep1 : ep2));
+                                    }
+                                    split_f16x2(e[0], e[1], o[0][0][c2], o[0][1][c2]);
+                                    split_f16x2(nn[0], nn[1], o[0][2][c2], o[0][3][c2]);
+                                }
+                            };
+                            if (ph == 0) fill.template operator()<0>();
+                            else if (ph == 1) fill.template operator()<1>();
+                            else fill.template operator()<2>();
                         } else {
                             pairs16(kk, 0, o);
                         }
@@ -1440,8 +1464,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                 const float fsc = F16 ? 1.f / f16_scale(__uint_as_float(a.fmax[(down_chain ? kF : 0) + 16 * q + (lane & 15)]))
                                       : 1.f;
                 const bool end = k == G.ie - 1;
-                fold_chain<MODE>(tq, lane, end, first, G.tgt, G.nt, F16, fsc, down_chain, a.tscale, half, part_i,
-                                 nparts);
+                fold_chain<MODE>(tq, lane, end, first, G.tgt, G.nt, F16, fsc, down_chain, a.tscale, sm.cs, half,
+                                 part_i, nparts);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sm.accfree);
@@ -1610,6 +1634,20 @@ __global__ void target_scales_kernel(const TcArgs a, float *__restrict__ tscale,
     tinv[G.tgt + row] = 1.f / sc;
 }
 
+// Tree passes: per target of a leaf group, the BLI bases (xi, then eta; n
+// floats each) over the nodes of the group's one DOWN slot, as down_basis gives
+// them.  One block per leaf group, thread t its target t.  Once per plan.
+__global__ void down_basis_store_kernel(const TcArgs a, float *__restrict__ out) {
+    const MixGroup G = a.groups[blockIdx.x];
+    const int row = threadIdx.x, n = a.d + 1;
+    if (row >= G.nt || G.ndown == 0) return;
+    const double *nodes = a.tgt_nodes + (size_t)a.items[G.ie - 1].off * 2 * n;
+    const double2 e = a.xieta[G.tgt + row];
+    float *o = out + (size_t)(G.tgt + row) * 2 * n;
+    down_basis(e.x, nodes, n, o);
+    down_basis(e.y, nodes + n, n, o + n);
+}
+
 // Per pool row, the FP32 coordinates relative to the centre of the row's own
 // panel (a leaf for points, the slot panel for proxies).  One block per range.
 __global__ void source_local_kernel(const double4 *__restrict__ pool, const int2 *__restrict__ ranges,
@@ -1771,6 +1809,10 @@ void launch_split_store16(const int32_t *bsrc, int64_t nunits, const float *wF, 
 
 void launch_target_scales(const TcArgs &a, float *tscale, float *tinv, cudaStream_t st) {
     if (a.ngroups > 0) target_scales_kernel<<<a.ngroups, kTcRows, 0, st>>>(a, tscale, tinv);
+}
+
+void launch_down_basis(const TcArgs &a, float *out, cudaStream_t st) {
+    if (a.ngroups > 0) down_basis_store_kernel<<<a.ngroups, kTcRows, 0, st>>>(a, out);
 }
 
 void launch_source_local(const double4 *pool, const int2 *ranges, const double4 *centres, int nranges, float4 *sloc,
