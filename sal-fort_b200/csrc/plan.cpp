@@ -27,7 +27,6 @@
 
 namespace sal {
 
-static constexpr int64_t kL2StoreBytes = 96ll << 20;   // a weight store that stays in the 126 MB L2
 static constexpr int kUpChunk = 4096;          // points per upward unit
 static constexpr double kProxyUnitPairs = 81.0 * 8192.0;  // pair budget of one proxy work unit (FP64 pass)
 
@@ -992,17 +991,14 @@ bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *e
         }
     }
     if (!tree) pl->tc_macs_down = pl->macs_down;
-    // Launch order: by cost, so that the CTAs that start last are short ones,
-    // while the weight store fits L2 (leaf pass at 40,962 cells, 541 groups on
-    // 148 SMs: 706 -> 582 us; 163,842: 2,288 -> 2,191).  Above that pool order,
-    // whose neighbours share weights in L2: by cost the pass at 2,313,486 cells
-    // takes 28.1 ms for 26.7, and its last wave is 1/180 of it.  A stage of a
-    // full group costs 2,900 cycles, one of a single row block 1,200.
-    if ((int64_t)pl->bsrc.size() * 256 <= kL2StoreBytes) {
-        auto cost = [](const MixGroup &m) { return (m.ie - m.ib) * (0.6 + 0.55 * ((m.nt + 31) / 32)); };
-        std::stable_sort(pl->tc_leaf_groups.begin(), pl->tc_leaf_groups.end(),
-                         [&](const MixGroup &x, const MixGroup &y) { return cost(x) > cost(y); });
-    }
+    // Launch order: groups of more row blocks first, so that the CTAs that start
+    // last are short ones (a full group's stage costs 2,900 cycles, one of a
+    // single row block 1,200); among equals pool order, whose neighbours share
+    // weights in L2.  Leaf pass at 40,962 cells (541 groups on 148 SMs) 706 ->
+    // 587 us, 163,842 cells 2,288 -> 2,192, 2,313,486 cells 26.7 ms either way.
+    // (By stages x cost a stage: 581 us, 2,180 us, but 28.1 ms.)
+    std::stable_sort(pl->tc_leaf_groups.begin(), pl->tc_leaf_groups.end(),
+                     [](const MixGroup &x, const MixGroup &y) { return (x.nt + 31) / 32 > (y.nt + 31) / 32; });
     plan_tile_offsets(pl, opt.tile_store > 1 ? opt.tile_store : 1);
 
     // ---- proxy pass: each target slot's items cut into units of at most
