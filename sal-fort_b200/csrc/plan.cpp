@@ -961,6 +961,13 @@ bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *e
         return true;
     };
 
+    // stages of kTcStage K columns of items [ib, ie)
+    auto stages = [](const std::vector<TcItem> &items, int32_t ib, int32_t ie) {
+        int32_t k = 0;
+        for (int32_t i = ib; i < ie; ++i) k += (items[i].cnt + kTcStage - 1) / kTcStage;
+        return k;
+    };
+
     // ---- leaf pass: groups of at most kTcRows targets in pool order
     std::vector<int32_t> gord(pl->leaf_groups.size());
     std::iota(gord.begin(), gord.end(), 0);
@@ -982,11 +989,12 @@ bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *e
         // DOWN items end the list (the work lists hold them after all others)
         int32_t ndown = 0;
         while (ndown < ie - ib && (pl->tc_items[ie - 1 - ndown].kind & 3) == 2) ++ndown;
+        const int32_t nst = stages(pl->tc_items, ib, ie), nstd = stages(pl->tc_items, ie - ndown, ie);
         for (int32_t r = 0; r < g.nt; r += kTcRows) {
             MixGroup m{};
             m.tgt = g.tgt + r; m.nt = std::min(kTcRows, g.nt - r); m.ib = ib; m.ie = ie; m.out = g.out;
             m.cx = t.cx[kt]; m.cy = t.cy[kt]; m.cz = t.cz[kt];
-            m.ndown = ndown;
+            m.ndown = ndown; m.nst = nst; m.nstd = nstd;
             pl->tc_leaf_groups.push_back(m);
         }
     }
@@ -1035,9 +1043,10 @@ bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *e
             const int32_t uo = ord[x];
             const U &u = units[uo];
             const int kt = pl->tgt_slot_panel[u.slot];
-            const int32_t ib = range[x].first, ie = range[x].second;
+            const int32_t ib = range[x].first, ie = range[x].second, nst = stages(pl->tc_proxy_items, ib, ie);
             for (int32_t r = 0; r < P; r += kTcProxyRows) {
                 MixGroup m{};
+                m.nst = nst;
                 m.tgt = u.slot; m.nt = std::min(kTcProxyRows, P - r); m.ib = ib; m.ie = ie; m.out = uo; m.row0 = r;
                 m.cx = t.cx[kt]; m.cy = t.cy[kt]; m.cz = t.cz[kt];
                 pl->tc_proxy_groups.push_back(m);
@@ -1070,8 +1079,10 @@ bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *e
                 ++nbk;
             }
         }
+        const int32_t nst = stages(pl->tc_up_items, ib, ie);
         for (int32_t r = 0; r < P; r += kTcRows) {
             MixGroup m{};
+            m.nst = nst;
             m.tgt = nodes_slot; m.nt = std::min(kTcRows, P - r); m.ib = ib; m.ie = ie; m.out = out; m.row0 = r;
             pl->tc_up_groups.push_back(m);
         }

@@ -111,9 +111,12 @@ struct UpUnit {          // upward-pass work unit
 // (four 16-row tensor-core tiles) with a local coordinate origin (cx, cy, cz)
 // near them.  row0: first target row of the group within its panel (proxy
 // groups) or 0.  ndown: DOWN items at the end of the list (tcgen05 leaf groups).
+// nst, nstd: the list's stages of kTcStage K columns, and its DOWN items' part of
+// them (tcgen05 groups).
 struct MixGroup {
-    int32_t tgt, nt, ib, ie, out, row0, ndown, pad1;
-    double cx, cy, cz, pad2;
+    int32_t tgt, nt, ib, ie, out, row0, ndown, nst;
+    double cx, cy, cz;
+    int32_t nstd, pad;
 };
 
 // Item of the tcgen05 leaf pass.  kind & 3 = 0 / 1: sources are pool rows
@@ -262,6 +265,7 @@ constexpr int kMixStage = 64;    // sources (or DOWN rows) staged per batched it
 constexpr int kMixRows = 64;     // targets per batched CTA
 constexpr int kTcRows = 128;     // targets per tcgen05 leaf group (the MMA's M)
 constexpr int kTcChunk = 64;     // sources (or DOWN rows) per tcgen05 item
+constexpr int kTcStage = 32;     // K columns of a TF32 stage
 constexpr int kTcProxyRows = 85;   // target proxies per tcgen05 proxy group: 3 x 85 <= 256
 constexpr int kMaxDegree = 14;   // a DOWN record (4(d+1)^2 + 2(d+1) doubles) fits one 8 KB stage
 constexpr int kMaxTreeDegree = 10;  // tree transfers of the batched form: their tiles fit shared memory up to here

@@ -37,7 +37,7 @@
 //               written once per solve by split_store_kernel) and the
 //               sources' coordinates (leaf and proxy passes) or BLI factors
 //               (upward pass), with bulk copies into a 4-deep ring, and
-//               prefetches the next item's tiles into L2.
+//               writes the stage's record (centre offset, flags) beside them.
 //   warps 10-13 fold finished accumulator chains into the running sums and
 //               write the outputs (warp w: tensor memory lanes 32(w%4)..+31).
 // FP16 leaf pass (sal_tune.f16): the same machine with kind::f16 MMAs, 16
@@ -86,7 +86,7 @@ constexpr int kProdWarps = 8;
 constexpr int kMmaWarp = kProdWarps, kLoadWarp = kProdWarps + 1;
 constexpr int kThreads = (kProdWarps + 2 + kFoldWarps) * 32;   // 448
 constexpr int kF = 64;                            // fields
-constexpr int kStageK = 32;                       // K columns per stage (four k-steps of 8)
+constexpr int kStageK = kTcStage;                 // K columns per stage (four k-steps of 8)
 constexpr int kStageKs = kStageK / 8;             // k-steps per stage
 constexpr int kKStages = 2;                       // kernel-tile ring
 constexpr int kWStages = 4;                       // weight / upward-factor ring
@@ -192,6 +192,13 @@ __device__ __forceinline__ float tf32_hi(float x) {
     uint32_t r;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
     return __uint_as_float(r);
+}
+
+// The same for kernel-tile values, in two integer instructions (the conversion
+// takes about four): half a unit of the last kept bit added to the magnitude, the
+// rest cut off.  (A NaN's hi may lose it; its lo = v - hi is NaN then.)
+__device__ __forceinline__ float tf32_hi_tile(float x) {
+    return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
 }
 
 // Hint: fetch a global range into L2 ahead of its bulk copy (16-byte
@@ -448,18 +455,20 @@ __device__ __forceinline__ int fold_per(bool end, int nt, int half) {
 // The MMA warp waits for the fold, so it is short: the chunks are contiguous
 // columns (16 i), taken 32 at a time; a kernel chain's factor is a power of
 // two, so factor and add are one packed fused multiply-add with the same bits;
-// and the next chain columns are on their way while a result is stored (full
-// group: 4,300 -> FOLDNEW cycles a chain).
+// and the next chain columns are on their way while a result is stored (16
+// columns at a time 4,300 cycles a chain of a full group and 1,750 of one row
+// block, so 4,000 and 1,100).
 template <int MODE>
-__device__ __noinline__ void fold_chain(uint32_t td, int lane, bool end, bool first, int tgt, int nt, bool scaled,
-                                        float fsc, bool down, const float *__restrict__ tscale, float *cs, int half,
-                                        int part_i, int nparts) {
+__device__ __noinline__ void fold_chain(uint32_t td, int lane, bool end, bool first, int nt, bool scaled, float fsc,
+                                        bool down, float4 tsc, float *cs, int half, int part_i, int nparts) {
     // DOWN chains: the targets' scales, which every fold warp writes to shared
     // memory for itself (the same values; the next such chain's are written
     // after every warp has handed this one's accumulator back)
     if (MODE == 0 && scaled && down) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) cs[32 * k + lane] = 32 * k + lane < nt ? tscale[tgt + 32 * k + lane] : 1.f;
+        cs[lane] = tsc.x;
+        cs[32 + lane] = tsc.y;
+        cs[64 + lane] = tsc.z;
+        cs[96 + lane] = tsc.w;
         __syncwarp();
     }
     const int per = fold_per<MODE>(end, nt, half);
@@ -627,7 +636,6 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
     static_assert(!F16 || MODE == 0, "FP16 operands in the leaf pass only");
     static_assert(TS == 0 || (MODE == 0 && F16 && !JOINT), "kernel-tile store: FP16 leaf pass of one grid");
     constexpr int SK = F16 ? kStageKF16 : kStageK;   // sources per stage
-    constexpr int SU = SK / 8;                        // store units (8 sources) per stage
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     constexpr int KS = TcSmem<TS>::KS, WS = TcSmem<TS>::WS;
     TcSmem<TS> &sm = *reinterpret_cast<TcSmem<TS> *>(smem_raw);
@@ -690,12 +698,13 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
         // ============================================================ producers
         // A stage's tasks are (row block of 32 targets, unit) pairs, one
         // 8-source unit of 32 rows each (a TF32 stage has 4 units, an FP16
-        // stage 8).  A stage costs the latency of the busiest warp's tasks,
-        // so the tasks of small groups (one or two row blocks: the second
-        // tile of a leaf with more than 128 points) are spread over all warps:
-        //   3-4 row blocks: warp w takes row block w % 4, units w / 4 + 2i
-        //   2 row blocks:   warp w takes row block w % 2, units w / 2 + 4i
-        //   1 row block:    warp w takes unit w (TF32: warps 4-7 only arrive)
+        // stage 8).  The stages are dealt to two teams of four warps in turn,
+        // and within a team (DOWN stages: over all eight warps w)
+        //   3-4 row blocks: warp w takes row block w % 4, all units
+        //                   (DOWN: units w / 4 + 2i)
+        //   2 row blocks:   row block w % 2, units w / 2 + 2i (w / 2 + 4i)
+        //   1 row block:    units w + 4i (unit w)
+        // so that a group of few row blocks uses every warp.
         // The source coordinates of a stage's k-steps (x[8] y[8] z[8] each,
         // relative to their panel's centre) arrive in shared memory with the
         // stage's weights: the loader warp copies them up to WS stages
@@ -712,14 +721,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             const int kstride8 = rb >= 3 ? 2 : rb == 2 ? 4 : 8;
             const int row = 32 * wb + lane;
             const bool active = 32 * wb < G.nt, rvalid = row < G.nt;
-            // canonical offsets (floats) of this thread's rows in a kernel tile:
-            // leaf east / north at rows t, half + t (half: the targets rounded
-            // up to 16); proxy x / y / z at 85c + r
+            // leaf: east / north of target t at rows t, half + t of a kernel tile
+            // (half: the targets rounded up to 16)
             const int half = (G.nt + 15) & ~15;
-            const int oe = canon(row, 0) >> 2;
-            const int on = canon(MODE == 0 ? half + row : kTcProxyRows + row, 0) >> 2;
-            const int oz = canon(MODE == 0 ? 0 : 2 * kTcProxyRows + row, 0) >> 2;
-            const bool row_in_tile = row < (MODE == 0 ? half : MODE == 1 ? kTcProxyRows : kTcRows);
+            const bool row_in_tile = row < half;
             // FP16 tiles: byte offset of the row's first K core matrix (8-row
             // groups 256 B apart, the two K halves 128 B apart)
             const int oe16 = (row >> 3) * 256 + (row & 7) * 16;
@@ -728,16 +733,12 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             float tl0 = 0.f, tl1 = 0.f, tl2 = 0.f, el0 = 0.f, el1 = 0.f, ep0 = 0.f, ep1 = 0.f, ep2 = 0.f;
             // FP16 leaf pass: this row's power-of-two scale of kernel values
             const float tsc = (F16 && rvalid) ? a.tscale[G.tgt + row] : 1.f;
-            // upward: this row's proxy p = row0 + row = up_i + up_j n
-            const int up_p = MODE == 2 ? G.row0 + (rvalid ? row : 0) : 0;
-            const int up_i = up_p % n, up_j = up_p / n;
-            if (MODE != 2 && rvalid) {
-                // leaf: the pool point; proxy: proxy row0 + row of target slot G.tgt
-                const double4 c = MODE == 0 ? a.tgt[G.tgt + row] : a.tgt[(size_t)G.tgt * P + G.row0 + row];
+            if (MODE == 0 && rvalid) {
+                const double4 c = a.tgt[G.tgt + row];
                 tl0 = (float)(c.x - G.cx);
                 tl1 = (float)(c.y - G.cy);
                 tl2 = (float)(c.z - G.cz);
-                if (MODE == 0 && (fabs(c.z - 1.0) > 1e-15) && (fabs(c.z + 1.0) > 1e-15)) {
+                if ((fabs(c.z - 1.0) > 1e-15) && (fabs(c.z + 1.0) > 1e-15)) {
                     const double omz = 1.0 - c.z * c.z, inv = 1.0 / sqrt(omz);
                     el0 = (float)(-c.y * inv);
                     el1 = (float)(c.x * inv);
@@ -791,9 +792,9 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     const uint32_t arrivals = down ? 1 : 2;
                     const uint32_t slot = st % KS, kpar = ((st / KS) - 1) & 1, jb = st % WS;
                     bool slot_free = st < (uint32_t)KS;
-                    wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err);
+                    const bool ok = wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err);
                     const float4 rec = sm.rec[jb];
-                    const int flags = __float_as_int(rec.w), nks = flags & kRecUnits;
+                    const int flags = ok ? __float_as_int(rec.w) : 0, nks = flags & kRecUnits;
                     if (TS == 3 && stored) {
                         // replay: the stage's first warp copies its chunks (MMA step
                         // q / 4, hi / lo, east / north) into the ring slot once the MMAs
@@ -887,8 +888,12 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                             store16(kk, o[0]);
                             store16(kk + kstride, o[1]);
                         }
-                    } else if (flags & kRecDown) {
-                        const int slot_id = sm.rec2[jb].x;
+                    }
+                    if (down) {
+                        // the tree passes have one slot a group (every warp must come to
+                        // the same barriers, so not by the record, which a time-out may
+                        // have left unread)
+                        const int slot_id = a.dbasis ? 0 : a.items[G.ib + k].off;
                         if (slot_id != cur_slot) {
                             // BLI bases of every target row in the new slot: thread
                             // t < 128 the xi basis of target t, thread 128 + t its
@@ -987,192 +992,222 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                 }
                 continue;
             }
-            // item records are read one item ahead, so their latency hides
-            // behind the current item's stages
-            TcItem nxt = a.items[G.ib];
-            for (int k = 0; k < ni; ++k) {
-                const TcItem it = nxt;
-                if (k + 1 < ni) nxt = a.items[G.ib + k + 1];
-                const int kind = it.kind & 3;
-                const int nst = (it.cnt + SK - 1) / SK;
-                if (MODE == 0 && kind == 2 && it.off != cur_slot) {
-                    // BLI bases of every target row in the new slot: thread
-                    // t < 128 the xi basis of target t, thread 128 + t its
-                    // eta basis
-                    cur_slot = it.off;
-                    producers_sync(32 * kProdWarps);
-                    const int brow = tid & (kTcRows - 1);
-                    if (brow < G.nt && tid < 2 * kTcRows) {
-                        const double2 e = a.xieta[G.tgt + brow];
-                        const double *nodes = a.tgt_nodes + (size_t)it.off * 2 * n;
-                        if (tid < kTcRows) down_basis(e.x, nodes, n, sm.fx[brow]);
-                        else down_basis(e.y, nodes + n, n, sm.fe[brow]);
-                    }
-                    producers_sync(32 * kProdWarps);
-                }
-                const float2 tx2 = f2(tl0 - it.dx), ty2 = f2(tl1 - it.dy), tz2 = f2(tl2 - it.dz);
-                // only the item whose sources are the group's own points holds
-                // self pairs (one test per item, the same for every thread)
-                const bool self_item = MODE == 0 && kind == 0 && it.off < G.tgt + G.nt && G.tgt < it.off + it.cnt;
-                for (int j = 0; j < nst; ++j, ++st) {
-                    const uint32_t slot = st % KS, kpar = ((st / KS) - 1) & 1;
-                    const int nks = (min(SK, it.cnt - SK * j) + 7) >> 3;   // k-steps of this stage
-                    // the MMAs that last read this slot must be done before
-                    // the first store into it
-                    bool slot_free = st < (uint32_t)KS;
-                    // the stage's upward factors (MODE 2) or source
-                    // coordinates (point and proxy sources) are in aux
-                    if ((MODE == 2 || kind != 2) && active && kfirst8 < nks)
-                        wait_bounded(&sm.wfull[st % WS], (st / WS) & 1, abort, err);
-                    const float4 *crd = reinterpret_cast<const float4 *>(sm.aux[st % WS]);
-                    // one task: the kernel-tile values of k-step kk for this
-                    // lane's row (east / north, or the three Cartesian
-                    // components in the proxy pass)
-                    auto values = [&](int kk, float (&ve)[8], float (&vn)[8], float (&vz)[8]) {
-                            if (MODE == 2) {
-                                // upward: the BLI basis of proxy (i, j) at the 8 points,
-                                // F_i(xi) G_j(eta) from the per-point factors
-                                const float *Fb = sm.aux[st % WS] + 16 * n * kk;
-                                const float4 f0 = *reinterpret_cast<const float4 *>(Fb + 8 * up_i);
-                                const float4 f1 = *reinterpret_cast<const float4 *>(Fb + 8 * up_i + 4);
-                                const float4 g0 = *reinterpret_cast<const float4 *>(Fb + 8 * n + 8 * up_j);
-                                const float4 g1 = *reinterpret_cast<const float4 *>(Fb + 8 * n + 8 * up_j + 4);
-                                ve[0] = f0.x * g0.x; ve[1] = f0.y * g0.y; ve[2] = f0.z * g0.z; ve[3] = f0.w * g0.w;
-                                ve[4] = f1.x * g1.x; ve[5] = f1.y * g1.y; ve[6] = f1.z * g1.z; ve[7] = f1.w * g1.w;
+            // TF32 stages: the same two teams.  Leaf pass: a stage's tasks to a
+            // team's warps by row block, as above.  Proxy and upward pass: warp w of
+            // the team takes unit w for all row blocks.  (Tasks dealt over eight
+            // warps left two idle at three row blocks, with an item record from
+            // global memory and a wait a stage for each.  Proxy passes of a solve
+            // at 2.3M cells x 64 fields: that 7.44 ms, teams 6.85, tf32_hi_tile
+            // 6.47, two row blocks side by side 6.28; half units over all eight
+            // warps, every stage: 7.08 with the first of these.)
+            constexpr int kB = MODE == 0 ? 1 : MODE == 1 ? (kTcProxyRows + 31) / 32 : kTcRows / 32;   // row blocks of a task
+            const int team = warp >> 2, tw = warp & 3;
+            const int n_all = G.nst, n_kern = G.nst - G.nstd;
+            float tl[kB][3];   // targets relative to the group's centre
+            int up_i[kB], up_j[kB];   // upward: proxy row0 + row = up_i + up_j n
 #pragma unroll
-                                for (int c = 0; c < 8; ++c) vn[c] = 0.f;
-                            } else if (MODE == 0 && kind == 2) {
-                                // DOWN: BLI basis of the target x its unit vector's
-                                // component of the Cartesian row
-                                const int *km0 = sm.kmap + it.row0 + SK * j + 8 * kk;
+            for (int b = 0; b < kB; ++b) {
+                const int r = 32 * b + lane;
+                tl[b][0] = tl0; tl[b][1] = tl1; tl[b][2] = tl2;
+                up_i[b] = up_j[b] = 0;
+                if (MODE == 1) {
+                    const double4 c = a.tgt[(size_t)G.tgt * P + G.row0 + (r < G.nt ? r : 0)];
+                    tl[b][0] = (float)(c.x - G.cx);
+                    tl[b][1] = (float)(c.y - G.cy);
+                    tl[b][2] = (float)(c.z - G.cz);
+                }
+                if (MODE == 2) {
+                    const int p = G.row0 + (r < G.nt ? r : 0);
+                    up_i[b] = p % n;
+                    up_j[b] = p / n;
+                }
+            }
+            // canonical offsets (floats) of row block 0's rows in a kernel tile (a
+            // row block is 256 floats on): leaf east / north at rows t, half + t;
+            // proxy x / y / z at 85 c + r
+            const int oe = canon(MODE == 0 ? row : lane, 0) >> 2;
+            const int on = canon(MODE == 0 ? half + row : kTcProxyRows + lane, 0) >> 2;
+            const int oz = canon(MODE == 0 ? 0 : 2 * kTcProxyRows + lane, 0) >> 2;
+#pragma unroll 1
+            for (int k = 0; k < n_all; ++k, ++st) {
+                const bool down = MODE == 0 && k >= n_kern;
+                if (!down && (st & 1) != (uint32_t)team) continue;
+                const uint32_t slot = st % KS, kpar = ((st / KS) - 1) & 1, jb = st % WS;
+                bool slot_free = st < (uint32_t)KS;
+                const bool ok = wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err);
+                const float4 rec = sm.rec[jb];
+                const int flags = ok ? __float_as_int(rec.w) : 0, nks = flags & kRecUnits;
+                // the MMAs that last read the slot must be done before the first
+                // store into it
+                auto claim = [&]() {
+                    if (!slot_free) wait_bounded(&sm.kempty[slot], kpar, abort, err);
+                    slot_free = true;
+                };
+                // kernel value x displacement (leaf: projected east, north; proxy: the
+                // Cartesian vector val (s - x)) of two columns for row block b; crd: the
+                // columns' x, and 4, 8 further on y and z (the same address in every lane:
+                // shared-memory broadcasts)
+                auto pair = [&](const float2 *crd, float2 tx2, float2 ty2, float2 tz2, float *vx, float *vy, float *vz) {
+                    const float2 dx = sub2(crd[0], tx2), dy = sub2(crd[4], ty2), dz = sub2(crd[8], tz2);
+                    // + 1e-20: mp = 0 only for a source on the target itself (or
+                    // a repeated point), and the floor keeps the value finite;
+                    // chords of neighbours (mp >= 1e-12) do not see it
+                    const float2 mp = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, f2(1e-20f))));
+                    const float2 r = make_float2(rsqrt_approx(mp.x), rsqrt_approx(mp.y));
+                    const float2 w = __fadd2_rn(__fmul2_rn(mp, r), f2(2.f));
+                    const float2 u = make_float2(rcp_approx(w.x), rcp_approx(w.y));
+                    const float2 inner = __ffma2_rn(f2(kC1F), r, __ffma2_rn(f2(kTwoC2F), u, f2(-kTwoC2F)));
+                    const float2 v = __fmul2_rn(inner, __fmul2_rn(r, r));
+                    float2 a, b;
+                    if (MODE == 0) {
+                        a = __fmul2_rn(v, __ffma2_rn(el1v, dy, __fmul2_rn(el0v, dx)));
+                        b = __fmul2_rn(v, __ffma2_rn(ep2v, dz, __ffma2_rn(ep1v, dy, __fmul2_rn(ep0v, dx))));
+                    } else {
+                        const float2 c = __fmul2_rn(v, dz);
+                        a = __fmul2_rn(v, dx);
+                        b = __fmul2_rn(v, dy);
+                        vz[0] = c.x;
+                        vz[1] = c.y;
+                    }
+                    vx[0] = a.x;
+                    vx[1] = a.y;
+                    vy[0] = b.x;
+                    vy[1] = b.y;
+                };
+                // four values of a row into a tile (hi; lo kTileFloats on): TF32 hi + lo
+                // (the tensor cores read lo's top 11 bits)
+                auto store = [&](float *th, const float *v) {
+                    const float4 h = make_float4(tf32_hi_tile(v[0]), tf32_hi_tile(v[1]), tf32_hi_tile(v[2]), tf32_hi_tile(v[3]));
+                    const float2 l01 = sub2(make_float2(v[0], v[1]), make_float2(h.x, h.y));
+                    const float2 l23 = sub2(make_float2(v[2], v[3]), make_float2(h.z, h.w));
+                    *reinterpret_cast<float4 *>(th) = h;
+                    *reinterpret_cast<float4 *>(th + kTileFloats) = make_float4(l01.x, l01.y, l23.x, l23.y);
+                };
+                if constexpr (MODE == 0) {
+                    // a DOWN slot's 3 P rows are slot_stages stages
+                    const int slot_stages = (3 * P + SK - 1) / SK;
+                    if (down && (k - n_kern) % slot_stages == 0) {
+                        // BLI bases of every target row in the new slot: thread t < 128
+                        // the xi basis of target t, thread 128 + t its eta basis
+                        const int slot_items = (3 * P + kTcChunk - 1) / kTcChunk;
+                        const int slot_id = a.items[G.ie - G.ndown + (k - n_kern) / slot_stages * slot_items].off;
+                        producers_sync(32 * kProdWarps);
+                        const int brow = tid & (kTcRows - 1);
+                        if (brow < G.nt) {
+                            const double2 e = a.xieta[G.tgt + brow];
+                            const double *nodes = a.tgt_nodes + (size_t)slot_id * 2 * n;
+                            down_basis(tid < kTcRows ? e.x : e.y, tid < kTcRows ? nodes : nodes + n, n,
+                                       tid < kTcRows ? sm.fx[brow] : sm.fe[brow]);
+                        }
+                        producers_sync(32 * kProdWarps);
+                    }
+                    const int kstride = down ? kstride8 : rb >= 3 ? 1 : rb == 2 ? 2 : 4;
+                    // units kk, kk + kstride, ... (K of them) of this row
+                    auto units = [&]<int K>(int kk) {
+                        float ve[K][8], vn[K][8];
+#pragma unroll
+                        for (int i = 0; i < K; ++i) {
+                            const int u = kk + i * kstride;
+                            if (down) {
+                                // BLI basis of the target x its unit vector's component of
+                                // the Cartesian row
+                                const int *km0 = sm.kmap + sm.rec2[jb].y + 8 * u;
                                 const float *fxr = sm.fx[row], *fer = sm.fe[row];
 #pragma unroll
                                 for (int c = 0; c < 8; ++c) {
                                     const int km = km0[c];
                                     const float b = fxr[km & 255] * fer[(km >> 8) & 255];
                                     const int comp = km >> 16;
-                                    ve[c] = comp == 2 ? 0.f : b * (comp == 0 ? el0 : el1);
-                                    vn[c] = b * (comp == 0 ? ep0 : (comp == 1 ? ep1 : ep2));
+                                    ve[i][c] = comp == 2 ? 0.f : b * (comp == 0 ? el0 : el1);
+                                    vn[i][c] = b * (comp == 0 ? ep0 : (comp == 1 ? ep1 : ep2));
                                 }
                             } else {
-                                // PP / PC: kernel value x projected displacement,
-                                // two columns per packed instruction
-                                // this k-step's x[8] y[8] z[8] (same address in every
-                                // lane: shared-memory broadcasts)
-                                float4 pre[6];
+                                const float2 *crd = reinterpret_cast<const float2 *>(sm.aux[jb]) + 12 * u;
+                                const float2 tx2 = f2(tl0 - rec.x), ty2 = f2(tl1 - rec.y), tz2 = f2(tl2 - rec.z);
 #pragma unroll
-                                for (int i = 0; i < 6; ++i) pre[i] = crd[6 * kk + i];
+                                for (int c2 = 0; c2 < 4; ++c2)
+                                    pair(crd + c2, tx2, ty2, tz2, ve[i] + 2 * c2, vn[i] + 2 * c2, nullptr);
+                                if (flags & kRecSelf) {
+                                    // the target itself among these 8 sources: the self pair
+                                    const int cs = my_pos - (sm.rec2[jb].x + 8 * u);
 #pragma unroll
-                                for (int c2 = 0; c2 < 4; ++c2) {
-                                    // pre[0..1] = x[8], pre[2..3] = y[8], pre[4..5] = z[8]
-                                    const float4 X = pre[c2 >> 1], Y = pre[2 + (c2 >> 1)], Z = pre[4 + (c2 >> 1)];
-                                    const float2 dx = sub2((c2 & 1) ? make_float2(X.z, X.w) : make_float2(X.x, X.y), tx2);
-                                    const float2 dy = sub2((c2 & 1) ? make_float2(Y.z, Y.w) : make_float2(Y.x, Y.y), ty2);
-                                    const float2 dz = sub2((c2 & 1) ? make_float2(Z.z, Z.w) : make_float2(Z.x, Z.y), tz2);
-                                    // + 1e-20: mp = 0 only for a source on the target itself (or
-                                    // a repeated point), and the floor keeps the value finite;
-                                    // chords of neighbours (mp >= 1e-12) do not see it
-                                    const float2 mp = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, f2(1e-20f))));
-                                    const float2 r = make_float2(rsqrt_approx(mp.x), rsqrt_approx(mp.y));
-                                    const float2 w = __fadd2_rn(__fmul2_rn(mp, r), f2(2.f));
-                                    const float2 u = make_float2(rcp_approx(w.x), rcp_approx(w.y));
-                                    const float2 inner = __ffma2_rn(f2(kC1F), r, __ffma2_rn(f2(kTwoC2F), u, f2(-kTwoC2F)));
-                                    const float2 v = __fmul2_rn(inner, __fmul2_rn(r, r));
-                                    if (MODE == 0) {
-                                        const float2 pe = __ffma2_rn(el1v, dy, __fmul2_rn(el0v, dx));
-                                        const float2 pn = __ffma2_rn(ep2v, dz, __ffma2_rn(ep1v, dy, __fmul2_rn(ep0v, dx)));
-                                        const float2 e2 = __fmul2_rn(v, pe), n2 = __fmul2_rn(v, pn);
-                                        ve[2 * c2] = e2.x;
-                                        ve[2 * c2 + 1] = e2.y;
-                                        vn[2 * c2] = n2.x;
-                                        vn[2 * c2 + 1] = n2.y;
-                                    } else {
-                                        // proxy targets: the Cartesian vector val (s - x)
-                                        const float2 x2 = __fmul2_rn(v, dx), y2 = __fmul2_rn(v, dy), z2 = __fmul2_rn(v, dz);
-                                        ve[2 * c2] = x2.x;
-                                        ve[2 * c2 + 1] = x2.y;
-                                        vn[2 * c2] = y2.x;
-                                        vn[2 * c2 + 1] = y2.y;
-                                        vz[2 * c2] = z2.x;
-                                        vz[2 * c2 + 1] = z2.y;
-                                    }
-                                }
-                                // the target itself among these 8 sources: the self pair
-                                if (self_item) {
-                                    const int cs = my_pos - (it.off + SK * j + 8 * kk);
-                                    if ((unsigned)cs < 8u) {
-#pragma unroll
-                                        for (int c = 0; c < 8; ++c)
-                                            if (c == cs) { ve[c] = self_e; vn[c] = self_n; }
-                                    }
+                                    for (int c = 0; c < 8; ++c)
+                                        if (c == cs) { ve[i][c] = self_e; vn[i][c] = self_n; }
                                 }
                             }
-                    };
-                    // its TF32 hi + lo split, stored into the kernel tile
-                    auto store = [&](int kk, const float (&ve)[8], const float (&vn)[8], const float (&vz)[8]) {
-                            // TF32 hi + lo (the tensor cores read lo's top 11 bits)
-                            float *th = sm.Kt(slot, kk, 0), *tlo = sm.Kt(slot, kk, 1);
-#pragma unroll
-                            for (int hh = 0; hh < 2; ++hh) {
-                                const float4 eh = make_float4(tf32_hi(ve[4 * hh]), tf32_hi(ve[4 * hh + 1]),
-                                                              tf32_hi(ve[4 * hh + 2]), tf32_hi(ve[4 * hh + 3]));
-                                const float4 nh = make_float4(tf32_hi(vn[4 * hh]), tf32_hi(vn[4 * hh + 1]),
-                                                              tf32_hi(vn[4 * hh + 2]), tf32_hi(vn[4 * hh + 3]));
-                                const float2 el01 = sub2(make_float2(ve[4 * hh], ve[4 * hh + 1]), make_float2(eh.x, eh.y));
-                                const float2 el23 = sub2(make_float2(ve[4 * hh + 2], ve[4 * hh + 3]), make_float2(eh.z, eh.w));
-                                const float2 nl01 = sub2(make_float2(vn[4 * hh], vn[4 * hh + 1]), make_float2(nh.x, nh.y));
-                                const float2 nl23 = sub2(make_float2(vn[4 * hh + 2], vn[4 * hh + 3]), make_float2(nh.z, nh.w));
-                                if (row_in_tile) {
-                                    *reinterpret_cast<float4 *>(th + oe + 32 * hh) = eh;
-                                    *reinterpret_cast<float4 *>(tlo + oe + 32 * hh) = make_float4(el01.x, el01.y, el23.x, el23.y);
-                                    if (MODE != 2) {
-                                        *reinterpret_cast<float4 *>(th + on + 32 * hh) = nh;
-                                        *reinterpret_cast<float4 *>(tlo + on + 32 * hh) = make_float4(nl01.x, nl01.y, nl23.x, nl23.y);
-                                    }
-                                }
-                                if (MODE == 1) {
-                                    const float4 zh = make_float4(tf32_hi(vz[4 * hh]), tf32_hi(vz[4 * hh + 1]),
-                                                                  tf32_hi(vz[4 * hh + 2]), tf32_hi(vz[4 * hh + 3]));
-                                    const float2 zl01 = sub2(make_float2(vz[4 * hh], vz[4 * hh + 1]), make_float2(zh.x, zh.y));
-                                    const float2 zl23 = sub2(make_float2(vz[4 * hh + 2], vz[4 * hh + 3]), make_float2(zh.z, zh.w));
-                                    if (row_in_tile) {
-                                        *reinterpret_cast<float4 *>(th + oz + 32 * hh) = zh;
-                                        *reinterpret_cast<float4 *>(tlo + oz + 32 * hh) = make_float4(zl01.x, zl01.y, zl23.x, zl23.y);
-                                    }
-                                }
-                            }
-                    };
-                    {
-                        // The proxy pass takes two tasks at a time (their values are
-                        // independent, so the second's arithmetic fills the first's
-                        // latencies; measured 5 % on that pass).  The leaf pass gains
-                        // nothing from it and keeps its registers.
-                        constexpr int kPair = MODE == 1 ? 2 : 1;
-#pragma unroll 1
-                        for (int kk = kfirst8; active && kk < nks; kk += kPair * kstride8) {
-                            float ve[8], vn[8], vz[8], ve2[8], vn2[8], vz2[8];
-                            const int k2 = kk + kstride8;
-                            const bool two = kPair == 2 && k2 < nks;
-                            values(kk, ve, vn, vz);
-                            if (kPair == 2) values(two ? k2 : kk, ve2, vn2, vz2);
-                            if (!slot_free) {
-                                wait_bounded(&sm.kempty[slot], kpar, abort, err);
-                                slot_free = true;
-                            }
-                            store(kk, ve, vn, vz);
-                            if (two) store(k2, ve2, vn2, vz2);
                         }
+                        claim();
+                        if (!row_in_tile) return;
+#pragma unroll
+                        for (int i = 0; i < K; ++i) {
+                            float *th = sm.Kt(slot, kk + i * kstride, 0);
+                            store(th + oe, ve[i]);
+                            store(th + oe + 32, ve[i] + 4);
+                            store(th + on, vn[i]);
+                            store(th + on + 32, vn[i] + 4);
+                        }
+                    };
+                    int kk = !active ? nks : down ? kfirst8 : rb >= 3 ? 0 : rb == 2 ? tw >> 1 : tw;
+                    if (!(flags & (kRecDown | kRecSelf))) {
+#pragma unroll 1
+                        for (; kk + kstride < nks; kk += 2 * kstride) units.template operator()<2>(kk);
                     }
-                    if (!slot_free) {
-                        // warps that wrote nothing: their arrival must still
-                        // not run a ring phase ahead of the MMAs
-                        wait_bounded(&sm.kempty[slot], kpar, abort, err);
-                    } else {
-                        dev::fence_proxy_async();
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sm.kfull[slot]);
+#pragma unroll 1
+                    for (; kk < nks; kk += kstride) units.template operator()<1>(kk);
+                } else if (tw < nks) {
+                    // unit tw for row blocks b0, b0 + 1 (NB of them side by side: the
+                    // second's arithmetic fills the first's latencies), then the next
+                    auto blocks = [&]<int NB>(int b0) {
+                        float v[NB][3][8];
+#pragma unroll
+                        for (int i = 0; i < NB; ++i) {
+                            const int b = b0 + i;
+                            if (MODE == 1) {
+                                const float2 *crd = reinterpret_cast<const float2 *>(sm.aux[jb]) + 12 * tw;
+                                const float2 tx2 = f2(tl[b][0] - rec.x), ty2 = f2(tl[b][1] - rec.y), tz2 = f2(tl[b][2] - rec.z);
+#pragma unroll
+                                for (int c2 = 0; c2 < 4; ++c2)
+                                    pair(crd + c2, tx2, ty2, tz2, v[i][0] + 2 * c2, v[i][1] + 2 * c2, v[i][2] + 2 * c2);
+                            } else {
+                                // upward: the BLI basis of proxy (i, j) at the 8 points, F_i(xi)
+                                // G_j(eta) from the per-point factors
+                                const float *Fb = sm.aux[jb] + 16 * n * tw;
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) {
+                                    const float4 f = *reinterpret_cast<const float4 *>(Fb + 8 * up_i[b] + 4 * h);
+                                    const float4 g = *reinterpret_cast<const float4 *>(Fb + 8 * n + 8 * up_j[b] + 4 * h);
+                                    v[i][0][4 * h] = f.x * g.x;
+                                    v[i][0][4 * h + 1] = f.y * g.y;
+                                    v[i][0][4 * h + 2] = f.z * g.z;
+                                    v[i][0][4 * h + 3] = f.w * g.w;
+                                }
+                            }
+                        }
+                        claim();
+#pragma unroll
+                        for (int i = 0; i < NB; ++i) {
+                            const int b = b0 + i;
+                            if (MODE == 1 && 32 * b + lane >= kTcProxyRows) break;
+                            float *th = sm.Kt(slot, tw, 0) + 256 * b;
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                store(th + oe + 32 * h, v[i][0] + 4 * h);
+                                if (MODE == 1) {
+                                    store(th + on + 32 * h, v[i][1] + 4 * h);
+                                    store(th + oz + 32 * h, v[i][2] + 4 * h);
+                                }
+                            }
+                        }
+                    };
+                    blocks.template operator()<2>(0);
+                    if (rb > 2) blocks.template operator()<kB - 2>(2);
                 }
+                // warps that wrote nothing: their arrival must still not run a ring
+                // phase ahead of the MMAs
+                claim();
+                dev::fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_n(&sm.kfull[slot], down ? 1 : 2);
             }
         }
     } else if (warp == kMmaWarp) {
@@ -1183,11 +1218,12 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             const int gk = grid_of(gi);
             const TcArgs &a = J.g[gk];
             const MixGroup G = a.groups[gi - J.beg[gk]];
-            // FP16 computing launches take an item's units and chain end from the
-            // loader's record
-            constexpr bool kRec = F16 && TS != 2;
+            // computing launches take a stage's units and chain end from the
+            // loader's record; a replay's stage is an item
+            constexpr bool kRec = TS != 2;
             ItemWindow w;
             if (!kRec) w.start(a.items, G.ib, G.ie, lane);
+            const int nstages = F16 ? G.ie - G.ib : G.nst;
             // the group's columns: component c of target t is column half c + t
             // (half: the targets rounded up to 16), so small groups' MMAs are
             // narrow; the proxy pass has three components of 85 rows, the
@@ -1196,70 +1232,67 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             const uint32_t idesc = idesc_n(F16 ? kIdescF16 : kIdesc, MODE == 0 ? 2 * half : MODE == 1 ? 256 : 128);
             // replay: bytes of one packed tile (east rows, then north rows)
             const uint32_t ptile = 2u * (uint32_t)half * 32u;
-            for (int k = G.ib; k < G.ie; ++k) {
+            for (int k = 0; k < nstages; ++k, ++st) {
                 TcItem it{};
-                if (!kRec) it = w.get(k, lane);
+                if (!kRec) it = w.get(G.ib + k, lane);
                 bool flush = it.kind & kTcFlush;
-                const int nst = kRec ? 1 : (it.cnt + SK - 1) / SK;
-                for (int j = 0; j < nst; ++j, ++st) {
-                    const uint32_t slot = st % KS, jb = st % WS;
-                    // replay: the stage's one barrier covers its weight and kernel tiles
-                    // (polled together: the one's latency hides the other's)
-                    bool ok = true;
-                    const bool wf = TS == 2 || dev::mbar_try_wait(&sm.wfull[jb], (st / WS) & 1);
-                    const bool kf = dev::mbar_try_wait(&sm.kfull[slot], (st / KS) & 1);
-                    if (!kf) ok = wait_bounded(&sm.kfull[slot], (st / KS) & 1, abort, err);
-                    if (!wf) ok = wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err) && ok;
-                    // a new chain overwrites the accumulator, whose last chain
-                    // (cc - 1) the fold warps must have read
-                    if (!chain_open && cc >= 1) ok = wait_bounded(&sm.accfree, (cc - 1) & 1, abort, err) && ok;
-                    ok = __all_sync(0xffffffffu, ok);
-                    tc_fence_after();
-                    int nks = (min(SK, it.cnt - SK * j) + 7) >> 3;
-                    if (kRec) {
-                        const int flags = __float_as_int(sm.rec[jb].w);
-                        nks = flags & kRecUnits;
-                        flush = flags & kRecFlush;
-                    }
-                    const uint32_t open = chain_open ? 1u : 0u;
-                    if (elect_one()) {
-                        if (ok) {
-                            if constexpr (TS == 2) {
-                                // packed tiles of MMA step s: hi at (2s) ptile, lo at (2s + 1) ptile
-                                const uint64_t aw = smem_desc_w16(sm.ring + TcSmem<TS>::kKtBytes + sm.woff[slot]);
-                                const uint64_t bt = smem_desc(sm.ring + sm.toff[slot]);
-#pragma unroll
-                                for (int s = 0; s < SK / 16; ++s)
-                                    if (2 * s < nks) {
-                                        const uint64_t a = aw + s * (2 * kW16UnitBytes >> 4), bh = bt + 2 * s * (ptile >> 4);
-                                        mma_ss_f16(tmem, a, bh, idesc, s ? 1u : open);
-                                        mma_ss_f16(tmem, a, bh + (ptile >> 4), idesc, 1u);
-                                    }
-                            } else {
-                                // FP16: 16 sources per MMA (weight units 2s and 2s + 1); TF32: 8
-                                constexpr uint32_t kStepW = kWStepFloats * 4 >> 4, kStepT = kTileFloats * 4 >> 4;
-                                const uint64_t aw = F16 ? smem_desc_w16(sm.Wt(jb)) : smem_desc(sm.Wt(jb));
-                                const uint64_t bt = smem_desc(sm.Kt(slot, 0, 0));
-#pragma unroll
-                                for (int s = 0; s < kStageKs; ++s)
-                                    if ((F16 ? 2 : 1) * s < nks) {
-                                        const uint64_t a = aw + s * kStepW, bh = bt + 2 * s * kStepT;
-                                        if (F16) {
-                                            mma_ss_f16(tmem, a, bh, idesc, s ? 1u : open);
-                                            mma_ss_f16(tmem, a, bh + kStepT, idesc, 1u);
-                                        } else {
-                                            mma_ss(tmem, a, bh, idesc, s ? 1u : open);
-                                            mma_ss(tmem, a, bh + kStepT, idesc, 1u);
-                                        }
-                                    }
-                            }
-                        }
-                        mma_commit(&sm.kempty[slot]);
-                        if (TS != 2) mma_commit(&sm.wempty[jb]);
-                    }
-                    chain_open = true;
-                    __syncwarp();
+                const uint32_t slot = st % KS, jb = st % WS;
+                // replay: the stage's one barrier covers its weight and kernel tiles
+                // (polled together: the one's latency hides the other's)
+                bool ok = true;
+                const bool wf = TS == 2 || dev::mbar_try_wait(&sm.wfull[jb], (st / WS) & 1);
+                const bool kf = dev::mbar_try_wait(&sm.kfull[slot], (st / KS) & 1);
+                if (!kf) ok = wait_bounded(&sm.kfull[slot], (st / KS) & 1, abort, err);
+                if (!wf) ok = wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err) && ok;
+                // a new chain overwrites the accumulator, whose last chain
+                // (cc - 1) the fold warps must have read
+                if (!chain_open && cc >= 1) ok = wait_bounded(&sm.accfree, (cc - 1) & 1, abort, err) && ok;
+                ok = __all_sync(0xffffffffu, ok);
+                tc_fence_after();
+                int nks = (it.cnt + 7) >> 3;
+                if (kRec) {
+                    const int flags = __float_as_int(sm.rec[jb].w);
+                    nks = flags & kRecUnits;
+                    flush = flags & kRecFlush;
                 }
+                const uint32_t open = chain_open ? 1u : 0u;
+                if (elect_one()) {
+                    if (ok) {
+                        if constexpr (TS == 2) {
+                            // packed tiles of MMA step s: hi at (2s) ptile, lo at (2s + 1) ptile
+                            const uint64_t aw = smem_desc_w16(sm.ring + TcSmem<TS>::kKtBytes + sm.woff[slot]);
+                            const uint64_t bt = smem_desc(sm.ring + sm.toff[slot]);
+#pragma unroll
+                            for (int s = 0; s < SK / 16; ++s)
+                                if (2 * s < nks) {
+                                    const uint64_t a = aw + s * (2 * kW16UnitBytes >> 4), bh = bt + 2 * s * (ptile >> 4);
+                                    mma_ss_f16(tmem, a, bh, idesc, s ? 1u : open);
+                                    mma_ss_f16(tmem, a, bh + (ptile >> 4), idesc, 1u);
+                                }
+                        } else {
+                            // FP16: 16 sources per MMA (weight units 2s and 2s + 1); TF32: 8
+                            constexpr uint32_t kStepW = kWStepFloats * 4 >> 4, kStepT = kTileFloats * 4 >> 4;
+                            const uint64_t aw = F16 ? smem_desc_w16(sm.Wt(jb)) : smem_desc(sm.Wt(jb));
+                            const uint64_t bt = smem_desc(sm.Kt(slot, 0, 0));
+#pragma unroll
+                            for (int s = 0; s < kStageKs; ++s)
+                                if ((F16 ? 2 : 1) * s < nks) {
+                                    const uint64_t a = aw + s * kStepW, bh = bt + 2 * s * kStepT;
+                                    if (F16) {
+                                        mma_ss_f16(tmem, a, bh, idesc, s ? 1u : open);
+                                        mma_ss_f16(tmem, a, bh + kStepT, idesc, 1u);
+                                    } else {
+                                        mma_ss(tmem, a, bh, idesc, s ? 1u : open);
+                                        mma_ss(tmem, a, bh + kStepT, idesc, 1u);
+                                    }
+                                }
+                        }
+                    }
+                    mma_commit(&sm.kempty[slot]);
+                    if (TS != 2) mma_commit(&sm.wempty[jb]);
+                }
+                chain_open = true;
+                __syncwarp();
                 if (flush) {
                     if (elect_one()) mma_commit(&sm.accfull);
                     __syncwarp();
@@ -1287,137 +1320,115 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             // rows, rounded up to 16 rows of 32 bytes)
             const unsigned char *tsrc = TS == 2 ? a.ktile + a.ktile_off[gi - J.beg[gk]] : nullptr;
             const uint32_t cb = (uint32_t)((G.nt + 15) & ~15) * 32u;
-            if constexpr (F16 && TS != 2) {
-                // FP16 computing launches: an item is one stage.  Lane l holds item
-                // k0 + l of the window: it writes the item's record itself, and the
-                // copies need two of its numbers only.  (The whole record by
-                // shuffles, twice, and an L2 prefetch of the next item's tiles, made
-                // this warp the slowest of a small group's stage: 1,240 cycles.)
+            if constexpr (TS != 2) {
+                // Lane l holds item k0 + l of the window: it writes its stages'
+                // records itself, and the copies need a few of its numbers only.
+                // (The whole record by shuffles, twice, and an L2 prefetch of the
+                // next item's tiles, made this warp the slowest of a small group's
+                // stage: 1,240 cycles.)
 #pragma unroll 1
-                for (int k = G.ib; k < G.ie; ++k, ++st) {
+                for (int k = G.ib; k < G.ie; ++k) {
                     w.seek(k, lane);
                     const int l = k - w.k0;
-                    const uint32_t jb = st % WS, ub = st / WS;
                     const TcItem &it = w.cur;
-                    const int units = (it.cnt + 7) >> 3;
-                    const bool self = (it.kind & 3) == 0 && it.off < G.tgt + G.nt && G.tgt < it.off + it.cnt;
-                    const int flags = units | (it.kind & 3) << 4 | ((it.kind & kTcFlush) ? kRecFlush : 0) | (self ? kRecSelf : 0);
-                    const int kb = __shfl_sync(0xffffffffu, it.kb, l), fl = __shfl_sync(0xffffffffu, flags, l);
-                    bool ok = true;
-                    if (ub > 0) ok = wait_bounded(&sm.wempty[jb], (ub - 1) & 1, abort, err);
-                    if (lane == l) {
-                        // before the arrival that its readers wait for
-                        sm.rec[jb] = make_float4(it.dx, it.dy, it.dz, __int_as_float(flags));
-                        sm.rec2[jb] = make_int2(it.off, it.row0);
-                    }
-                    ok = __all_sync(0xffffffffu, ok);
-                    __syncwarp();
-                    if (elect_one()) {
-                        // whole 16-source MMA steps (the store has a spare unit at its
-                        // end), and the point and proxy sources' coordinates (24 floats
-                        // per unit; DOWN rows need none)
-                        const uint32_t nks = fl & kRecUnits, wbytes = ((nks + 1) & ~1u) * kW16UnitBytes;
-                        const uint32_t lbytes = (fl & kRecDown) ? 0u : nks * 96u;
-                        dev::mbar_expect_tx(&sm.wfull[jb], wbytes + lbytes);
-                        if (ok) {
-                            if (lbytes) dev::bulk_g2s(sm.aux[jb], a.sxyz + (size_t)kb * 24, lbytes, &sm.wfull[jb]);
-                            dev::bulk_g2s(sm.Wt(jb), static_cast<const char *>(a.bstore16) + (size_t)kb * kW16UnitBytes, wbytes,
-                                          &sm.wfull[jb]);
-                        }
-                    }
-                    __syncwarp();
-                }
-                continue;
-            }
-            for (int k = G.ib; k < G.ie; ++k) {
-                const TcItem it = w.get(k, lane);
-                if (k + 1 < G.ie) {
-                    const TcItem nxt = w.get(k + 1, lane);
-                    // the next item's weight tiles (and source coordinates)
-                    // into L2 while this item's stages run
-                    if (MODE != 2 && elect_one()) {
-                        const uint32_t nks = (uint32_t)(nxt.cnt + 7) >> 3;
-                        if (F16)
-                            prefetch_l2(static_cast<const char *>(a.bstore16) + (size_t)nxt.kb * kW16UnitBytes,
-                                        ((nks + 1) & ~1u) * kW16UnitBytes);
-                        else
-                            prefetch_l2(a.bstore + (size_t)nxt.kb * kWStepFloats, nks * kWStepFloats * 4u);
-                        if (TS != 2 && (nxt.kind & 3) != 2) prefetch_l2(a.sxyz + (size_t)nxt.kb * 24, nks * 96u);
-                    }
-                }
-                const int nst = (it.cnt + SK - 1) / SK;
-                for (int j = 0; j < nst; ++j, ++st) {
-                    const int nks = (min(SK, it.cnt - SK * j) + 7) >> 3;
-                    if constexpr (TS == 2) {
-                        // the stage's kernel tiles and weight tiles, each one
-                        // bulk copy into its ring (from the start of a ring
-                        // when they do not fit before its end), once the stage
-                        // slot and both ranges are free: stages retire in order
-                        const uint32_t nsteps = (uint32_t)(nks + 1) >> 1;
-                        const uint32_t sb = nsteps * 4u * cb, wb = nsteps * 2u * kW16UnitBytes;
-                        const uint32_t tpos = thead + sb > (uint32_t)kTRingBytes ? 0u : thead;
-                        const uint32_t wpos = whead + wb > (uint32_t)kWRingBytes ? 0u : whead;
-                        while (oldest < st) {
-                            bool clash = st - oldest >= (uint32_t)KS;
-                            for (uint32_t x = oldest; !clash && x < st; ++x) {
-                                const uint32_t xs = x % KS;
-                                const uint32_t t0 = sm.toff[xs], t1 = t0 + sm.tlen[xs];
-                                const uint32_t w0 = sm.woff[xs], w1 = w0 + sm.wlen[xs];
-                                clash = (tpos < t1 && t0 < tpos + sb) || (wpos < w1 && w0 < wpos + wb);
-                            }
-                            if (!clash) break;
-                            wait_bounded(&sm.kempty[oldest % KS], (oldest / KS) & 1, abort, err);
-                            ++oldest;
-                        }
-                        const uint32_t slot = st % KS;
-                        if (elect_one()) {
-                            sm.toff[slot] = tpos;
-                            sm.tlen[slot] = sb;
-                            sm.woff[slot] = wpos;
-                            sm.wlen[slot] = wb;
-                            // the offsets are written before the arrival the MMA warp waits on
-                            dev::mbar_expect_tx(&sm.kfull[slot], sb + wb);
-                            if (!*abort) {
-                                // the tiles are read once per solve: they leave L2 first, to
-                                // the weight tiles, which other groups read again
-                                dev::bulk_g2s_hint(sm.ring + tpos, tsrc, sb, &sm.kfull[slot], dev::l2_evict_first());
-                                dev::bulk_g2s_hint(sm.ring + TcSmem<TS>::kKtBytes + wpos,
-                                                   static_cast<const char *>(a.bstore16) + (size_t)(it.kb + SU * j) * kW16UnitBytes,
-                                                   wb, &sm.kfull[slot], dev::l2_evict_last());
-                            }
-                        }
-                        __syncwarp();
-                        tsrc += sb;
-                        thead = tpos + sb;
-                        whead = wpos + wb;
-                    } else {
+                    const int kind = it.kind & 3;
+                    const bool self = MODE == 0 && kind == 0 && it.off < G.tgt + G.nt && G.tgt < it.off + it.cnt;
+                    const int iflags = kind << 4 | ((it.kind & kTcFlush) ? kRecFlush : 0) | (self ? kRecSelf : 0);
+                    // F16: an item is one stage
+                    const int kb = __shfl_sync(0xffffffffu, it.kb, l), down = __shfl_sync(0xffffffffu, kind, l) == 2;
+                    const int cnt = __shfl_sync(0xffffffffu, it.cnt, l);
+                    const int row0 = MODE == 2 ? __shfl_sync(0xffffffffu, it.row0, l) : 0;
+#pragma unroll 1
+                    for (int b = 0; b < cnt; b += SK, ++st) {
                         const uint32_t jb = st % WS, ub = st / WS;
-                        if (ub > 0) wait_bounded(&sm.wempty[jb], (ub - 1) & 1, abort, err);
+                        const uint32_t nks = (uint32_t)(min(SK, cnt - b) + 7) >> 3;
+                        bool ok = true;
+                        if (ub > 0) ok = wait_bounded(&sm.wempty[jb], (ub - 1) & 1, abort, err);
+                        if (lane == l) {
+                            // before the arrival that its readers wait for; a chain ends
+                            // with an item's last stage
+                            const int flags = (int)nks | (b + SK < cnt ? iflags & ~kRecFlush : iflags);
+                            sm.rec[jb] = make_float4(it.dx, it.dy, it.dz, __int_as_float(flags));
+                            sm.rec2[jb] = make_int2(kind == 2 ? it.off : it.off + b, it.row0 + b);
+                        }
+                        ok = __all_sync(0xffffffffu, ok);
+                        __syncwarp();
                         if (elect_one()) {
-                            // FP16: whole 16-source MMA steps (the store has a spare unit at its end)
-                            const uint32_t wbytes = F16 ? (uint32_t)((nks + 1) & ~1) * kW16UnitBytes
-                                                        : (uint32_t)nks * kWStepFloats * 4;
-                            // with the weights: the stage's BLI factors (upward) or
-                            // its point / proxy sources' coordinates (24 floats per
-                            // k-step; DOWN rows need none)
-                            const uint32_t lbytes = MODE == 2 ? (uint32_t)nks * 64 * n
-                                                    : (it.kind & 3) != 2 ? (uint32_t)nks * 96u : 0u;
+                            // FP16: whole 16-source MMA steps (the store has a spare unit at
+                            // its end).  With the weights come the point and proxy sources'
+                            // coordinates (24 floats per unit; DOWN rows need none), or the
+                            // upward pass's BLI factors.
+                            const uint32_t wbytes = F16 ? ((nks + 1) & ~1u) * kW16UnitBytes : nks * kWStepFloats * 4u;
+                            const uint32_t lbytes = MODE == 2 ? nks * 64u * n : down ? 0u : nks * 96u;
+                            const size_t u = (size_t)kb + b / 8;
                             dev::mbar_expect_tx(&sm.wfull[jb], wbytes + lbytes);
-                            if (!*abort) {
+                            if (ok) {
                                 if (lbytes)
                                     dev::bulk_g2s(sm.aux[jb],
-                                                  MODE == 2 ? (const void *)(a.basis + (size_t)(it.row0 + SU * j) * 16 * n)
-                                                            : (const void *)(a.sxyz + (size_t)(it.kb + SU * j) * 24),
+                                                  MODE == 2 ? (const void *)(a.basis + ((size_t)row0 + b / 8) * 16 * n)
+                                                            : (const void *)(a.sxyz + u * 24),
                                                   lbytes, &sm.wfull[jb]);
-                                const void *wsrc =
-                                    F16 ? static_cast<const void *>(static_cast<const char *>(a.bstore16) +
-                                                                    (size_t)(it.kb + SU * j) * kW16UnitBytes)
-                                        : static_cast<const void *>(a.bstore + (size_t)(it.kb + SU * j) * kWStepFloats);
-                                dev::bulk_g2s(sm.Wt(jb), wsrc, wbytes, &sm.wfull[jb]);
+                                dev::bulk_g2s(sm.Wt(jb),
+                                              F16 ? (const void *)(static_cast<const char *>(a.bstore16) + u * kW16UnitBytes)
+                                                  : (const void *)(a.bstore + u * kWStepFloats),
+                                              wbytes, &sm.wfull[jb]);
                             }
                         }
                         __syncwarp();
                     }
+                }
+            } else {
+                for (int k = G.ib; k < G.ie; ++k, ++st) {
+                    const TcItem it = w.get(k, lane);
+                    if (k + 1 < G.ie) {
+                        // the next item's weight tiles into L2 while this item's stage runs
+                        const TcItem nxt = w.get(k + 1, lane);
+                        const uint32_t nks = (uint32_t)(nxt.cnt + 7) >> 3;
+                        if (elect_one())
+                            prefetch_l2(static_cast<const char *>(a.bstore16) + (size_t)nxt.kb * kW16UnitBytes,
+                                        ((nks + 1) & ~1u) * kW16UnitBytes);
+                    }
+                    // the stage's kernel tiles and weight tiles, each one bulk copy
+                    // into its ring (from the start of a ring when they do not fit
+                    // before its end), once the stage slot and both ranges are free:
+                    // stages retire in order
+                    const uint32_t nsteps = (uint32_t)(((it.cnt + 7) >> 3) + 1) >> 1;
+                    const uint32_t sb = nsteps * 4u * cb, wb = nsteps * 2u * kW16UnitBytes;
+                    const uint32_t tpos = thead + sb > (uint32_t)kTRingBytes ? 0u : thead;
+                    const uint32_t wpos = whead + wb > (uint32_t)kWRingBytes ? 0u : whead;
+                    while (oldest < st) {
+                        bool clash = st - oldest >= (uint32_t)KS;
+                        for (uint32_t x = oldest; !clash && x < st; ++x) {
+                            const uint32_t xs = x % KS;
+                            const uint32_t t0 = sm.toff[xs], t1 = t0 + sm.tlen[xs];
+                            const uint32_t w0 = sm.woff[xs], w1 = w0 + sm.wlen[xs];
+                            clash = (tpos < t1 && t0 < tpos + sb) || (wpos < w1 && w0 < wpos + wb);
+                        }
+                        if (!clash) break;
+                        wait_bounded(&sm.kempty[oldest % KS], (oldest / KS) & 1, abort, err);
+                        ++oldest;
+                    }
+                    const uint32_t slot = st % KS;
+                    if (elect_one()) {
+                        sm.toff[slot] = tpos;
+                        sm.tlen[slot] = sb;
+                        sm.woff[slot] = wpos;
+                        sm.wlen[slot] = wb;
+                        // the offsets are written before the arrival the MMA warp waits on
+                        dev::mbar_expect_tx(&sm.kfull[slot], sb + wb);
+                        if (!*abort) {
+                            // the tiles are read once per solve: they leave L2 first, to
+                            // the weight tiles, which other groups read again
+                            dev::bulk_g2s_hint(sm.ring + tpos, tsrc, sb, &sm.kfull[slot], dev::l2_evict_first());
+                            dev::bulk_g2s_hint(sm.ring + TcSmem<TS>::kKtBytes + wpos,
+                                               static_cast<const char *>(a.bstore16) + (size_t)it.kb * kW16UnitBytes,
+                                               wb, &sm.kfull[slot], dev::l2_evict_last());
+                        }
+                    }
+                    __syncwarp();
+                    tsrc += sb;
+                    thead = tpos + sb;
+                    whead = wpos + wb;
                 }
             }
         }
@@ -1450,22 +1461,34 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             }
             bool first = true;
             const int half = MODE == 0 ? (G.nt + 15) & ~15 : 128;   // columns per component
+            // everything a fold needs from global memory is read before its chain is
+            // awaited: the MMA warp waits for the fold
+            float fsc_kern = 1.f, fsc_down = 1.f;
+            if (F16) {
+                fsc_kern = 1.f / f16_scale(__uint_as_float(a.fmax[16 * q + (lane & 15)]));
+                fsc_down = 1.f / f16_scale(__uint_as_float(a.fmax[kF + 16 * q + (lane & 15)]));
+            }
             ItemWindow w;
             w.start(a.items, G.ib, G.ie, lane);
             for (int k = G.ib; k < G.ie; ++k) {
                 const int kind = w.kind(k, lane);
                 if (!(kind & kTcFlush)) continue;
-                wait_bounded(&sm.accfull, cc & 1, abort, err);
-                tc_fence_after();
                 // FP16: the chain's weight rows are the fields' source weights
                 // (scaled per field) against scaled kernel columns, or their
                 // potentials (scaled per field) against unscaled DOWN columns
                 const bool down_chain = (kind & 3) == 2;
-                const float fsc = F16 ? 1.f / f16_scale(__uint_as_float(a.fmax[(down_chain ? kF : 0) + 16 * q + (lane & 15)]))
-                                      : 1.f;
+                const float fsc = !F16 ? 1.f : down_chain ? fsc_down : fsc_kern;
                 const bool end = k == G.ie - 1;
-                fold_chain<MODE>(tq, lane, end, first, G.tgt, G.nt, F16, fsc, down_chain, a.tscale, sm.cs, half,
-                                 part_i, nparts);
+                float4 tsc = make_float4(1.f, 1.f, 1.f, 1.f);   // DOWN chains: scales of targets 32 k + lane
+                if (MODE == 0 && F16 && down_chain) {
+                    tsc.x = lane < G.nt ? a.tscale[G.tgt + lane] : 1.f;
+                    tsc.y = 32 + lane < G.nt ? a.tscale[G.tgt + 32 + lane] : 1.f;
+                    tsc.z = 64 + lane < G.nt ? a.tscale[G.tgt + 64 + lane] : 1.f;
+                    tsc.w = 96 + lane < G.nt ? a.tscale[G.tgt + 96 + lane] : 1.f;
+                }
+                wait_bounded(&sm.accfull, cc & 1, abort, err);
+                tc_fence_after();
+                fold_chain<MODE>(tq, lane, end, first, G.nt, F16, fsc, down_chain, tsc, sm.cs, half, part_i, nparts);
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sm.accfree);
