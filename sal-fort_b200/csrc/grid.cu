@@ -454,7 +454,7 @@ static int64_t batched_launches(const GridImpl &g, int FT) {
     if (tree) k += levels(pl.m2m_level_beg);
     k += 1;                                                                // store (proxies)
     if (!pl.tc_proxy_groups.empty()) k += 2 + (tree ? levels(pl.l2l_level_beg) : 0);   // proxy, finalize, l2l
-    k += pl.tc_opt.f16 ? 3 : 1;                                            // leaf store: maxima + FP16, or TF32
+    k += pl.tc_opt.f16 ? 2 : 1;                                            // leaf store: maxima + FP16, or TF32
     return k + 1;                                                          // leaf pass
 }
 

@@ -1513,6 +1513,13 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
     }
 }
 
+// Row of a split store entry s: weight row s, potential row -2 - s, or (-1, a
+// padding row: the caller puts zeros) the first weight row, so that a thread's
+// eight loads need no branches and are in flight together.
+__device__ __forceinline__ const float *store_row(int32_t s, const float *wF, const float *phiF) {
+    return s <= -2 ? phiF + (size_t)(-2 - s) * kF : wF + (size_t)(s >= 0 ? s : 0) * kF;
+}
+
 // Split weight store (k-steps [k0, k1) of it, with bsrc and bstore offset
 // by the caller): per k-step of 8 store rows, the 64-field rows as one
 // 128-row TF32 tile (field f's hi part at row wrow(f, 0), lo part at
@@ -1528,7 +1535,7 @@ __global__ void split_store_kernel(const int32_t *__restrict__ bsrc, int64_t nk,
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         const int32_t s = bsrc[ks * 8 + r];
-        const float v = s >= 0 ? wF[(size_t)s * kF + f] : (s <= -2 ? phiF[(size_t)(-2 - s) * kF + f] : 0.f);
+        const float x = store_row(s, wF, phiF)[f], v = s == -1 ? 0.f : x;
         hi[r] = tf32_hi(v);
         lo[r] = tf32_hi(v - hi[r]);
     }
@@ -1540,14 +1547,18 @@ __global__ void split_store_kernel(const int32_t *__restrict__ bsrc, int64_t nk,
     *reinterpret_cast<float4 *>(base + ol + 32) = make_float4(lo[4], lo[5], lo[6], lo[7]);
 }
 
-// FP16 leaf pass: per field the largest |value| of nrows rows of 64 fields
-// (one float4 of 4 fields per thread and row, contiguous reads), merged into
-// out[f] as float bits with atomicMax (non-negative floats order as their
-// bits).
-__global__ void field_max_kernel(const float4 *__restrict__ x, int64_t nrows, unsigned *__restrict__ out) {
+// FP16 leaf pass: per field the largest |value| of the weight rows (blockIdx.y
+// 0, out[f]) and of the potential rows (1, out[64 + f]): one float4 of 4 fields
+// per thread and row, contiguous reads, merged as float bits with atomicMax
+// (non-negative floats order as their bits).
+__global__ void field_max_kernel(const float4 *__restrict__ w, int64_t nw, const float4 *__restrict__ phi, int64_t np,
+                                 unsigned *__restrict__ out) {
     __shared__ float part[16][kF];
+    const float4 *x = blockIdx.y ? phi : w;
+    const int64_t nrows = blockIdx.y ? np : nw;
     const int c4 = threadIdx.x & 15;
     float m0 = 0.f, m1 = 0.f, m2 = 0.f, m3 = 0.f;
+#pragma unroll 4
     for (int64_t r = (int64_t)blockIdx.x * 16 + (threadIdx.x >> 4); r < nrows; r += (int64_t)gridDim.x * 16) {
         const float4 v = x[r * 16 + c4];
         m0 = fmaxf(m0, fabsf(v.x));
@@ -1563,56 +1574,50 @@ __global__ void field_max_kernel(const float4 *__restrict__ x, int64_t nrows, un
     if (threadIdx.x < kF) {
         float m = 0.f;
         for (int i = 0; i < 16; ++i) m = fmaxf(m, part[i][threadIdx.x]);
-        atomicMax(out + threadIdx.x, __float_as_uint(m));
+        atomicMax(out + blockIdx.y * kF + threadIdx.x, __float_as_uint(m));
     }
 }
 
 // FP16 hi/lo weight store: per unit of 8 store rows, the 64-field rows as
 // one 128-row FP16 tile (field f's hi part at row wrow(f, 0), lo at
 // wrow(f, 1); row m at byte (m / 8) 128 + (m % 8) 16, 8 halves), source
-// weights scaled by their field's power of two, potentials by theirs.  One
-// thread per (unit, 4 fields): float4 row loads, 64-byte row-group stores.
-__global__ void split_store16_kernel(const int32_t *__restrict__ bsrc, int64_t nu, const float *__restrict__ wF,
-                                     const float *__restrict__ phiF, const unsigned *__restrict__ fmax,
-                                     unsigned char *__restrict__ out) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nu * (kF / 4)) return;
-    const int64_t u = t / (kF / 4);
-    const int f0 = 4 * (int)(t % (kF / 4));
-    float sw[4], sp[4];
+// weights scaled by their field's power of two, potentials by theirs.  Bound by
+// memory: thread (unit, field) reads its field of the unit's rows (a warp: 128
+// contiguous bytes a row) and writes 16 bytes of hi and lo each beside its
+// neighbours'; kStoreUnits units a thread, for its two scales.  At 655,362
+// cells (0.96 GB) 255 -> 155 us: the eight rows' loads stood behind a branch
+// each (see store_row).
+constexpr int kStoreUnits = 4;
+__global__ void __launch_bounds__(256) split_store16_kernel(const int4 *__restrict__ bsrc, int64_t nu,
+                                                            const float *__restrict__ wF, const float *__restrict__ phiF,
+                                                            const unsigned *__restrict__ fmax,
+                                                            unsigned char *__restrict__ out) {
+    const int f = threadIdx.x & (kF - 1);
+    const int64_t u0 = ((int64_t)blockIdx.x * (256 / kF) + (threadIdx.x >> 6)) * kStoreUnits;
+    const float sw = f16_scale(__uint_as_float(fmax[f])), sp = f16_scale(__uint_as_float(fmax[kF + f]));
+    const int mh = wrow(f, 0), ml = wrow(f, 1);
+    const int oh = (mh >> 3) * 128 + (mh & 7) * 16, ol = (ml >> 3) * 128 + (ml & 7) * 16;
+#pragma unroll 2
+    for (int i = 0; i < kStoreUnits; ++i) {
+        const int64_t u = u0 + i;
+        if (u >= nu) return;
+        const int4 s0 = bsrc[2 * u], s1 = bsrc[2 * u + 1];
+        const int src[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+        float v[8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        sw[i] = f16_scale(__uint_as_float(fmax[f0 + i]));
-        sp[i] = f16_scale(__uint_as_float(fmax[kF + f0 + i]));
-    }
-    float v[4][8];   // [field][row]
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int32_t s = bsrc[u * 8 + r];
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float *sc = sw;
-        if (s >= 0) {
-            x = *reinterpret_cast<const float4 *>(wF + (size_t)s * kF + f0);
-        } else if (s <= -2) {
-            x = *reinterpret_cast<const float4 *>(phiF + (size_t)(-2 - s) * kF + f0);
-            sc = sp;
+        for (int r = 0; r < 8; ++r) {
+            const int s = src[r];
+            const float x = store_row(s, wF, phiF)[f] * (s >= 0 ? sw : sp);
+            v[r] = s == -1 ? 0.f : x;
         }
-        v[0][r] = x.x * sc[0];
-        v[1][r] = x.y * sc[1];
-        v[2][r] = x.z * sc[2];
-        v[3][r] = x.w * sc[3];
-    }
-    unsigned char *base = out + u * kW16UnitBytes;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
         uint4 hi, lo;
-        split_f16x2(v[i][0], v[i][1], hi.x, lo.x);
-        split_f16x2(v[i][2], v[i][3], hi.y, lo.y);
-        split_f16x2(v[i][4], v[i][5], hi.z, lo.z);
-        split_f16x2(v[i][6], v[i][7], hi.w, lo.w);
-        const int mh = wrow(f0 + i, 0), ml = wrow(f0 + i, 1);
-        *reinterpret_cast<uint4 *>(base + (mh >> 3) * 128 + (mh & 7) * 16) = hi;
-        *reinterpret_cast<uint4 *>(base + (ml >> 3) * 128 + (ml & 7) * 16) = lo;
+        split_f16x2(v[0], v[1], hi.x, lo.x);
+        split_f16x2(v[2], v[3], hi.y, lo.y);
+        split_f16x2(v[4], v[5], hi.z, lo.z);
+        split_f16x2(v[6], v[7], hi.w, lo.w);
+        unsigned char *base = out + u * kW16UnitBytes;
+        *reinterpret_cast<uint4 *>(base + oh) = hi;
+        *reinterpret_cast<uint4 *>(base + ol) = lo;
     }
 }
 
@@ -1814,20 +1819,18 @@ void launch_split_store(const int32_t *bsrc, int64_t k0, int64_t k1, const float
 }
 
 void launch_field_max(const float *wF, int64_t nw, const float *phiF, int64_t np, unsigned *fmax, cudaStream_t st) {
-    if (nw > 0)
-        field_max_kernel<<<(unsigned)std::min<int64_t>((nw + 15) / 16, 148 * 16), 256, 0, st>>>(
-            reinterpret_cast<const float4 *>(wF), nw, fmax);
-    if (np > 0)
-        field_max_kernel<<<(unsigned)std::min<int64_t>((np + 15) / 16, 148 * 16), 256, 0, st>>>(
-            reinterpret_cast<const float4 *>(phiF), np, fmax + kF);
+    const int64_t blocks = (std::max(nw, np) + 15) / 16;
+    if (blocks > 0)
+        field_max_kernel<<<dim3((unsigned)std::min<int64_t>(blocks, 148 * 8), 2), 256, 0, st>>>(
+            reinterpret_cast<const float4 *>(wF), nw, reinterpret_cast<const float4 *>(phiF), np, fmax);
 }
 
 void launch_split_store16(const int32_t *bsrc, int64_t nunits, const float *wF, const float *phiF,
                           const unsigned *fmax, void *bstore16, cudaStream_t st) {
     if (nunits <= 0) return;
-    const int64_t threads = nunits * (kF / 4);
-    split_store16_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(bsrc, nunits, wF, phiF, fmax,
-                                                                            static_cast<unsigned char *>(bstore16));
+    constexpr int64_t per = 256 / kF * kStoreUnits;   // units a block
+    split_store16_kernel<<<(unsigned)((nunits + per - 1) / per), 256, 0, st>>>(
+        reinterpret_cast<const int4 *>(bsrc), nunits, wF, phiF, fmax, static_cast<unsigned char *>(bstore16));
 }
 
 void launch_target_scales(const TcArgs &a, float *tscale, float *tinv, cudaStream_t st) {
