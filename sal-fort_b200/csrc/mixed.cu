@@ -40,8 +40,11 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
     return r;
 }
+// hi + lo, both rounded to nearest.  hi in two integer instructions (the
+// conversion takes about four): half a unit of the last kept bit added to the
+// magnitude, the rest cut off.  A NaN's hi may lose it, its lo keeps it.
 __device__ __forceinline__ void split_tf32(float x, uint32_t &hi, uint32_t &lo) {
-    hi = to_tf32(x);
+    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
     lo = to_tf32(x - __uint_as_float(hi));
 }
 // D = A * B + D, m16n8k8, TF32 inputs, FP32 accumulate (warp-wide).
@@ -83,12 +86,18 @@ __device__ __forceinline__ float val32(float mp) {
     return mp > 0.f ? v : 0.f;
 }
 
+// Sized for the field tiles it holds: with 32 fields three CTAs share an SM (the
+// buffers of 64 fields, 80 KB, allowed two: leaf pass at 163,842 cells x 24
+// fields 7.85 ms; with the integer rounding of split_tf32 6.22, with full groups
+// first 6.08.  Four CTAs in 128 registers, or the products of several
+// accumulators interleaved, changed nothing.)
+template <int NT>
 struct Smem {
-    // B tiles as copied, double-buffered: kS rows x FT floats each (sized for FT = 64)
-    float B[2][kS * 64];
+    // B tiles as copied, double-buffered: kS rows x FT floats each
+    float B[2][kS * 8 * NT];
     // the current item's B tile split into TF32 hi/lo, in mma fragment order:
     // [k-step][n-tile][lane] = (b0 hi, b1 hi, b0 lo, b1 lo)
-    float4 Bf[(kS / 8) * 8 * 32];
+    float4 Bf[(kS / 8) * NT * 32];
     double4 raw[2][kS];              // staged FP64 source coordinates
     float4 loc[kS];                  // sources relative to the group's centre (FP32)
     float fx[kMixRows][kMaxDegree + 1];  // BLI bases: of targets (leaf DOWN) or sources (upward)
@@ -103,7 +112,7 @@ __global__ void __launch_bounds__(kThr) mix_kernel(MixArgs a) {
     constexpr int NC = KIND == 0 ? 2 : (KIND == 1 ? 3 : 1);
     constexpr int FT = NT * 8;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+    Smem<NT> &sm = *reinterpret_cast<Smem<NT> *>(smem_raw);
     const MixGroup G = a.groups[blockIdx.x];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int n = a.d + 1, P = a.P;
@@ -432,7 +441,7 @@ __global__ void __launch_bounds__(kFinThreads) finalize_mix_kernel(const int32_t
 
 template <int KIND, int NT>
 static void launch_kind(const MixArgs &a, int ngroups, cudaStream_t st) {
-    const size_t smem = sizeof(Smem);
+    const size_t smem = sizeof(Smem<NT>);
     static std::atomic<unsigned long long> done{0};
     smem_attr_once((const void *)mix_kernel<KIND, NT>, (int)smem, done);
     mix_kernel<KIND, NT><<<ngroups, kThr, smem, st>>>(a);
@@ -464,8 +473,6 @@ void launch_finalize_mix(const int32_t *unit_beg, const float *partial, int nslo
     finalize_mix_kernel<<<dim3((unsigned)nslots, (unsigned)((per + kFinThreads - 1) / kFinThreads)), kFinThreads, 0, st>>>(
         unit_beg, reinterpret_cast<const float4 *>(partial), per, reinterpret_cast<float4 *>(dst));
 }
-
-size_t mix_smem_bytes() { return sizeof(Smem); }
 
 }  // namespace mix
 }  // namespace sal

@@ -46,7 +46,6 @@ void launch_prep_mix(const double *area, const double *ssh, int64_t ld, const in
                      int FT, float *wF, cudaStream_t st);
 void launch_finalize_mix(const int32_t *unit_beg, const float *partial, int nslots, int rows_per_slot, int FT,
                          float *dst, cudaStream_t st);
-size_t mix_smem_bytes();
 // tcgen05 leaf pass (64-field blocks), tc_leaf.cu
 struct TcArgs {
     const MixGroup *groups;   // leaf groups of <= 128 targets, pool order

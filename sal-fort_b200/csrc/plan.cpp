@@ -641,6 +641,9 @@ void plan_build_mix(const Tree &t, Plan *pl) {
                     pl->mix_leaf_groups.push_back(m);
                 }
             }
+            // the short groups (a leaf's last rows) fill in at the end
+            std::stable_sort(pl->mix_leaf_groups.begin(), pl->mix_leaf_groups.end(),
+                             [](const MixGroup &x, const MixGroup &y) { return (x.nt + 15) / 16 > (y.nt + 15) / 16; });
             pl->mix_proxy_groups.clear();
             pl->mix_proxy_items.clear();
             for (const Group &g : pl->proxy_groups) {
