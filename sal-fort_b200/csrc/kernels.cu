@@ -41,6 +41,7 @@ void launch_prep(const double4 *xyz, const double *area, const double *ssh, cons
 constexpr int kUpTile = 128;
 template <int N>
 __global__ void __launch_bounds__(64 * ((N + 2) / 3)) upward_kernel(UpArgs a) {
+    after_previous();
     constexpr int KB = (N + 2) / 3, T = 64 * KB, P = N * N, NS = N | 1;   // odd row strides: no bank conflicts
     __shared__ double fx[kUpTile][NS];
     __shared__ double fe[kUpTile][NS];
@@ -120,7 +121,7 @@ static_assert(kMaxDegree + 1 == 15, "the dispatch covers every degree");
 
 template <int N>
 static void launch_upward_n(const UpArgs &a, int nunits, cudaStream_t st) {
-    upward_kernel<N><<<nunits, 64 * ((N + 2) / 3), 0, st>>>(a);
+    launch_next(upward_kernel<N>, nunits, 64 * ((N + 2) / 3), 0, st, a);
 }
 
 void launch_upward(const UpArgs &a, int d, int nunits, cudaStream_t st) {
@@ -133,6 +134,7 @@ void launch_upward(const UpArgs &a, int d, int nunits, cudaStream_t st) {
 // mom6_fast_sum_module.f90:63-70 produces.
 __global__ void upward_finalize_kernel(const int32_t *__restrict__ unit_beg, const double *__restrict__ partial,
                                        int nslots, int d, int transposed, double4 *__restrict__ pool_proxy) {
+    after_previous();
     const int n = d + 1, P = n * n;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)nslots * P) return;
@@ -148,7 +150,7 @@ void launch_upward_finalize(const int32_t *unit_beg, const double *partial, int 
                             double4 *pool_proxy, cudaStream_t st) {
     long long tot = (long long)nslots * (d + 1) * (d + 1);
     if (tot <= 0) return;
-    upward_finalize_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(unit_beg, partial, nslots, d, transposed,
+    launch_next(upward_finalize_kernel, (unsigned)((tot + 255) / 256), 256, 0, st, unit_beg, partial, nslots, d, transposed,
                                                                           pool_proxy);
 }
 
@@ -181,6 +183,7 @@ constexpr int kEvalWarps = kEvalThreads / 32;
 
 template <int FORM>
 __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs a) {
+    after_previous();
     __shared__ __align__(128) double4 buf[kRing][kMaxStage];
     __shared__ __align__(8) uint64_t full[kRing], empty[kRing];
     __shared__ int abort_;
@@ -404,8 +407,8 @@ static_assert(kEvalThreads >= kMaxStage, "a thread per target at the end (leaves
 
 void launch_eval(int form, const EvalArgs &a, int nunits, cudaStream_t st) {
     if (nunits <= 0) return;
-    if (form == 0) eval_kernel<0><<<nunits, kEvalThreads, 0, st>>>(a);
-    else eval_kernel<1><<<nunits, kEvalThreads, 0, st>>>(a);
+    if (form == 0) launch_next(eval_kernel<0>, nunits, kEvalThreads, 0, st, a);
+    else launch_next(eval_kernel<1>, nunits, kEvalThreads, 0, st, a);
 }
 
 // ------------------------------------------------------------------ leaf ends
@@ -419,6 +422,7 @@ void launch_eval(int form, const EvalArgs &a, int nunits, cudaStream_t st) {
 constexpr int kFinThreads = 256, kFinSlots = 4;
 template <int N, int FORM>
 __global__ void __launch_bounds__(kFinThreads) leaf_fin_kernel(FinArgs a) {
+    after_previous();
     constexpr int P = N * N, R = P + (2 * N + 3) / 4;   // double4 per record
     __shared__ double4 rec[kFinSlots][R];
     __shared__ double red[3][kFinThreads];
@@ -497,8 +501,8 @@ __global__ void __launch_bounds__(kFinThreads) leaf_fin_kernel(FinArgs a) {
 
 template <int N>
 static void launch_leaf_fin_n(int form, const FinArgs &a, int nfin, cudaStream_t st) {
-    if (form == 0) leaf_fin_kernel<N, 0><<<nfin, kFinThreads, 0, st>>>(a);
-    else leaf_fin_kernel<N, 1><<<nfin, kFinThreads, 0, st>>>(a);
+    if (form == 0) launch_next(leaf_fin_kernel<N, 0>, nfin, kFinThreads, 0, st, a);
+    else launch_next(leaf_fin_kernel<N, 1>, nfin, kFinThreads, 0, st, a);
 }
 
 void launch_leaf_fin(int form, int d, const FinArgs &a, int nfin, cudaStream_t st) {
@@ -509,6 +513,7 @@ void launch_leaf_fin(int form, int d, const FinArgs &a, int nfin, cudaStream_t s
 // Sums each target slot's unit partials in unit order into its record.
 __global__ void proxy_finalize_kernel(const int32_t *__restrict__ unit_beg, const double4 *__restrict__ partial,
                                       int nslots, int P, int rec_stride, double *__restrict__ records) {
+    after_previous();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)nslots * P) return;
     const int s = (int)(t / P), p = (int)(t % P);
@@ -527,7 +532,7 @@ void launch_proxy_finalize(const int32_t *unit_beg, const double4 *partial, int 
                            double *records, cudaStream_t st) {
     long long tot = (long long)nslots * P;
     if (tot <= 0) return;
-    proxy_finalize_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(unit_beg, partial, nslots, P, rec_stride,
+    launch_next(proxy_finalize_kernel, (unsigned)((tot + 255) / 256), 256, 0, st, unit_beg, partial, nslots, P, rec_stride,
                                                                          records);
 }
 

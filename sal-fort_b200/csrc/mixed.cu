@@ -424,6 +424,7 @@ constexpr int kFinThreads = 256;
 __global__ void __launch_bounds__(kFinThreads) finalize_mix_kernel(const int32_t *__restrict__ unit_beg,
                                                                    const float4 *__restrict__ partial, int per,
                                                                    float4 *__restrict__ dst) {
+    dev::after_previous();
     const int s = blockIdx.x, rf = blockIdx.y * kFinThreads + threadIdx.x;
     if (rf >= per) return;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
@@ -470,7 +471,7 @@ void launch_finalize_mix(const int32_t *unit_beg, const float *partial, int nslo
                          float *dst, cudaStream_t st) {
     const int per = rows_per_slot * FT / 4;   // FT: 32 or 64
     if (nslots <= 0 || per <= 0) return;
-    finalize_mix_kernel<<<dim3((unsigned)nslots, (unsigned)((per + kFinThreads - 1) / kFinThreads)), kFinThreads, 0, st>>>(
+    dev::launch_next(finalize_mix_kernel, dim3((unsigned)nslots, (unsigned)((per + kFinThreads - 1) / kFinThreads)), kFinThreads, 0, st,
         unit_beg, reinterpret_cast<const float4 *>(partial), per, reinterpret_cast<float4 *>(dst));
 }
 

@@ -633,6 +633,7 @@ struct ItemWindow {
 // producers only write the outputs of groups without sources.
 template <int MODE, bool JOINT, bool F16, int TS = 0>
 __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_constant__ TcJoint J, int *err) {
+    dev::after_previous();
     static_assert(!F16 || MODE == 0, "FP16 operands in the leaf pass only");
     static_assert(TS == 0 || (MODE == 0 && F16 && !JOINT), "kernel-tile store: FP16 leaf pass of one grid");
     constexpr int SK = F16 ? kStageKF16 : kStageK;   // sources per stage
@@ -1527,6 +1528,7 @@ __device__ __forceinline__ const float *store_row(int32_t s, const float *wF, co
 // (k-step, field).
 __global__ void split_store_kernel(const int32_t *__restrict__ bsrc, int64_t nk, const float *__restrict__ wF,
                                    const float *__restrict__ phiF, float *__restrict__ bstore) {
+    dev::after_previous();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nk * kF) return;
     const int64_t ks = t / kF;
@@ -1553,6 +1555,7 @@ __global__ void split_store_kernel(const int32_t *__restrict__ bsrc, int64_t nk,
 // (non-negative floats order as their bits).
 __global__ void field_max_kernel(const float4 *__restrict__ w, int64_t nw, const float4 *__restrict__ phi, int64_t np,
                                  unsigned *__restrict__ out) {
+    dev::after_previous();
     __shared__ float part[16][kF];
     const float4 *x = blockIdx.y ? phi : w;
     const int64_t nrows = blockIdx.y ? np : nw;
@@ -1592,6 +1595,7 @@ __global__ void __launch_bounds__(256) split_store16_kernel(const int4 *__restri
                                                             const float *__restrict__ wF, const float *__restrict__ phiF,
                                                             const unsigned *__restrict__ fmax,
                                                             unsigned char *__restrict__ out) {
+    dev::after_previous();
     const int f = threadIdx.x & (kF - 1);
     const int64_t u0 = ((int64_t)blockIdx.x * (256 / kF) + (threadIdx.x >> 6)) * kStoreUnits;
     const float sw = f16_scale(__uint_as_float(fmax[f])), sp = f16_scale(__uint_as_float(fmax[kF + f]));
@@ -1766,7 +1770,8 @@ static void launch_tc(const TcJoint &J, int nsm, int cta_groups, int *err, cudaS
     const int per = cta_groups > 0 ? cta_groups : 1;
     int grid = (total + per - 1) / per;
     if (grid < nsm) grid = total < nsm ? total : nsm;
-    tc_leaf_kernel<MODE, JOINT, F16, TS><<<grid, kThreads, smem, st>>>(J, err);
+    if constexpr (JOINT) tc_leaf_kernel<MODE, JOINT, F16, TS><<<grid, kThreads, smem, st>>>(J, err);
+    else dev::launch_next(tc_leaf_kernel<MODE, JOINT, F16, TS>, grid, kThreads, smem, st, J, err);
 }
 
 template <int MODE, bool F16 = false, int TS = 0>
@@ -1814,7 +1819,7 @@ void launch_split_store(const int32_t *bsrc, int64_t k0, int64_t k1, const float
     const int64_t nk = k1 - k0;
     if (nk <= 0) return;
     const int64_t threads = nk * kF;
-    split_store_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(bsrc + k0 * 8, nk, wF, phiF,
+    dev::launch_next(split_store_kernel, (unsigned)((threads + 255) / 256), 256, 0, st, bsrc + k0 * 8, nk, wF, phiF,
                                                                           bstore + k0 * kWStepFloats);
 }
 
@@ -1829,8 +1834,8 @@ void launch_split_store16(const int32_t *bsrc, int64_t nunits, const float *wF, 
                           const unsigned *fmax, void *bstore16, cudaStream_t st) {
     if (nunits <= 0) return;
     constexpr int64_t per = 256 / kF * kStoreUnits;   // units a block
-    split_store16_kernel<<<(unsigned)((nunits + per - 1) / per), 256, 0, st>>>(
-        reinterpret_cast<const int4 *>(bsrc), nunits, wF, phiF, fmax, static_cast<unsigned char *>(bstore16));
+    dev::launch_next(split_store16_kernel, (unsigned)((nunits + per - 1) / per), 256, 0, st,
+                     reinterpret_cast<const int4 *>(bsrc), nunits, wF, phiF, fmax, static_cast<unsigned char *>(bstore16));
 }
 
 void launch_target_scales(const TcArgs &a, float *tscale, float *tinv, cudaStream_t st) {

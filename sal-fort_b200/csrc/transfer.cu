@@ -66,6 +66,7 @@ __device__ __forceinline__ float4 add4(float4 a, float4 b) {
 template <int N>
 __global__ void __launch_bounds__(kQ * N) m2m_kernel(const int32_t *__restrict__ tasks, const double *__restrict__ H,
                                                      float4 *__restrict__ w) {
+    dev::after_previous();
     constexpr int P = N * N;
     extern __shared__ __align__(16) float smf[];
     float4 *T = reinterpret_cast<float4 *>(smf);   // two tiles, children in turn
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(kQ * N) m2m_kernel(const int32_t *__restrict__
 template <int N>
 __global__ void __launch_bounds__(kQ * N) l2l_kernel(const int32_t *__restrict__ tasks, const double *__restrict__ H,
                                                      float4 *__restrict__ phi) {
+    dev::after_previous();
     constexpr int P = N * N;
     extern __shared__ __align__(16) float smf[];
     float4 *T = reinterpret_cast<float4 *>(smf);
@@ -174,14 +176,14 @@ template <int N>
 static void launch_m2m_n(const int32_t *tasks, int ntasks, const double *H, float *w, cudaStream_t st) {
     static std::atomic<unsigned long long> done{0};
     smem_attr_once((const void *)m2m_kernel<N>, (int)transfer_smem<N>(2), done);
-    m2m_kernel<N><<<ntasks, kQ * N, transfer_smem<N>(2), st>>>(tasks, H, reinterpret_cast<float4 *>(w));
+    dev::launch_next(m2m_kernel<N>, ntasks, kQ * N, transfer_smem<N>(2), st, tasks, H, reinterpret_cast<float4 *>(w));
 }
 
 template <int N>
 static void launch_l2l_n(const int32_t *tasks, int ntasks, const double *H, float *phi, cudaStream_t st) {
     static std::atomic<unsigned long long> done{0};
     smem_attr_once((const void *)l2l_kernel<N>, (int)transfer_smem<N>(1), done);
-    l2l_kernel<N><<<3 * ntasks, kQ * N, transfer_smem<N>(1), st>>>(tasks, H, reinterpret_cast<float4 *>(phi));
+    dev::launch_next(l2l_kernel<N>, 3 * ntasks, kQ * N, transfer_smem<N>(1), st, tasks, H, reinterpret_cast<float4 *>(phi));
 }
 
 // N = d + 1 from 2 to kMaxTreeDegree + 1 (the plan turns the tree passes off
