@@ -7,7 +7,7 @@
 // pass is described below.
 //
 // One CTA per SM at a time, each walking leaf groups of up to 128 targets
-// in pool order with a stride of the grid size.  A group's work is a list of
+// (fuller ones first) with a stride of the grid size.  A group's work is a list of
 // items (<= 64 sources, or <= 64 Cartesian rows of a DOWN interpolation), cut
 // into stages of 32 K columns (four k-steps of 8).  The contraction is
 //     D[field part, target component] += W[field part, k] * T[k, target component]
@@ -21,14 +21,14 @@
 // (207 in this kernel, whatever N: half of the MMA warp's time).  Elected
 // issue and narrow groups: leaf pass 34.9 -> 33.5 ms at 2.3M cells x 64
 // fields, where the producers' tile arithmetic is what the MMA warp then waits
-// for.
+// for; with waits that suspend, records, teams and the plan's DOWN bases 26.6.
 // Warp roles:
 //   warps 0-7   producers.  A task is one k-step of a 32-target row block:
 //               8 kernel-tile entries per component and row in FP32, split
 //               into TF32 hi + lo, stored to shared memory in the canonical
-//               K-major layout (the MMA's B operand).  A stage's tasks are
-//               dealt so that small groups use every warp (see the producer
-//               branch).  The self pair enters as the tile's diagonal entry:
+//               K-major layout (the MMA's B operand).  Two teams of four
+//               warps take the stages in turn, a stage's tasks dealt so that
+//               small groups use every warp (see the producer branch).  The self pair enters as the tile's diagonal entry:
 //               the reference kernel's FP64 value at distance zero (rounding
 //               noise).  The sources' FP32 coordinates (per k-step x[8] y[8]
 //               z[8]) come from shared memory, copied there by the loader.
