@@ -5,6 +5,7 @@
 // a few bytes against ~60 FP64 operations.
 #include <cuda_runtime.h>
 
+#include "eval_cut.hpp"
 #include "kernels.cuh"
 
 namespace sal {
@@ -178,8 +179,9 @@ void launch_upward_finalize(const int32_t *unit_beg, const double *partial, int 
 // about 2.5 cycles of a scheduler's pipe (50 for a far pair's 20, in a loop of
 // nothing else), and 8 pairs at a time on 4 warps a scheduler come closest to
 // that (24 warps of 80 registers and 4 pairs: 3 % slower).
-constexpr int kEvalThreads = 256, kEvalCtas = 2, kIlp = 8, kNearIlp = 4, kRing = 4, kAhead = 2, kSlots = 2;
-constexpr int kEvalWarps = kEvalThreads / 32;
+constexpr int kEvalThreads = 256, kEvalCtas = 2, kIlp = 8, kNearIlp = 4, kRing = 4, kAhead = 2;
+constexpr int kSlots = kEvalSlots;
+static_assert(kEvalWarps == kEvalThreads / 32, "eval_cut.hpp deals to the warps of a CTA");
 
 template <int FORM>
 __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs a) {
@@ -195,36 +197,20 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs 
     const int ns = se - sb;
     const uint32_t polls = a.polls ? a.polls : kDefaultPolls;
     const int nissue = (a.skip_last && !U.proxy) ? ns - 1 : ns;
-    // chunks of 32 (target, residue) lanes; the last one's weight is 1 / (its
-    // residues side by side)
-    const int F = U.fold, nid = U.nt * F, nch = (nid + 31) >> 5, nlast = nid - 32 * (nch - 1), rlast = 32 / nlast;
-    const float wlast = 1.f / (float)rlast, per = ((float)(nch - 1) + wlast) * (1.f / kEvalWarps);
-    // this warp's run of the plane
-    const float lo = per * (float)warp, hi = per * (float)(warp + 1);
-    const int c0 = min((int)lo, nch - 1);
+    const EvalCut cut(U.nt, U.fold);
     // the slots' state; a stage's range takes one slot into registers
     struct Slot {
         double x, y, z;            // the target
         double A[3], ax, ay;       // sums: far pairs Sum val w s (Cartesian proxies Sum val w (s - x)); near pairs
-        float f0, f1, rstep;       // this run's fraction of the chunk's sources, 1 / step
-        int ti, res, step, work;   // target, residue and modulus of its sources
+        EvalShare sh;              // the lane's sources
+        bool work;
     } slot[kSlots];
 #pragma unroll 1
     for (int i = 0; i < kSlots; ++i) {
-        const int c = c0 + i;
-        const bool last = c == nch - 1;
-        const int n = last ? nlast : 32, l = lane % n, id = 32 * c + l;
-        const float base = (float)c, wc = last ? wlast : 1.f;
         Slot w{};
-        w.step = last ? F * rlast : F;
-        w.rstep = 1.f / (float)w.step;
-        w.ti = id % U.nt;
-        w.res = id / U.nt + F * (lane / n);
-        // neighbouring warps compute a shared boundary from the same numbers
-        w.f0 = lo <= base ? 0.f : fminf((lo - base) / wc, 1.f);
-        w.f1 = (warp == kEvalWarps - 1 || hi >= base + wc) ? 1.f : fmaxf((hi - base) / wc, 0.f);
-        if (c < nch && w.res < w.step && w.f0 < w.f1) {
-            const double4 q = U.proxy ? a.tgt_proxy[(size_t)U.tgt * a.P + w.ti] : a.pool[U.tgt + w.ti];
+        w.sh = eval_share(cut, warp, lane, i);
+        if (w.sh.work) {
+            const double4 q = U.proxy ? a.tgt_proxy[(size_t)U.tgt * a.P + w.sh.ti] : a.pool[U.tgt + w.sh.ti];
             w.x = q.x;
             w.y = q.y;
             w.z = q.z;
@@ -276,9 +262,8 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs 
         for (int i = 0; i < kSlots; ++i) {
             if (!slot[i].work) continue;
             const double x = slot[i].x, y = slot[i].y, z = slot[i].z;
-            const float f0 = slot[i].f0, f1 = slot[i].f1;
-            const int res = slot[i].res, step = slot[i].step, ti = slot[i].ti;
-            const float rstep = slot[i].rstep;
+            const EvalShare sh = slot[i].sh;
+            const int step = sh.step;
             double A[3] = {slot[i].A[0], slot[i].A[1], slot[i].A[2]}, ax = slot[i].ax, ay = slot[i].ay;
             // an unmasked stage is one run of sources, a masked one a run per item
 #pragma unroll 1
@@ -286,14 +271,15 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs 
                 int beg = 0, n = S.cnt;
                 if (masked) {
                     const EvalItem it = a.items[v];
-                    if (!((a.masks[it.mask + (ti >> 5)] >> (ti & 31)) & 1u)) continue;
+                    if (!((a.masks[it.mask + (sh.ti >> 5)] >> (sh.ti & 31)) & 1u)) continue;
                     beg = it.dst;
                     n = it.cnt;
                 }
                 // this run's share of the blocks of `step` sources
-                const float nb = floorf(((float)(n + step) - 0.5f) * rstep);   // ceil(n / step), exact for n <= 256
-                int s = beg + (int)(nb * f0) * step + res;
-                const int e = min(beg + (int)(nb * f1) * step, beg + n);
+                int s, e;
+                sh.sources(n, s, e);
+                s += beg;
+                e += beg;
                 if (cart) {
                     for (; s + (kNearIlp - 1) * step < e; s += kNearIlp * step)
                         cart_pairs<kNearIlp>(x, y, z, src + s, step, A);
@@ -362,10 +348,10 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs 
     // order; then each target's F lanes, in order
     double *fold = red + 3 * 32 * kSlots * kEvalWarps;
     double rx = 0.0, ry = 0.0, rz = 0.0;
-    if (tid < nid) {
-        const int c = tid >> 5, n = c == nch - 1 ? nlast : 32, r = c == nch - 1 ? rlast : 1;
+    if (tid < cut.nid) {
+        const int c = tid >> 5, n = c == cut.nch - 1 ? cut.nlast : 32, r = c == cut.nch - 1 ? cut.rlast : 1;
         for (int v = 0; v < kEvalWarps; ++v) {
-            const int i = c - min((int)(per * (float)v), nch - 1);
+            const int i = cut.slot_of(v, c);
             if (i < 0 || i >= kSlots) continue;
             const double *o = red + ((v * kSlots + i) * 3) * 32 + lane;
             for (int k = 0; k < r; ++k) {
@@ -375,13 +361,13 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs 
             }
         }
     }
-    if (F > 1) {
+    if (U.fold > 1) {
         fold[tid] = rx;
         fold[kEvalThreads + tid] = ry;
         fold[2 * kEvalThreads + tid] = rz;
         __syncthreads();
         if (tid < U.nt)
-            for (int id = tid + U.nt; id < nid; id += U.nt) {
+            for (int id = tid + U.nt; id < cut.nid; id += U.nt) {
                 rx += fold[id];
                 ry += fold[kEvalThreads + id];
                 rz += fold[2 * kEvalThreads + id];
@@ -401,7 +387,6 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs 
 }
 static_assert(sizeof(double) * 3 * (kSlots + 1) * kEvalThreads <= sizeof(double4) * kRing * kMaxStage,
               "the warps' sums and the folded lanes' fit the ring");
-static_assert(kEvalMaxChunks <= kEvalWarps && kSlots == 2, "a warp's run is a chunk at most: it meets two");
 static_assert(32 * kEvalMaxChunks <= kEvalThreads, "a thread per lane of the folded set");
 static_assert(kEvalThreads >= kMaxStage, "a thread per target at the end (leaves and proxy sets hold at most 256)");
 

@@ -23,6 +23,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "eval_cut.hpp"
 #include "sal_internal.hpp"
 
 namespace sal {
@@ -156,24 +157,6 @@ struct EvalBounds {
 // 3,000 cells).
 static constexpr double kEvalUnits = 8.0 * 2 * 148, kEvalMinPairs = 32768.0;
 static constexpr double kEvalNearCost = 1.35;   // a near pair's cost in far pairs
-
-// How often a set of nt targets is taken (EvalUnit::fold): the number that
-// leaves the fewest idle lanes in chunks of 32, up to one chunk a warp (81
-// proxies: 3 x 81 lanes fill 8 chunks to 95 %, 84 % unfolded).  More chunks
-// than warps were no faster at 2.3M cells (148 targets in 19 chunks: 19.9 ms
-// for the leaf units, as unfolded): what the lanes gain, the state that a warp
-// swaps per chunk and stage takes back.
-static int32_t eval_fold(int32_t nt) {
-    int32_t best = 1;
-    double least = 1e30;
-    for (int32_t f = 1; f <= 8; ++f) {
-        const int32_t nid = nt * f, nch = (nid + 31) / 32, nlast = nid - 32 * (nch - 1);
-        if (nch > kEvalMaxChunks && f > 1) break;
-        const double c = (nch - 1 + 1.0 / (32 / nlast)) * 32.0 / nid;   // the last chunk takes 32 / nlast residues at once
-        if (c < least - 1e-12) { least = c; best = f; }
-    }
-    return best;
-}
 
 static void plan_build_eval(const Tree &t, const EvalBounds &bd, const std::vector<std::vector<EvalSrc>> &lsrc,
                             const std::vector<std::vector<EvalSrc>> &tsrc,

@@ -98,7 +98,6 @@ struct EvalUnit {
     int32_t proxy;       // 1: proxy targets
     int32_t fold;        // the targets are taken this often, each time for one residue of the sources
 };
-constexpr int kEvalMaxChunks = 8;   // chunks of 32 lanes of a folded target set (one a warp; 256 targets fill 8 unfolded)
 struct LeafFin {         // a leaf's end: partial sums of `parts` units, then DOWN interpolation from its slots
     int32_t tgt, nt, part, parts, db, de;
 };
