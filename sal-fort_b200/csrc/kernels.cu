@@ -3,6 +3,7 @@
 // All passes are compute-bound on the FP64 pipe: every staged source tile is
 // reused by every target of its group (up to 256), so HBM traffic per pair is
 // a few bytes against ~60 FP64 operations.
+#include <cmath>
 #include <cuda_runtime.h>
 
 #include "eval_cut.hpp"
@@ -183,6 +184,39 @@ constexpr int kEvalThreads = 256, kEvalCtas = 2, kIlp = 8, kNearIlp = 4, kRing =
 constexpr int kSlots = kEvalSlots;
 static_assert(kEvalWarps == kEvalThreads / 32, "eval_cut.hpp deals to the warps of a CTA");
 
+// The far pairs of one lane once more, pair by pair as the near ones: for sums
+// that are not finite.  The vector of gref_far turns an infinite weight, or one
+// whose products overflow, into NaN at its projection, where the pair itself is
+// a signed infinity or finite.  From the pool, nothing staged; a sum that is NaN
+// already (a NaN weight) stays so and ends it.
+__device__ __noinline__ void far_again(const double4 *pool, const EvalStage *stages, const EvalItem *items,
+                                       const uint32_t *masks, int sb, int se, const EvalShare &sh, double x, double y,
+                                       double z, double &ax, double &ay) {
+    Tgt T;
+    T.x = x;
+    T.y = y;
+    T.z = z;
+    T.omx32 = tgt_omx32(z);
+    for (int k = sb; k < se; ++k) {
+        const EvalStage S = stages[k];
+        if (S.flags & kEvalNear) continue;
+        int s = 0, e = 0;
+        for (int v = S.ib; v < S.ie; ++v) {
+            const EvalItem it = items[v];
+            if (S.flags & kEvalMasked) {
+                if (!((masks[it.mask + (sh.ti >> 5)] >> (sh.ti & 31)) & 1u)) continue;
+                sh.sources(it.cnt, s, e);
+                s += it.dst;
+                e += it.dst;
+            } else if (v == S.ib) {
+                sh.sources(S.cnt, s, e);
+            }
+            for (; s < min(e, it.dst + it.cnt); s += sh.step) gref_near<1>(T, pool + it.off + (s - it.dst), 1, ax, ay);
+        }
+        if (ax != ax && ay != ay) return;
+    }
+}
+
 template <int FORM>
 __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs a) {
     after_previous();
@@ -319,13 +353,17 @@ __global__ void __launch_bounds__(kEvalThreads, kEvalCtas) eval_kernel(EvalArgs 
         // the kernel's constant; leaves and reference proxies: the projection
         // of the far pairs' vector and the target factor 1/sqrt(1 - tz^2)
         // (zero inside the pole guard, and in slots without work)
-        const Slot &w = slot[i];
+        Slot &w = slot[i];
         double rx = 0.0, ry = 0.0, rz = 0.0;
         if (cart) {
             rx = kCons * w.A[0];
             ry = kCons * w.A[1];
             rz = kCons * w.A[2];
         } else if (w.work) {
+            if (!(fabs(w.A[0]) + fabs(w.A[1]) + fabs(w.A[2]) < INFINITY)) {
+                w.A[0] = w.A[1] = w.A[2] = 0.0;
+                far_again(a.pool, a.stages, a.items, a.masks, sb, se, w.sh, w.x, w.y, w.z, w.ax, w.ay);
+            }
             Tgt T;
             tgt_init(T, w.x, w.y, w.z);
             const double tf = kCons * T.inv_mp2;

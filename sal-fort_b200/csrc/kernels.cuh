@@ -215,9 +215,8 @@ __device__ __forceinline__ double val_chord(double mp, double w) {
     const double n = fma(-2.0 * kC2, mp, fma(kC1 - 2.0 * kC2, q, 2.0 * kC1));
     const double t = fma(2.0, q, mp);
     const double d = kReg ? fma(mp, t, fma(1e-16 * (1.0 + 2.0 * kC2 / kC1), q, 2e-16)) : mp * t;
-    const double r = rcp_seed(d), e = fma(-d, r, 1.0);
-    const double u = n * w * r;
-    return fma(u, fma(e, e, e), u);
+    const double r = rcp_seed(d), e = fma(-d, r, 1.0), u = n * r;
+    return fma(u, fma(e, e, e), u) * w;   // w last: an infinite one gives a signed infinity
 }
 
 // Where val_chord<true> stands for the reference's expressions: q >= 1e-3
