@@ -207,7 +207,10 @@ int sal_grid_sync(sal_grid *g, void *stream);
  * the reference).  polls > 0: in the next FP64 solve on the grid, the leaf
  * pass leaves the last staging copy of every target group unissued and bounds
  * each staging wait to `polls` polls, so every group's last wait runs out
- * with no copy in flight.  That solve's outputs are undefined, and the next
+ * with no copy in flight; or, if a batched solve in 64-field blocks comes
+ * first, the leaf pass of its first block leaves all but the first staging copy
+ * of every CTA unissued, and its waits run out at their own limit (2 s, the
+ * CTAs side by side).  That solve's outputs are undefined, and the next
  * sal_grid_sync (or the host entry point that ran the solve) returns
  * SAL_ETIMEOUT and clears the flag; later solves are unaffected.  polls = 0
  * cancels a pending injection. */

@@ -130,7 +130,7 @@ struct GridImpl {
     std::vector<GraphShape> seen;     // shapes solved once: captured on their second solve
     std::mutex graph_mu;              // guards use_graphs, graphs and seen
     double *h_w = nullptr;                                        // device, P*npanels
-    uint32_t inject_polls = 0;        // sal_grid_inject_timeout: applies to the next FP64 solve
+    uint32_t inject_polls = 0;        // sal_grid_inject_timeout: applies to the next FP64 solve or 64-field leaf pass
     std::vector<void *> allocs;
     std::mutex mu;
     // optional per-pass timers: events recorded on the launching stream
@@ -848,7 +848,12 @@ static void solve_mixed_block(GridImpl &g, const double *ssh, int64_t ld_ssh, in
         // later ones (stream-ordered after it) replay them: all of them (2), or
         // one item in tile_store beside the producers' (3)
         const int tiles = g.ktile ? (!g.tile_recorded ? 1 : pl.tc_opt.tile_store > 1 ? 3 : 2) : 0;
-        mix::launch_tc_leaf(leaf_args(g, ox, oy, ld_out, f0, nf), g.nsm, cg, g.err, st, tiles);
+        mix::TcArgs t = leaf_args(g, ox, oy, ld_out, f0, nf);
+        if (g.inject_polls) {
+            t.inject = 2;
+            g.inject_polls = 0;
+        }
+        mix::launch_tc_leaf(t, g.nsm, cg, g.err, st, tiles);
         if (tiles == 1) g.tile_recorded = true;
     } else {
         a.groups = g.mix_leaf_groups;

@@ -48,7 +48,7 @@ void launch_finalize_mix(const int32_t *unit_beg, const float *partial, int nslo
                          float *dst, cudaStream_t st);
 // tcgen05 leaf pass (64-field blocks), tc_leaf.cu
 struct TcArgs {
-    const MixGroup *groups;   // leaf groups of <= 128 targets, pool order
+    const MixGroup *groups;   // leaf groups of <= 128 targets, more row blocks first, else pool order
     int ngroups;
     const TcItem *items;
     const float *sxyz;        // per source k-step of the split store: x[8], y[8], z[8] relative to the panel centre
@@ -79,6 +79,7 @@ struct TcArgs {
     unsigned char *ktile;
     const int64_t *ktile_off;
     int tile_every;
+    uint32_t inject;          // test hook: > 0 leaves every CTA's stages from inject - 1 on uncopied
 };
 // cta_groups: groups one CTA walks at most (the grid has every SM busy
 // otherwise)

@@ -148,12 +148,16 @@ struct TcSmem {
     float fx[kReplay ? 1 : kTcRows][kMaxDegree + 1];              // per target row: BLI bases in the current DOWN slot
     float fe[kReplay ? 1 : kTcRows][kMaxDegree + 1];
     int kmap[kReplay ? 1 : kKmap];
-    // FP16 computing launches, per weight stage, its item as the loader saw it:
-    // (dx, dy, dz, flags: kRec*) and (off, row0)
     alignas(16) float cs[kTcRows];                                // folds: the group's column scales (DOWN chains)
+    // computing launches, per weight stage, its item as the loader saw it: (dx,
+    // dy, dz, flags: kRec*) and (off, row0)
     float4 rec[kReplay ? 1 : kWStages];
     int2 rec2[kReplay ? 1 : kWStages];
     uint32_t toff[KS], tlen[KS], woff[KS], wlen[KS];             // replay: each stage slot's ranges in the rings
+    // partial replay: the copies of a slot's tiles, and the parity of the slot's
+    // last one (+ 2: there was one)
+    uint64_t kcopy[kKStages];
+    uint32_t clast[kKStages];
     uint64_t kfull[KS], kempty[KS], wfull[WS], wempty[WS], accfull, accfree, fin;
     uint32_t tmem_base;
     int abort;
@@ -227,6 +231,12 @@ __device__ __forceinline__ bool wait_bounded(uint64_t *bar, uint32_t parity, vol
     atomicExch(err, dev::kErrTimeout);
     return false;
 }
+// The same for a warp that keeps a failure: the usual case, a phase that is
+// complete, touches nothing but the barrier.
+__device__ __forceinline__ void wait_or_die(uint64_t *bar, uint32_t parity, volatile int *abort, int *err, bool &dead) {
+    if (dev::mbar_try_wait(bar, parity)) return;
+    if (!wait_bounded(bar, parity, abort, err)) dead = true;
+}
 // Bounded wait that ignores the abort flag (drains copies and MMAs in flight
 // before the CTA exits).
 __device__ __forceinline__ void wait_drain(uint64_t *bar, uint32_t parity, int *err) {
@@ -238,10 +248,10 @@ __device__ __forceinline__ void wait_drain(uint64_t *bar, uint32_t parity, int *
     atomicExch(err, dev::kErrTimeout);
 }
 
-// Named barrier 1 over the producer warps.
 __device__ __forceinline__ void mbar_arrive_n(uint64_t *bar, uint32_t n) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(n) : "memory");
 }
+// Named barrier 1 over the producer warps.
 __device__ __forceinline__ void producers_sync(int threads) { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -670,6 +680,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             dev::mbar_init(&sm.wfull[j], 1);
             dev::mbar_init(&sm.wempty[j], 1);
         }
+        for (int j = 0; j < kKStages; ++j) {
+            dev::mbar_init(&sm.kcopy[j], 1);
+            sm.clast[j] = 0;
+        }
         dev::mbar_init(&sm.accfull, 1);
         // replay: the idle producer warps fold too, three warps per lane quarter
         dev::mbar_init(&sm.accfree, TS == 2 ? kFoldWarps + kProdWarps : kFoldWarps);
@@ -694,6 +708,13 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
     tc_fence_after();
     const uint32_t tmem = sm.tmem_base;
     uint32_t st = 0;   // stages this CTA has gone through
+    // Set by a producer or MMA warp's first wait that gave up, and kept: from then
+    // on it uses no stage's buffers and signals no stage (the abort flag ends the
+    // others' waits).  Beyond a stage that was never issued the barriers' parities
+    // mean nothing (a slot that missed a lap looks full), and an arrival out of
+    // turn, a team's for two among DOWN stages' for one, can take a barrier's count
+    // below zero, which is a fault.
+    bool dead = false;
 
     if (TS != 2 && warp < kProdWarps) {
         // ============================================================ producers
@@ -710,7 +731,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
         // relative to their panel's centre) arrive in shared memory with the
         // stage's weights: the loader warp copies them up to WS stages
         // ahead, so no global-memory latency sits in a producer task.
-
+        uint32_t cpar = 0;   // partial replay: per slot, the parity of its next copy
         for (int gi = blockIdx.x; gi < total; gi += gridDim.x) {
             const int gk = grid_of(gi);
             const TcArgs &a = J.g[gk];
@@ -786,6 +807,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     const bool down = k >= ni - ndown;
                     // an item the kernel-tile store holds (one in tile_every)
                     const bool stored = (TS == 1 || TS == 3) && k % a.tile_every == a.tile_every - 1;
+                    const uint32_t cpar_st = (cpar >> (st % KS)) & 1;   // its copy's phase of kcopy
+                    if (TS == 3 && stored) cpar ^= 1u << (st % KS);
                     if (!down && (st & 1) != (uint32_t)team) {
                         if (stored) gtile += (size_t)4 * ((((a.items[G.ib + k].cnt + 7) >> 3) + 1) >> 1) * cb;
                         continue;
@@ -793,29 +816,26 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     const uint32_t arrivals = down ? 1 : 2;
                     const uint32_t slot = st % KS, kpar = ((st / KS) - 1) & 1, jb = st % WS;
                     bool slot_free = st < (uint32_t)KS;
-                    const bool ok = wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err);
+                    wait_or_die(&sm.wfull[jb], (st / WS) & 1, abort, err, dead);
                     const float4 rec = sm.rec[jb];
-                    const int flags = ok ? __float_as_int(rec.w) : 0, nks = flags & kRecUnits;
+                    const int flags = dead ? 0 : __float_as_int(rec.w), nks = flags & kRecUnits;
                     if (TS == 3 && stored) {
                         // replay: the stage's first warp copies its chunks (MMA step
                         // q / 4, hi / lo, east / north) into the ring slot once the MMAs
-                        // that last read it are done; its arrival carries the bytes
+                        // that last read it are done, on a barrier of the copies' own
                         const int nq = 4 * ((nks + 1) >> 1);
-                        if (!slot_free) wait_bounded(&sm.kempty[slot], kpar, abort, err);
-                        if (down ? warp == 0 : tw == 0) {
-                            if (lane == 0) {
-                                dev::mbar_expect_tx(&sm.kfull[slot], (uint32_t)(nq * cb));
-                                if (!down) mbar_arrive(&sm.kfull[slot]);
-                            }
+                        if (!slot_free) wait_or_die(&sm.kempty[slot], kpar, abort, err, dead);
+                        if ((down ? warp == 0 : tw == 0) && __all_sync(0xffffffffu, !dead)) {
+                            if (lane == 0) dev::mbar_expect_tx(&sm.kcopy[slot], (uint32_t)(nq * cb));
                             __syncwarp();
-                            if (lane < nq && !*abort)
+                            if (lane < nq)
                                 dev::bulk_g2s_hint(
                                     reinterpret_cast<unsigned char *>(sm.Kt(slot, lane >> 2, (lane >> 1) & 1)) + (lane & 1) * cb,
-                                    gtile + (size_t)lane * cb, (uint32_t)cb, &sm.kfull[slot], dev::l2_evict_first());
-                        } else if (lane == 0) {
-                            mbar_arrive_n(&sm.kfull[slot], arrivals);
+                                    gtile + (size_t)lane * cb, (uint32_t)cb, &sm.kcopy[slot], dev::l2_evict_first());
+                            if (lane == 0) sm.clast[slot] = 2u | cpar_st;
                         }
                         __syncwarp();
+                        if (lane == 0 && !dead) mbar_arrive_n(&sm.kfull[slot], arrivals);
                         gtile += (size_t)nq * cb;
                         continue;
                     }
@@ -873,7 +893,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     // the MMAs that last read the slot must be done before the first
                     // store into it
                     auto claim = [&]() {
-                        if (!slot_free) wait_bounded(&sm.kempty[slot], kpar, abort, err);
+                        if (!slot_free) wait_or_die(&sm.kempty[slot], kpar, abort, err, dead);
                         slot_free = true;
                     };
                     // units: a team's warp w takes row block w (w % 2, 0), units i (w / 2
@@ -988,7 +1008,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     claim();
                     dev::fence_proxy_async();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_n(&sm.kfull[slot], arrivals);
+                    if (lane == 0 && !dead) mbar_arrive_n(&sm.kfull[slot], arrivals);
                     if (TS == 1 && stored) gtile += (size_t)4 * ((nks + 1) >> 1) * cb;
                 }
                 continue;
@@ -1035,13 +1055,13 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                 if (!down && (st & 1) != (uint32_t)team) continue;
                 const uint32_t slot = st % KS, kpar = ((st / KS) - 1) & 1, jb = st % WS;
                 bool slot_free = st < (uint32_t)KS;
-                const bool ok = wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err);
+                wait_or_die(&sm.wfull[jb], (st / WS) & 1, abort, err, dead);
                 const float4 rec = sm.rec[jb];
-                const int flags = ok ? __float_as_int(rec.w) : 0, nks = flags & kRecUnits;
+                const int flags = dead ? 0 : __float_as_int(rec.w), nks = flags & kRecUnits;
                 // the MMAs that last read the slot must be done before the first
                 // store into it
                 auto claim = [&]() {
-                    if (!slot_free) wait_bounded(&sm.kempty[slot], kpar, abort, err);
+                    if (!slot_free) wait_or_die(&sm.kempty[slot], kpar, abort, err, dead);
                     slot_free = true;
                 };
                 // kernel value x displacement (leaf: projected east, north; proxy: the
@@ -1208,12 +1228,13 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                 claim();
                 dev::fence_proxy_async();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_n(&sm.kfull[slot], down ? 1 : 2);
+                if (lane == 0 && !dead) mbar_arrive_n(&sm.kfull[slot], down ? 1 : 2);
             }
         }
     } else if (warp == kMmaWarp) {
         // ============================================================ MMA issue
         uint32_t cc = 0;           // chains started
+        uint32_t cpar = 0;         // partial replay: as the producers'
         bool chain_open = false;
         for (int gi = blockIdx.x; gi < total; gi += gridDim.x) {
             const int gk = grid_of(gi);
@@ -1240,15 +1261,18 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                 const uint32_t slot = st % KS, jb = st % WS;
                 // replay: the stage's one barrier covers its weight and kernel tiles
                 // (polled together: the one's latency hides the other's)
-                bool ok = true;
                 const bool wf = TS == 2 || dev::mbar_try_wait(&sm.wfull[jb], (st / WS) & 1);
                 const bool kf = dev::mbar_try_wait(&sm.kfull[slot], (st / KS) & 1);
-                if (!kf) ok = wait_bounded(&sm.kfull[slot], (st / KS) & 1, abort, err);
-                if (!wf) ok = wait_bounded(&sm.wfull[jb], (st / WS) & 1, abort, err) && ok;
+                if (!kf) wait_or_die(&sm.kfull[slot], (st / KS) & 1, abort, err, dead);
+                if (!wf) wait_or_die(&sm.wfull[jb], (st / WS) & 1, abort, err, dead);
+                if (TS == 3 && k % a.tile_every == a.tile_every - 1) {
+                    wait_or_die(&sm.kcopy[slot], (cpar >> slot) & 1, abort, err, dead);
+                    cpar ^= 1u << slot;
+                }
                 // a new chain overwrites the accumulator, whose last chain
                 // (cc - 1) the fold warps must have read
-                if (!chain_open && cc >= 1) ok = wait_bounded(&sm.accfree, (cc - 1) & 1, abort, err) && ok;
-                ok = __all_sync(0xffffffffu, ok);
+                if (!chain_open && cc >= 1) wait_or_die(&sm.accfree, (cc - 1) & 1, abort, err, dead);
+                dead = __any_sync(0xffffffffu, dead);
                 tc_fence_after();
                 int nks = (it.cnt + 7) >> 3;
                 if (kRec) {
@@ -1256,38 +1280,37 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                     nks = flags & kRecUnits;
                     flush = flags & kRecFlush;
                 }
+                flush = flush && !dead;
                 const uint32_t open = chain_open ? 1u : 0u;
-                if (elect_one()) {
-                    if (ok) {
-                        if constexpr (TS == 2) {
-                            // packed tiles of MMA step s: hi at (2s) ptile, lo at (2s + 1) ptile
-                            const uint64_t aw = smem_desc_w16(sm.ring + TcSmem<TS>::kKtBytes + sm.woff[slot]);
-                            const uint64_t bt = smem_desc(sm.ring + sm.toff[slot]);
+                if (!dead && elect_one()) {
+                    if constexpr (TS == 2) {
+                        // packed tiles of MMA step s: hi at (2s) ptile, lo at (2s + 1) ptile
+                        const uint64_t aw = smem_desc_w16(sm.ring + TcSmem<TS>::kKtBytes + sm.woff[slot]);
+                        const uint64_t bt = smem_desc(sm.ring + sm.toff[slot]);
 #pragma unroll
-                            for (int s = 0; s < SK / 16; ++s)
-                                if (2 * s < nks) {
-                                    const uint64_t a = aw + s * (2 * kW16UnitBytes >> 4), bh = bt + 2 * s * (ptile >> 4);
+                        for (int s = 0; s < SK / 16; ++s)
+                            if (2 * s < nks) {
+                                const uint64_t a = aw + s * (2 * kW16UnitBytes >> 4), bh = bt + 2 * s * (ptile >> 4);
+                                mma_ss_f16(tmem, a, bh, idesc, s ? 1u : open);
+                                mma_ss_f16(tmem, a, bh + (ptile >> 4), idesc, 1u);
+                            }
+                    } else {
+                        // FP16: 16 sources per MMA (weight units 2s and 2s + 1); TF32: 8
+                        constexpr uint32_t kStepW = kWStepFloats * 4 >> 4, kStepT = kTileFloats * 4 >> 4;
+                        const uint64_t aw = F16 ? smem_desc_w16(sm.Wt(jb)) : smem_desc(sm.Wt(jb));
+                        const uint64_t bt = smem_desc(sm.Kt(slot, 0, 0));
+#pragma unroll
+                        for (int s = 0; s < kStageKs; ++s)
+                            if ((F16 ? 2 : 1) * s < nks) {
+                                const uint64_t a = aw + s * kStepW, bh = bt + 2 * s * kStepT;
+                                if (F16) {
                                     mma_ss_f16(tmem, a, bh, idesc, s ? 1u : open);
-                                    mma_ss_f16(tmem, a, bh + (ptile >> 4), idesc, 1u);
+                                    mma_ss_f16(tmem, a, bh + kStepT, idesc, 1u);
+                                } else {
+                                    mma_ss(tmem, a, bh, idesc, s ? 1u : open);
+                                    mma_ss(tmem, a, bh + kStepT, idesc, 1u);
                                 }
-                        } else {
-                            // FP16: 16 sources per MMA (weight units 2s and 2s + 1); TF32: 8
-                            constexpr uint32_t kStepW = kWStepFloats * 4 >> 4, kStepT = kTileFloats * 4 >> 4;
-                            const uint64_t aw = F16 ? smem_desc_w16(sm.Wt(jb)) : smem_desc(sm.Wt(jb));
-                            const uint64_t bt = smem_desc(sm.Kt(slot, 0, 0));
-#pragma unroll
-                            for (int s = 0; s < kStageKs; ++s)
-                                if ((F16 ? 2 : 1) * s < nks) {
-                                    const uint64_t a = aw + s * kStepW, bh = bt + 2 * s * kStepT;
-                                    if (F16) {
-                                        mma_ss_f16(tmem, a, bh, idesc, s ? 1u : open);
-                                        mma_ss_f16(tmem, a, bh + kStepT, idesc, 1u);
-                                    } else {
-                                        mma_ss(tmem, a, bh, idesc, s ? 1u : open);
-                                        mma_ss(tmem, a, bh + kStepT, idesc, 1u);
-                                    }
-                                }
-                        }
+                            }
                     }
                     mma_commit(&sm.kempty[slot]);
                     if (TS != 2) mma_commit(&sm.wempty[jb]);
@@ -1310,6 +1333,12 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
         // ============================================================ loads
         // replay: ring heads, the oldest stage still in flight
         uint32_t thead = 0, whead = 0, oldest = 0;
+        // After a wait that gave up nothing more is expected or issued: a phase
+        // whose bytes never come would hold the drain below for its whole limit.
+        // Test hook: nothing from stage inject - 1 on.
+        bool live = true;
+        uint32_t issued = 0;   // stages issued
+        const uint32_t stop = J.g[0].inject ? J.g[0].inject - 1 : 0xffffffffu;
         for (int gi = blockIdx.x; gi < total; gi += gridDim.x) {
             const int gk = grid_of(gi);
             const TcArgs &a = J.g[gk];
@@ -1352,9 +1381,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                             sm.rec[jb] = make_float4(it.dx, it.dy, it.dz, __int_as_float(flags));
                             sm.rec2[jb] = make_int2(kind == 2 ? it.off : it.off + b, it.row0 + b);
                         }
-                        ok = __all_sync(0xffffffffu, ok);
+                        live = __all_sync(0xffffffffu, ok) && live && st < stop;
+                        if (live) issued = st + 1;
                         __syncwarp();
-                        if (elect_one()) {
+                        if (live && elect_one()) {
                             // FP16: whole 16-source MMA steps (the store has a spare unit at
                             // its end).  With the weights come the point and proxy sources'
                             // coordinates (24 floats per unit; DOWN rows need none), or the
@@ -1363,17 +1393,15 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                             const uint32_t lbytes = MODE == 2 ? nks * 64u * n : down ? 0u : nks * 96u;
                             const size_t u = (size_t)kb + b / 8;
                             dev::mbar_expect_tx(&sm.wfull[jb], wbytes + lbytes);
-                            if (ok) {
-                                if (lbytes)
-                                    dev::bulk_g2s(sm.aux[jb],
-                                                  MODE == 2 ? (const void *)(a.basis + ((size_t)row0 + b / 8) * 16 * n)
-                                                            : (const void *)(a.sxyz + u * 24),
-                                                  lbytes, &sm.wfull[jb]);
-                                dev::bulk_g2s(sm.Wt(jb),
-                                              F16 ? (const void *)(static_cast<const char *>(a.bstore16) + u * kW16UnitBytes)
-                                                  : (const void *)(a.bstore + u * kWStepFloats),
-                                              wbytes, &sm.wfull[jb]);
-                            }
+                            if (lbytes)
+                                dev::bulk_g2s(sm.aux[jb],
+                                              MODE == 2 ? (const void *)(a.basis + ((size_t)row0 + b / 8) * 16 * n)
+                                                        : (const void *)(a.sxyz + u * 24),
+                                              lbytes, &sm.wfull[jb]);
+                            dev::bulk_g2s(sm.Wt(jb),
+                                          F16 ? (const void *)(static_cast<const char *>(a.bstore16) + u * kW16UnitBytes)
+                                              : (const void *)(a.bstore + u * kWStepFloats),
+                                          wbytes, &sm.wfull[jb]);
                         }
                         __syncwarp();
                     }
@@ -1410,21 +1438,21 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
                         ++oldest;
                     }
                     const uint32_t slot = st % KS;
-                    if (elect_one()) {
+                    live = __all_sync(0xffffffffu, !*abort) && live && st < stop;
+                    if (live) issued = st + 1;
+                    if (live && elect_one()) {
                         sm.toff[slot] = tpos;
                         sm.tlen[slot] = sb;
                         sm.woff[slot] = wpos;
                         sm.wlen[slot] = wb;
                         // the offsets are written before the arrival the MMA warp waits on
                         dev::mbar_expect_tx(&sm.kfull[slot], sb + wb);
-                        if (!*abort) {
-                            // the tiles are read once per solve: they leave L2 first, to
-                            // the weight tiles, which other groups read again
-                            dev::bulk_g2s_hint(sm.ring + tpos, tsrc, sb, &sm.kfull[slot], dev::l2_evict_first());
-                            dev::bulk_g2s_hint(sm.ring + TcSmem<TS>::kKtBytes + wpos,
-                                               static_cast<const char *>(a.bstore16) + (size_t)it.kb * kW16UnitBytes,
-                                               wb, &sm.kfull[slot], dev::l2_evict_last());
-                        }
+                        // the tiles are read once per solve: they leave L2 first, to
+                        // the weight tiles, which other groups read again
+                        dev::bulk_g2s_hint(sm.ring + tpos, tsrc, sb, &sm.kfull[slot], dev::l2_evict_first());
+                        dev::bulk_g2s_hint(sm.ring + TcSmem<TS>::kKtBytes + wpos,
+                                           static_cast<const char *>(a.bstore16) + (size_t)it.kb * kW16UnitBytes,
+                                           wb, &sm.kfull[slot], dev::l2_evict_last());
                     }
                     __syncwarp();
                     tsrc += sb;
@@ -1434,12 +1462,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
             }
         }
         // no bulk copy may still be landing when the CTA exits
-        if (TS == 2 && lane == 0)
-            for (uint32_t x = oldest; x < st; ++x) wait_drain(&sm.kfull[x % KS], (x / KS) & 1, err);
-        if (TS != 2 && lane == 0)
-            for (uint32_t j = 0; j < (uint32_t)WS && j < st; ++j) {
-                const uint32_t uses = (st - 1 - j) / WS + 1;
-                wait_drain(&sm.wfull[j], (uses - 1) & 1, err);
+        if (lane == 0)
+            for (uint32_t x = issued > (TS == 2 ? KS : WS) ? issued - (TS == 2 ? KS : WS) : 0; x < issued; ++x) {
+                if (TS == 2) wait_drain(&sm.kfull[x % KS], (x / KS) & 1, err);
+                else wait_drain(&sm.wfull[x % WS], (x / WS) & 1, err);
             }
         __syncwarp();
     }
@@ -1508,6 +1534,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
     }
     tc_fence_before();
     __syncthreads();
+    // a wait gave up: copies that the MMA warp did not wait for
+    if (TS == 3 && tid == 32 && *abort)
+        for (int j = 0; j < kKStages; ++j)
+            if (sm.clast[j]) wait_drain(&sm.kcopy[j], sm.clast[j] & 1, err);
     if (warp == 0) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");

@@ -385,8 +385,9 @@ class Grid:
 
     def inject_timeout(self, polls):
         """Test hook (sal_grid_inject_timeout): the next FP64 solve's leaf
-        pass gives up a staging wait on every group after `polls` polls; the
-        host then sees SAL_ETIMEOUT."""
+        pass (or the next batched solve's first 64-field leaf pass) gives up a
+        staging wait on every group after `polls` polls (batched: after 2 s);
+        the host then sees SAL_ETIMEOUT."""
         _check(lib().sal_grid_inject_timeout(self.handle, int(polls)))
 
     def set_graphs(self, enable=True):
