@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -208,14 +209,14 @@ struct Uploads {
         unsigned char *base = nullptr;
         int rc = dalloc(g, &base, total);
         if (rc) return rc;
-        std::vector<unsigned char> host(total);
+        const std::unique_ptr<unsigned char[]> host(new unsigned char[total]);   // every part is filled below, nothing first
         size_t at = 0;
         for (const Part &q : parts) {
             *q.p = q.bytes ? base + at : nullptr;
-            if (q.bytes) std::memcpy(host.data() + at, q.src, q.bytes);
+            if (q.bytes) std::memcpy(host.get() + at, q.src, q.bytes);
             at += (q.bytes + 255) & ~size_t(255);
         }
-        if (total) CK(cudaMemcpy(base, host.data(), total, cudaMemcpyHostToDevice));
+        if (total) CK(cudaMemcpy(base, host.get(), total, cudaMemcpyHostToDevice));
         return SAL_OK;
     }
 };
@@ -468,7 +469,7 @@ extern "C" int sal_grid_stats_get(const sal_grid *G, sal_grid_stats *s) {
     s->nleaves = pl.nleaves;
     s->degree = pl.d;
     s->mode = pl.mode;
-    s->list_count = (int64_t)pl.leaf_items.size();
+    s->list_count = pl.list_items;
     s->pairs_pp = pl.pairs[0];
     s->pairs_pc = pl.pairs[1];
     s->pairs_cp = pl.pairs[2];

@@ -230,70 +230,90 @@ static void plan_build_eval(const Tree &t, const EvalBounds &bd, const std::vect
     double total = 0.0;
     for (const Set &S : sets) total += S.cost;
     const double target = std::max(kEvalMinPairs, total / kEvalUnits);
-    struct U { EvalUnit u; double cost; };
-    std::vector<U> pu, lu;
-    pl->eval_stages.clear();
-    pl->eval_items.clear();
-    pl->leaf_fin.clear();
-    pl->down_slots.clear();
-    pl->eval_proxy_unit_beg.assign(ntgt + 1, 0);
-    pl->leaf_part_rows = 0;
+    // Where each set's parts of the flat lists begin, then the lists on every
+    // host thread (set after set: 22 of the plan's 325 ms at 2.3M cells).
+    struct At {
+        int64_t stage, item, unit, fin, down, row;
+    };
+    std::vector<At> at(nsets);
+    std::vector<int32_t> parts(nsets);
+    At cur{};
+    int64_t nlu = 0;   // leaf units
     for (int64_t x = 0; x < nsets; ++x) {
         const bool proxy = x >= nl;
         const Set &S = sets[x];
-        const int32_t s0 = (int32_t)pl->eval_stages.size(), i0 = (int32_t)pl->eval_items.size();
         const int32_t ns = (int32_t)S.stages.size();
-        for (EvalStage e : S.stages) {
+        // units of about equal cost, whole stages each
+        parts[x] = std::max<int32_t>(proxy && ns == 0 ? 0 : 1, (int32_t)std::min<double>(ns, std::floor(S.cost / target + 0.5)));
+        int64_t &nu = proxy ? cur.unit : nlu;   // leaf and proxy units are numbered apart
+        at[x] = cur;
+        at[x].unit = nu;
+        cur.stage += ns;
+        cur.item += (int64_t)S.items.size();
+        nu += parts[x];
+        if (proxy) continue;
+        cur.down += (int64_t)ldown[x].size();
+        if (parts[x] == 1 && ldown[x].empty()) continue;   // straight to the outputs
+        ++cur.fin;
+        cur.row += (int64_t)parts[x] * S.nt;
+    }
+    struct U { EvalUnit u; double cost; };
+    std::vector<U> lu(nlu), pu(cur.unit);
+    pl->eval_stages.resize(cur.stage);
+    pl->eval_items.resize(cur.item);
+    pl->leaf_fin.resize(cur.fin);
+    pl->down_slots.resize(cur.down);
+    pl->eval_proxy_unit_beg.assign(ntgt + 1, 0);
+    pl->leaf_part_rows = cur.row;
+#pragma omp parallel for schedule(dynamic, 16)
+    for (int64_t x = 0; x < nsets; ++x) {
+        const bool proxy = x >= nl;
+        const Set &S = sets[x];
+        const At &A = at[x];
+        const int32_t s0 = (int32_t)A.stage, i0 = (int32_t)A.item, ns = (int32_t)S.stages.size();
+        for (int32_t k = 0; k < ns; ++k) {
+            EvalStage e = S.stages[k];
             e.ib += i0;
             e.ie += i0;
-            pl->eval_stages.push_back(e);
+            pl->eval_stages[s0 + k] = e;
         }
-        pl->eval_items.insert(pl->eval_items.end(), S.items.begin(), S.items.end());
-        // units of about equal cost, whole stages each
-        const int32_t parts = std::max<int32_t>(proxy && ns == 0 ? 0 : 1,
-                                                (int32_t)std::min<double>(ns, std::floor(S.cost / target + 0.5)));
+        std::copy(S.items.begin(), S.items.end(), pl->eval_items.begin() + i0);
         EvalUnit u{};
         u.tgt = proxy ? (int32_t)(x - nl) : (int32_t)t.p[leaves[x]].begin;
         u.nt = S.nt;
         u.proxy = proxy;
         u.fold = eval_fold(S.nt);
-        LeafFin f{};
+        bool straight = false;
         if (proxy) {
-            pl->eval_proxy_unit_beg[x - nl] = (int32_t)pu.size();
+            pl->eval_proxy_unit_beg[x - nl] = (int32_t)A.unit;
         } else {
-            f.tgt = u.tgt;
-            f.nt = S.nt;
-            f.parts = parts;
-            f.db = (int32_t)pl->down_slots.size();
-            pl->down_slots.insert(pl->down_slots.end(), ldown[x].begin(), ldown[x].end());
-            f.de = (int32_t)pl->down_slots.size();
-            f.part = (int32_t)pl->leaf_part_rows;
+            std::copy(ldown[x].begin(), ldown[x].end(), pl->down_slots.begin() + A.down);
+            straight = parts[x] == 1 && ldown[x].empty();
+            if (!straight) {
+                LeafFin &f = pl->leaf_fin[A.fin];
+                f.tgt = u.tgt;
+                f.nt = S.nt;
+                f.parts = parts[x];
+                f.part = (int32_t)A.row;
+                f.db = (int32_t)A.down;
+                f.de = f.db + (int32_t)ldown[x].size();
+            }
         }
-        const bool straight = !proxy && parts == 1 && f.db == f.de;
         int32_t i = 0;
         double done = 0.0;
-        for (int32_t k = 0; k < parts; ++k) {
+        for (int32_t k = 0; k < parts[x]; ++k) {
             const int32_t b = i;
             double c = 0.0;
-            const double want = (S.cost - done) / (parts - k);
-            while (i < ns && (k == parts - 1 || ((c == 0.0 || c + 0.5 * cost_of(S.stages[i], S.nt) < want) &&
-                                                 ns - i > parts - 1 - k)))
+            const double want = (S.cost - done) / (parts[x] - k);
+            while (i < ns && (k == parts[x] - 1 || ((c == 0.0 || c + 0.5 * cost_of(S.stages[i], S.nt) < want) &&
+                                                    ns - i > parts[x] - 1 - k)))
                 c += cost_of(S.stages[i++], S.nt);
             done += c;
             u.sb = s0 + b;
             u.se = s0 + i;
             u.sm = s0 + std::min(std::max(S.mid, b), i);
-            if (proxy) {
-                u.out = (int32_t)pu.size();
-                pu.push_back(U{u, c});
-            } else {
-                u.out = straight ? -1 : f.part + k * S.nt;
-                lu.push_back(U{u, c});
-            }
-        }
-        if (!proxy && !straight) {
-            pl->leaf_fin.push_back(f);
-            pl->leaf_part_rows += (int64_t)parts * S.nt;
+            u.out = proxy ? (int32_t)(A.unit + k) : straight ? -1 : (int32_t)A.row + k * S.nt;
+            (proxy ? pu : lu)[A.unit + k] = U{u, c};
         }
     }
     pl->eval_proxy_unit_beg[ntgt] = (int32_t)pu.size();
@@ -302,6 +322,7 @@ static void plan_build_eval(const Tree &t, const EvalBounds &bd, const std::vect
     std::stable_sort(pu.begin(), pu.end(), by_cost);
     std::stable_sort(lu.begin(), lu.end(), by_cost);
     pl->eval_units.clear();
+    pl->eval_units.reserve(pu.size() + lu.size());
     for (const U &u : pu) pl->eval_units.push_back(u.u);
     for (const U &u : lu) pl->eval_units.push_back(u.u);
     // upward units: about the same number, 256 to 4096 points each
@@ -339,13 +360,16 @@ bool plan_build(const Tree &t, const double *xs, const double *ys, const double 
     for (auto k : leaves)
         if (t.p[k].count() > 256) { *err = "leaves with more than 256 points are not supported (cluster_thresh <= 257)"; return false; }
     // leaves under panel k: contiguous in range order
-    auto leaf_range = [&](int k, int32_t *lb, int32_t *le) {
+    std::vector<std::pair<int32_t, int32_t>> under(np);
+#pragma omp parallel for schedule(static)
+    for (int k = 0; k < np; ++k) {
         const Panel &q = t.p[k];
-        *lb = (int32_t)(std::lower_bound(leaf_begin.begin(), leaf_begin.end(), q.begin) - leaf_begin.begin());
-        *le = (int32_t)(std::lower_bound(leaf_begin.begin(), leaf_begin.end(), q.end) - leaf_begin.begin());
-    };
+        under[k] = {(int32_t)(std::lower_bound(leaf_begin.begin(), leaf_begin.end(), q.begin) - leaf_begin.begin()),
+                    (int32_t)(std::lower_bound(leaf_begin.begin(), leaf_begin.end(), q.end) - leaf_begin.begin())};
+    }
     std::vector<int32_t> leaf_of_pos(n, -1);
-    for (size_t i = 0; i < leaves.size(); ++i)
+#pragma omp parallel for schedule(static)
+    for (int64_t i = 0; i < (int64_t)leaves.size(); ++i)
         for (int64_t p = t.p[leaves[i]].begin; p < t.p[leaves[i]].end; ++p) leaf_of_pos[p] = (int32_t)i;
     // ---------------------------------------------------------------- slots
     std::vector<int32_t> src_slot(np, -1), tgt_slot(np, -1);
@@ -402,22 +426,40 @@ bool plan_build(const Tree &t, const double *xs, const double *ys, const double 
     std::vector<std::vector<int32_t>> ldown(leaves.size());
     pl->masks.clear();
     if (dtt) {
-        for (int64_t i = 0; i < nlist; ++i) {
-            int k_t = list[3 * i] - 1, k_s = list[3 * i + 1] - 1, ty = list[3 * i + 2];
-            const Panel &T = t.p[k_t], &S = t.p[k_s];
-            if (T.count() == 0 || S.count() == 0) continue;
-            if (ty == 0 || ty == 1) {
-                int32_t lb, le;
-                leaf_range(k_t, &lb, &le);
-                for (int32_t l = lb; l < le; ++l) lsrc[l].push_back(EvalSrc{k_s, ty, -1});
-                pl->pairs[ty] += (double)T.count() * (ty == 0 ? S.count() : P);
-            } else {
-                tsrc[tgt_slot[k_t]].push_back(EvalSrc{k_s, ty - 2, -1});
-                pl->pairs[ty] += (double)P * (ty == 2 ? S.count() : P);
-            }
-        }
-        // the same as work-list items, each set in list order
+        // each leaf's and target slot's sources, and each leaf's DOWN slots (every
+        // leaf under a target slot interpolates its potentials); counted first, so
+        // that no list grows
         const int64_t nl = (int64_t)leaves.size();
+        std::vector<int32_t> nsrcs(nl + ntgt, 0), ndowns(nl, 0);
+        auto each = [&](auto &&leaf, auto &&slot) {
+            for (int64_t i = 0; i < nlist; ++i) {
+                const int k_t = list[3 * i] - 1, k_s = list[3 * i + 1] - 1, ty = list[3 * i + 2];
+                if (t.p[k_t].count() == 0 || t.p[k_s].count() == 0) continue;
+                if (ty >= 2) slot(tgt_slot[k_t], EvalSrc{k_s, ty - 2, -1});
+                else
+                    for (int32_t l = under[k_t].first; l < under[k_t].second; ++l) leaf(l, EvalSrc{k_s, ty, -1});
+            }
+        };
+        each([&](int32_t l, const EvalSrc &) { ++nsrcs[l]; }, [&](int32_t s, const EvalSrc &) { ++nsrcs[nl + s]; });
+        for (int32_t s = 0; s < ntgt; ++s)
+            for (int32_t l = under[pl->tgt_slot_panel[s]].first; l < under[pl->tgt_slot_panel[s]].second; ++l) ++ndowns[l];
+#pragma omp parallel for schedule(static)
+        for (int64_t x = 0; x < nl + ntgt; ++x) {
+            (x < nl ? lsrc[x] : tsrc[x - nl]).reserve(nsrcs[x]);
+            if (x < nl) ldown[x].reserve(ndowns[x]);
+        }
+        each([&](int32_t l, const EvalSrc &e) { lsrc[l].push_back(e); }, [&](int32_t s, const EvalSrc &e) { tsrc[s].push_back(e); });
+        for (int32_t s = 0; s < ntgt; ++s) {
+            for (int32_t l = under[pl->tgt_slot_panel[s]].first; l < under[pl->tgt_slot_panel[s]].second; ++l) ldown[l].push_back(s);
+            pl->macs_down += (double)t.p[pl->tgt_slot_panel[s]].count() * P;
+        }
+        for (int64_t i = 0; i < nlist; ++i) {
+            const Panel &T = t.p[list[3 * i] - 1], &S = t.p[list[3 * i + 1] - 1];
+            const int ty = list[3 * i + 2];
+            if (T.count() == 0 || S.count() == 0) continue;
+            pl->pairs[ty] += (ty >= 2 ? (double)P : (double)T.count()) * (ty == 0 || ty == 2 ? (double)S.count() : (double)P);
+        }
+        // the same as work-list items, each set in list order, DOWN items last
 #pragma omp parallel for schedule(dynamic, 16)
         for (int64_t x = 0; x < nl + ntgt; ++x) {
             const bool proxy = x >= nl;
@@ -430,17 +472,11 @@ bool plan_build(const Tree &t, const double *xs, const double *ys, const double 
                 else push_range(v, proxy_off(e.panel), P, 1, -1);
                 c += (e.kind == 0 ? (double)S.count() : (double)P) * nt;
             }
-        }
-        // DOWN items: every leaf under a target slot interpolates its potentials
-        for (int32_t s = 0; s < ntgt; ++s) {
-            int32_t lb, le;
-            leaf_range(pl->tgt_slot_panel[s], &lb, &le);
-            for (int32_t l = lb; l < le; ++l) {
-                litems[l].push_back(Item{s, 0, -1, 2});
-                ldown[l].push_back(s);
-                lcost[l] += (double)P * t.p[leaves[l]].count() * 0.5;
+            if (proxy) continue;
+            for (int32_t s : ldown[x]) {
+                v.push_back(Item{s, 0, -1, 2});
+                c += (double)P * nt * 0.5;
             }
-            pl->macs_down += (double)t.p[pl->tgt_slot_panel[s]].count() * P;
         }
     } else {
         // STT: per-point pairs become per-leaf items with per-target bitmasks.
@@ -471,7 +507,8 @@ bool plan_build(const Tree &t, const double *xs, const double *ys, const double 
             put(pp, npp, 0);
         }
         std::vector<std::vector<uint32_t>> lmask(leaves.size());
-#pragma omp parallel for schedule(dynamic, 16)
+        int64_t nitems = 0;
+#pragma omp parallel for schedule(dynamic, 16) reduction(+ : nitems)
         for (int64_t l = 0; l < (int64_t)leaves.size(); ++l) {
             const int64_t nt = t.p[leaves[l]].count();
             const int words = (int)((nt + 31) / 32);
@@ -491,12 +528,11 @@ bool plan_build(const Tree &t, const double *xs, const double *ys, const double 
                 }
                 mk[(size_t)slot * words + recs[r].local / 32] |= 1u << (recs[r].local % 32);
             }
-            // emit items in (kind, panel) order for locality; mask offsets are
+            // sources in (panel, kind) order for locality; mask offsets are
             // leaf-local here and rebased below
             std::vector<int32_t> ordk(keys.size());
             std::iota(ordk.begin(), ordk.end(), 0);
             std::sort(ordk.begin(), ordk.end(), [&](int a, int b) { return keys[a] < keys[b]; });
-            double c = 0;
             for (int32_t a : ordk) {
                 int32_t k_s = keys[a] / 2, kind = keys[a] % 2;
                 // an item that every target of the leaf takes needs no mask
@@ -504,15 +540,12 @@ bool plan_build(const Tree &t, const double *xs, const double *ys, const double 
                 for (int w = 0; w < words && all; ++w)
                     all = mk[(size_t)a * words + w] == (w + 1 < words || nt % 32 == 0 ? ~0u : (1u << (nt % 32)) - 1u);
                 lsrc[l].push_back(EvalSrc{k_s, kind, all ? -1 : a * words});
-                if (kind == 0) push_range(litems[l], t.p[k_s].begin, t.p[k_s].count(), 0, a * words);
-                else push_range(litems[l], proxy_off(k_s), P, 1, a * words);
-                c += (double)(kind == 0 ? t.p[k_s].count() : P) * nt;
+                nitems += ((kind == 0 ? t.p[k_s].count() : (int64_t)P) + kMaxStage - 1) / kMaxStage;
             }
-            lcost[l] = c;
         }
+        pl->list_items = nitems;
         for (size_t l = 0; l < leaves.size(); ++l) {
             int32_t base = (int32_t)pl->masks.size();
-            for (auto &it : litems[l]) it.mask += base;
             for (auto &e : lsrc[l])
                 if (e.mask >= 0) e.mask += base;
             pl->masks.insert(pl->masks.end(), lmask[l].begin(), lmask[l].end());
@@ -521,24 +554,27 @@ bool plan_build(const Tree &t, const double *xs, const double *ys, const double 
         for (int64_t i = 0; i < npp; ++i) pl->pairs[0] += (double)t.p[pp[2 * i + 1] - 1].count();
     }
     // ---------------------------------------------------------------- groups, sorted by cost
-    {
+    // (the batched form's: single-tree plans have none)
+    pl->leaf_groups.clear();
+    pl->leaf_items.clear();
+    if (dtt) {
         std::vector<int32_t> ord(leaves.size());
         std::iota(ord.begin(), ord.end(), 0);
         std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return lcost[a] > lcost[b]; });
-        pl->leaf_groups.clear();
-        pl->leaf_items.clear();
-        pl->max_nt = 0;
         for (int32_t l : ord) {
             const Panel &L = t.p[leaves[l]];
             Group g{};
             g.tgt = (int32_t)L.begin; g.nt = (int32_t)L.count();
-            g.ib = (int32_t)pl->leaf_items.size();
-            pl->leaf_items.insert(pl->leaf_items.end(), litems[l].begin(), litems[l].end());
-            g.ie = (int32_t)pl->leaf_items.size();
+            g.ib = (int32_t)pl->list_items;
+            pl->list_items += (int64_t)litems[l].size();
+            g.ie = (int32_t)pl->list_items;
             g.out = l;
-            pl->max_nt = std::max(pl->max_nt, g.nt);
             pl->leaf_groups.push_back(g);
         }
+        pl->leaf_items.resize(pl->list_items);
+#pragma omp parallel for schedule(dynamic, 16)
+        for (int64_t x = 0; x < (int64_t)ord.size(); ++x)
+            std::copy(litems[ord[x]].begin(), litems[ord[x]].end(), pl->leaf_items.begin() + pl->leaf_groups[x].ib);
     }
     {
         // proxy groups: each target slot's items split into units of bounded work
@@ -680,14 +716,16 @@ void plan_build_mix(const Tree &t, Plan *pl) {
 // 16, 32 bytes per row.
 void plan_tile_offsets(Plan *pl, int every) {
     pl->tc_tile_off.assign(pl->tc_leaf_groups.size() + 1, 0);
-    for (size_t gi = 0; gi < pl->tc_leaf_groups.size(); ++gi) {
+#pragma omp parallel for schedule(static)
+    for (int64_t gi = 0; gi < (int64_t)pl->tc_leaf_groups.size(); ++gi) {
         const MixGroup &m = pl->tc_leaf_groups[gi];
         const int64_t cb = (int64_t)((m.nt + 15) & ~15) * 32;
         int64_t b = 0;
         for (int32_t i = m.ib; i < m.ie; ++i)
             if ((i - m.ib) % every == every - 1) b += (int64_t)(((pl->tc_items[i].cnt + 7) / 8 + 1) / 2) * 4 * cb;
-        pl->tc_tile_off[gi + 1] = pl->tc_tile_off[gi] + b;
+        pl->tc_tile_off[gi + 1] = b;
     }
+    for (size_t gi = 0; gi < pl->tc_leaf_groups.size(); ++gi) pl->tc_tile_off[gi + 1] += pl->tc_tile_off[gi];
 }
 
 bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *err) {
@@ -925,8 +963,18 @@ bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *e
     struct Job {
         int32_t ib, ie, kt, extra;
     };
+    // a job's items, the DOWN items at their end (the work lists hold them after
+    // all others), and the stages of kTcStage K columns of both
+    struct Range {
+        int32_t ib, ie, ndown, nst, nstd;
+    };
+    auto stages = [](const TcItem *b, const TcItem *e) {
+        int32_t k = 0;
+        for (; b < e; ++b) k += (b->cnt + kTcStage - 1) / kTcStage;
+        return k;
+    };
     auto convert_all = [&](const std::vector<Item> &src, const std::vector<Job> &jobs, std::vector<TcItem> &dst,
-                           std::vector<std::pair<int32_t, int32_t>> &range) -> bool {
+                           std::vector<Range> &range) -> bool {
         const int64_t nj = (int64_t)jobs.size();
         std::vector<std::vector<TcItem>> part(nj);
         int bad = 0;
@@ -942,16 +990,12 @@ bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *e
 #pragma omp parallel for schedule(dynamic, 32)
         for (int64_t j = 0; j < nj; ++j) {
             std::copy(part[j].begin(), part[j].end(), dst.begin() + off[j]);
-            range[j] = {(int32_t)off[j], (int32_t)off[j + 1]};
+            const TcItem *b = part[j].data(), *e = b + part[j].size(), *d = e;
+            while (d > b && (d[-1].kind & 3) == 2) --d;
+            range[j] = {(int32_t)off[j], (int32_t)off[j + 1], (int32_t)(e - d), stages(b, e), stages(d, e)};
+            std::vector<TcItem>().swap(part[j]);
         }
         return true;
-    };
-
-    // stages of kTcStage K columns of items [ib, ie)
-    auto stages = [](const std::vector<TcItem> &items, int32_t ib, int32_t ie) {
-        int32_t k = 0;
-        for (int32_t i = ib; i < ie; ++i) k += (items[i].cnt + kTcStage - 1) / kTcStage;
-        return k;
     };
 
     // ---- leaf pass: groups of at most kTcRows targets in pool order
@@ -960,7 +1004,7 @@ bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *e
     std::sort(gord.begin(), gord.end(), [&](int a, int b) { return pl->leaf_groups[a].tgt < pl->leaf_groups[b].tgt; });
     pl->tc_macs_down = 0;
     std::vector<Job> jobs;
-    std::vector<std::pair<int32_t, int32_t>> range;
+    std::vector<Range> range;
     jobs.reserve(gord.size());
     for (int32_t gi : gord) {
         const Group &g = pl->leaf_groups[gi];
@@ -970,17 +1014,13 @@ bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *e
     for (size_t x = 0; x < gord.size(); ++x) {
         const Group &g = pl->leaf_groups[gord[x]];
         const int kt = leaves[g.out];
-        const int32_t ib = range[x].first, ie = range[x].second;
         if (tree && leaf_phi_block[g.out] >= 0) pl->tc_macs_down += (double)g.nt * P;
-        // DOWN items end the list (the work lists hold them after all others)
-        int32_t ndown = 0;
-        while (ndown < ie - ib && (pl->tc_items[ie - 1 - ndown].kind & 3) == 2) ++ndown;
-        const int32_t nst = stages(pl->tc_items, ib, ie), nstd = stages(pl->tc_items, ie - ndown, ie);
+        const Range &q = range[x];
         for (int32_t r = 0; r < g.nt; r += kTcRows) {
             MixGroup m{};
-            m.tgt = g.tgt + r; m.nt = std::min(kTcRows, g.nt - r); m.ib = ib; m.ie = ie; m.out = g.out;
+            m.tgt = g.tgt + r; m.nt = std::min(kTcRows, g.nt - r); m.ib = q.ib; m.ie = q.ie; m.out = g.out;
             m.cx = t.cx[kt]; m.cy = t.cy[kt]; m.cz = t.cz[kt];
-            m.ndown = ndown; m.nst = nst; m.nstd = nstd;
+            m.ndown = q.ndown; m.nst = q.nst; m.nstd = q.nstd;
             pl->tc_leaf_groups.push_back(m);
         }
     }
@@ -1029,7 +1069,7 @@ bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *e
             const int32_t uo = ord[x];
             const U &u = units[uo];
             const int kt = pl->tgt_slot_panel[u.slot];
-            const int32_t ib = range[x].first, ie = range[x].second, nst = stages(pl->tc_proxy_items, ib, ie);
+            const int32_t ib = range[x].ib, ie = range[x].ie, nst = range[x].nst;
             for (int32_t r = 0; r < P; r += kTcProxyRows) {
                 MixGroup m{};
                 m.nst = nst;
@@ -1065,7 +1105,7 @@ bool plan_build_tc(const Tree &t, Plan *pl, const TcOptions &opt, std::string *e
                 ++nbk;
             }
         }
-        const int32_t nst = stages(pl->tc_up_items, ib, ie);
+        const int32_t nst = stages(pl->tc_up_items.data() + ib, pl->tc_up_items.data() + ie);
         for (int32_t r = 0; r < P; r += kTcRows) {
             MixGroup m{};
             m.nst = nst;

@@ -244,7 +244,7 @@ struct Plan {
     double tc_macs_up = 0, tc_macs_down = 0;      // per field: basis MACs of the batched form's upward / DOWN work
     double pairs[4] = {0, 0, 0, 0};               // PP, PC, CP, CC evaluations per field
     double macs_up = 0, macs_down = 0;
-    int32_t max_nt = 0;
+    int64_t list_items = 0;                       // leaf work-list items (single-tree plans: counted only)
 };
 
 // Builds the plan of a DTT list (triplets) or STT lists (pairs).
