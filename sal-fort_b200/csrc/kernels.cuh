@@ -207,14 +207,17 @@ __device__ __forceinline__ double fast_sqrt(double x) {
 // one square root, one reciprocal, no cancellation.  kReg: p1's + 1e-16,
 // folded into D: c (2 + b q) there takes c kC1/q^6 off N / D up to 4 c/q of it
 // (c = 1e-16, b = 1 + 2 kC2/kC1); p2's is below 2e-13 of the value for
-// q > 1e-3.  15 FP64 instructions (16 with kReg) against 31 of the two
-// denominators' form with its FP32 seeds.
+// q > 1e-3.  Without kReg (far pairs, q > 0.0122, where c is 5e-11 of q^3) b q
+// is a constant, its value at q = 0.01225: 1e-13 of the value left, at q = 0.02,
+// and no instruction more than with no c at all.  14 FP64 instructions (15 with
+// kReg) against 31 of the two denominators' form with its FP32 seeds.
 template <bool kReg>
 __device__ __forceinline__ double val_chord(double mp, double w) {
     const double q = fast_sqrt(mp);
     const double n = fma(-2.0 * kC2, mp, fma(kC1 - 2.0 * kC2, q, 2.0 * kC1));
     const double t = fma(2.0, q, mp);
-    const double d = kReg ? fma(mp, t, fma(1e-16 * (1.0 + 2.0 * kC2 / kC1), q, 2e-16)) : mp * t;
+    constexpr double b = 1e-16 * (1.0 + 2.0 * kC2 / kC1);
+    const double d = fma(mp, t, kReg ? fma(b, q, 2e-16) : 2e-16 + 0.01225 * b);
     const double r = rcp_seed(d), e = fma(-d, r, 1.0), u = n * r;
     return fma(u, fma(e, e, e), u) * w;   // w last: an infinite one gives a signed infinity
 }

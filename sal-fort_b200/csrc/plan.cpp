@@ -141,7 +141,7 @@ struct EvalBounds {
     // needed: a fused dot product's 2 - 2g is within 2e-16 / 1.5e-4 = 1.5e-12
     // of the reference's at the nearest such pair (chord 0.012; with more than
     // a thousand such pairs in a sum and nearer ones above them, below 2e-13
-    // of it), and neither the + 1e-16 nor the antipode is in reach.
+    // of it), and the antipode is not in reach.
     bool near(int kt, bool proxy, const EvalSrc &s) const {
         const double rt = proxy ? rbox[kt] : rpts[kt], rs = s.kind ? rbox[s.panel] : rpts[s.panel];
         const double d = dist(kt, t.cx[s.panel], t.cy[s.panel], t.cz[s.panel]);
