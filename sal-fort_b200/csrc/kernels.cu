@@ -2,7 +2,7 @@
 //
 // All passes are compute-bound on the FP64 pipe: every staged source tile is
 // reused by every target of its group (up to 256), so HBM traffic per pair is
-// a few bytes against ~60 FP64 operations.
+// a few bytes against 20 FP64 instructions (far pairs) or 27 (near ones).
 #include <cmath>
 #include <cuda_runtime.h>
 
@@ -168,12 +168,11 @@ void launch_upward_finalize(const int32_t *unit_beg, const double *partial, int 
 // waste), and a last chunk of m <= 16 lanes takes 32 / m residues more.  The
 // (chunk, source) plane is cut into one equal run per warp: a fraction of the
 // sources of at most two chunks, the same ones in every stage, whose sums the
-// warp keeps.  (One thread per target and whole source splits left a leaf of
-// 148 targets with 5 of 8 warps at work, two of them on one scheduler: 62 % of
-// the FP64 pipe.)  The sums are added in a fixed order at the end, so results
-// are deterministic.  Stages
-// are near (gref_near: the reference's operation order where its rounding
-// noise counts) or far (gref_far).
+// warp keeps (eval_cut.hpp).  (One thread per target and whole source splits
+// left a leaf of 148 targets with 5 of 8 warps at work, two of them on one
+// scheduler: 62 % of the FP64 pipe.)  The sums are added in a fixed order at the
+// end, so results are deterministic.  Stages are near (gref_near: the reference's
+// operation order where its rounding noise counts) or far (gref_far).
 //   Leaf units and FORM 0 proxies: the reference kernel.  FORM 1 proxies: the
 //   Cartesian sum val (s - x) w with the antipode-stable val.
 // Bound by the FP64 pipe: an instruction with three register operands takes

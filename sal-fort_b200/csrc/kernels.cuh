@@ -42,7 +42,6 @@ inline void launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem
 constexpr double kCons = -2.343256857908601e-9;
 constexpr double kC1 = 1.0 - 6.21196;
 constexpr double kC2 = 2.7 + 6.0;
-constexpr int kThreads = 256;
 constexpr int kErrTimeout = 1;
 
 // ----------------------------------------------------------------- PTX helpers
@@ -299,7 +298,7 @@ __device__ __forceinline__ void gref_near(const Tgt &t, const double4 *s, int st
 // target (nx = tx Ay - ty Ax, ny = (1 - tz^2) Az - tz (tx Ax + ty Ay)).  The
 // vector cancels by the chord on projection, and no chord is below 0.012, so
 // its rounding stays below 1e-13 of a sum of thousands of pairs.  mt = -2 t.
-// 20 FP64 instructions against 28 of gref_near's plain branch.
+// 20 FP64 instructions against 27 of gref_near's plain branch.
 // K sources s[0], s[stride], ...: independent chains side by side.
 template <int K>
 __device__ __forceinline__ void gref_far(const double (&mt)[3], const double4 *s, int stride, double (&A)[3]) {

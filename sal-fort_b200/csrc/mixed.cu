@@ -71,7 +71,7 @@ __device__ __forceinline__ int bofs(int k, int f) {
 }
 
 // val / kCons of the kernel in FP32 from the chord length squared mp = |s - t|^2
-// (the antipode-stable form of dev::vstable without its 1e-16 terms, which
+// (the antipode-stable form, as dev::val_chord, without the 1e-16 terms, which
 // only matter at s == t):  with r = 1/q and u = 1/(2 + q),
 //   kC1/q^3 - 2 kC2 (1 + q)/(q^2 (2 + q)) = r^2 (kC1 r - 2 kC2 (1 - u)).
 // mp == 0 (the self pair, added separately in FP64) gives 0.  The constant

@@ -56,8 +56,8 @@
 // writes them to device memory; a replaying launch (TS 2) has the loader copy
 // each stage's tiles and weights into two shared-memory byte rings, and the
 // idle producer warps fold beside the fold warps; a partial replay (TS 3)
-// has producer warp 0 copy the stored items' tiles into the ring slot while
-// the producers compute the others.  All three give the computing launch's
+// has a team's first producer warp copy the stored items' tiles into the ring
+// slot while the producers compute the others.  All three give the computing launch's
 // results bit for bit.
 // The tensor cores accumulate with truncation, so one chain over all of a
 // target's sources would bias the result toward zero: a chain ends after about
@@ -124,9 +124,8 @@ constexpr int kRecUnits = 15, kRecDown = 32, kRecFlush = 64, kRecSelf = 128;
 // go into two byte rings (a stage takes its own size, so the small groups'
 // stages do not hold whole 64 KB slots), with up to kRStages stages in
 // flight.  A stage's tiles are packed: per MMA step and hi / lo, the group's
-// east rows then its north rows (rows rounded up to 16); an MMA reads 256
-// rows from a tile's start, the rows past the group's are columns no fold
-// reads.
+// east rows then its north rows (rows rounded up to 16), which are the rows an
+// MMA reads.
 constexpr int kRStages = 8;
 constexpr int kTRingBytes = 180 * 1024;
 constexpr int kWRingBytes = 44 * 1024;
@@ -695,13 +694,6 @@ __global__ void __launch_bounds__(kThreads, 1) tc_leaf_kernel(const __grid_const
         const int kk = k < 3 * P ? k : 0;
         const int p = kk / 3;
         sm.kmap[k] = (p % n) | ((p / n) << 8) | ((kk % 3) << 16);
-    }
-    if (TS == 2) {
-        // replay copies only a group's rows: the ring's other rows hold
-        // zeros or an earlier group's finite values (columns no output reads)
-        uint4 *z = reinterpret_cast<uint4 *>(sm.ring);
-        for (int i = tid; i < (int)(sizeof(sm.ring) / sizeof(uint4)); i += kThreads) z[i] = make_uint4(0u, 0u, 0u, 0u);
-        dev::fence_proxy_async();
     }
     tc_fence_before();
     __syncthreads();
