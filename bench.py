@@ -684,16 +684,15 @@ def main():
         achieved = leaf_flops / (leaf_ms * 1e-3) / 1e12
         prec = "FP16" if f16 else "TF32"
         src = "bf16_tflops of measured" if "bf16_tflops" in peaks else "1.59 PFLOP/s bf16 fallback"
-        roof = {"bound": "tensor", "kernel": f"tc_leaf_kernel<0> (tcgen05 {prec} hi/lo, M=128 field parts x N=256 "
-                          "target components; PP+PC kernel tiles, DOWN interpolation) + its weight store",
+        roof = {"bound": "tensor", "kernel": f"tc_leaf_kernel<0> (tcgen05 {prec} hi/lo, M=128 field parts x N = "
+                          "2 x the group's targets, rounded up to 16; PP+PC kernel tiles, DOWN interpolation) + its weight store",
                 "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "peak_source": (f"FP16 dense = {src}" if f16 else f"TF32 dense = {src} / 2"),
                 "flops_counted": "algorithmic 4*F per pair (2 components x FMA x F fields); the hi/lo split "
                                  "executes 4x these on the tensor cores (W_hi,W_lo x T_hi,T_lo), plus padding",
                 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one tc_leaf_kernel launch on the
-                # 655,362-cell, 64-field case (FP16: 4.01 + 2.76 GB; TF32: 3.95 + 2.65 GB), scaled by the
-                # cell count
-                "traffic": (6.767e9 if f16 else 6.600e9) * g.n / 655362 if F == 64 else None,
+                # 655,362-cell, 64-field case (FP16: 7.26 GB; TF32: 8.18 GB), scaled by the cell count
+                "traffic": (7.26e9 if f16 else 8.18e9) * g.n / 655362 if F == 64 else None,
                 "traffic_source": "ncu capture on 655,362 cells x 64 fields, scaled by cells",
                 "leaf_ms": leaf_ms, "proxy_ms": proxy_ms, "prep_upward_ms": up_ms}
         if tile:

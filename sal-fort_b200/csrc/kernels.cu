@@ -563,7 +563,7 @@ void launch_proxy_finalize(const int32_t *unit_beg, const double4 *partial, int 
 // target per thread, sources staged through shared memory, gref_near 4 pairs
 // at a time (g in the reference's operation order, val_ref for the self pair
 // and the other pairs whose value is rounding noise).  Bound by the FP64 pipe:
-// 27 instructions a pair (10,000 targets x 655,362 sources: 12.5 ms, 72 cycles
+// 27 instructions a pair (10,000 targets x 655,362 sources: 12.3 ms, 71 cycles
 // a pair and scheduler of the 68 that a loop of nothing else takes), where
 // IEEE division and square root took about 110 (31.4 ms).  The sources are split into
 // chunks (blockIdx.y) whose partial sums are added in a fixed order.
